@@ -195,7 +195,10 @@ int wbg_eigh_batched_noalloc(const void* H, long long strideH, int nw, int nk, d
  * herm[f] | 4: X[fsel[f]] holds only its lower triangle (wbg_r2k_columns output); it is read
  * as the Hermitian matrix with that lower triangle and a real diagonal.
  * fp64 == 0 and nw == 32 run on the tensor cores (tcgen05, products split into three TF32
- * terms, FP32 accumulation) when X is 16-byte aligned; other cases on the CUDA cores. */
+ * terms, FP32 accumulation) when X is 16-byte aligned.  fp64 == 1 with 4 <= nw <= 128 and fp64 == 2
+ * with 32 < nw <= 128 (16-byte aligned U and X) also run on the tensor cores: operands in 8-bit slices
+ * whose fp16 products sum exactly, one rounding per GEMM; a field (or U) with a non-finite element
+ * gives NaN throughout.  Other cases on the CUDA cores. */
 int wbg_rotate(const void* U, long long strideU, const void* X, int nFin, const int* fsel, const int* herm,
                int nFrot, void* Xbar, int nw, int nk, int fp64, void* stream);
 
@@ -468,6 +471,8 @@ int wbg_scan_finalize(const void* hist, int nEF, int ncomp, double scale, double
  *   WBG_TUNE_EIGH_VECTORS_GROUP  matrices per block of the inverse iteration and
  *                                back-transform                                variant: eigh mode & 3
  *   WBG_TUNE_ROTATE_KPOINTS      k-points per block of the CUDA-core tiled U^dagger X U  variant: fp64
+ *                                (FP64: listed and kept for saved tables; the tensor-core
+ *                                rotation that serves FP64 does not read it)
  *   WBG_TUNE_ROTATE_ENGINE       1 tensor cores, warp-specialised (two tiles in flight), 2 CUDA
  *                                cores, 3 tensor cores one tile at a time (the built-in choice;
  *                                where they serve the case)                    variant: fp64

@@ -12,6 +12,7 @@
 #include "wbgpu_common.cuh"
 #include "wbgpu_df64.cuh"
 #include "wbgpu_fixed.cuh"
+#include <type_traits>
 #include "wbgpu_band.cuh"
 #include "wbgpu_tune.cuh"
 #include "wbgpu_spin.cuh"
@@ -1769,6 +1770,8 @@ template <typename T, typename VO = typename C2<T>::t>
 int launch_rotate(const void* U, long long strideU, const void* X, int nFin, const int* fsel, const int* herm,
                   int nFrot, void* Xbar, int nw, int nk, cudaStream_t stream) {
   typedef typename C2<T>::t V;
+  // FP64 comes here below WBG_OZ_MIN_NW only (wbg_rotate_oz_supported)
+  if constexpr (!std::is_same<T, double>::value) {
   if (nw > 64) {  // row panels: the per-k matrices no longer fit in shared memory together
     if (nw > 4 * 256 / (PANEL_RP / 4)) return WBG_ERR_SIZE;  // threads = (RP/4) * ceil(nw/4) <= 256
     const int np = (nw + PANEL_RP - 1) / PANEL_RP;
@@ -1795,6 +1798,7 @@ int launch_rotate(const void* U, long long strideU, const void* X, int nFin, con
       return wbg_cuda_status(cudaGetLastError());
     }
   }
+  }
   const size_t sm = 3 * (size_t)nw * nw * sizeof(V);
   if (sm > 220 * 1024) return WBG_ERR_SIZE;
   // rotate_kernel writes every element (treats herm == 2 like 1): the full Hermitian part is a
@@ -1816,8 +1820,11 @@ int wbg_rotate_run(const void* U, long long strideU, const void* X, int nFin, co
   if (wbg_rotate_tc_supported(nw, fp64, nFrot) && (reinterpret_cast<uintptr_t>(X) & 15) == 0 && engine != 2)
     return wbg_rotate_tc_run(U, strideU, X, nFin, fsel, herm, nFrot, Xbar, nw, nk, stream, engine != 1);
   if (fp64 < 0 || fp64 > 2) return WBG_ERR_ARG;
+  if (wbg_rotate_oz_supported(U, X, nw, fp64))
+    return wbg_rotate_oz_run(U, strideU, X, nFin, fsel, herm, nFrot, Xbar, nw, nk, fp64, stream);
   if (fp64 == 2)  // double-float U and X, products in double-float, Xbar rounded to complex64
     return launch_rotate<df64, float2>(U, strideU, X, nFin, fsel, herm, nFrot, Xbar, nw, nk, stream);
+  if (fp64 && nw > 128) return WBG_ERR_SIZE;
   if (fp64) return launch_rotate<double>(U, strideU, X, nFin, fsel, herm, nFrot, Xbar, nw, nk, stream);
   return launch_rotate<float>(U, strideU, X, nFin, fsel, herm, nFrot, Xbar, nw, nk, stream);
 }

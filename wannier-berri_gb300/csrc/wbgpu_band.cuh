@@ -12,6 +12,11 @@ bool wbg_rotate_tc_supported(int nw, int fp64, int nFrot);
 // serial = true: the one-tile-at-a-time kernel (two CTAs per SM) instead of the warp-specialised one
 int wbg_rotate_tc_run(const void* U, long long strideU, const void* X, int nFin, const int* fsel, const int* herm,
                       int nFrot, void* Xbar, int nw, int nk, cudaStream_t stream, bool serial = false);
+// FP64 / double-float rotation on the fp16 tensor cores (8-bit slices, exact sums); 16-byte aligned operands
+#define WBG_OZ_MIN_NW 4
+bool wbg_rotate_oz_supported(const void* U, const void* X, int nw, int fp64);
+int wbg_rotate_oz_run(const void* U, long long strideU, const void* X, int nFin, const int* fsel, const int* herm,
+                      int nFrot, void* Xbar, int nw, int nk, int fp64, cudaStream_t stream);
 int wbg_device_flags_run(unsigned int* flags, int clear);
 int wbg_tc_wait_limit_run(unsigned long long ns);
 int wbg_tc_wait_probe_run(int* result, cudaStream_t stream);

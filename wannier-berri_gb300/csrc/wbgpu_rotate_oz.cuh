@@ -1,0 +1,799 @@
+// Band-basis rotation Xbar = U^dagger X U in FP64 (and double-float) accuracy on the fp16 tensor
+// cores: the operands are cut into 8-bit slices whose products the tensor cores sum exactly.
+// Included by wbgpu_rotate_tc.cu inside its namespace (shared tcgen05 / mbarrier helpers).
+//
+// Every operand is brought to 64-bit fixed point relative to the largest exponent of its matrix,
+// v with |v| < 2^62, and written as signed digits v = sum_i d_i 2^(56 - 8 i), d_i in [-128, 127]:
+// the bytes of v + 0x8080..80, less 128 each.  A digit is an exact fp16 number, a product of two
+// an integer below 2^14, and the products of one significance g = i + j, summed over K <= 256 and
+// the pairs of a group, stay below 2^24 (up to K = 128; beyond, only the groups g >= 4 could pass it,
+// whose last unit is 2^-44 of the result): FP32 accumulation in tensor memory is exact.  The NG
+// groups g < NG are kept (8 for FP64: 36 pairs; 7 for double-float: 28) and recombined in 64-bit
+// integers: sum_g acc_g 2^(8 (NG - 1 - g)).  The dropped pairs lie 2^-58 (FP64) and 2^-50
+// (double-float) below the largest products, so each GEMM rounds once, like an FP64 sum of exact
+// products.  Against 113-bit products, 2-norm, random X and unitary U: 5.0e-17 at nw = 32 and
+// 7.4e-17 at nw = 128, where the CUDA-core FP64 chains gave 3.8e-16 and 7.6e-16.  The scale is one per
+// matrix: with elements spread over e^+-16 the error is 1e-16 (chains: 4e-16) up to nw = 32 and
+// 1.3e-15 (chains: 6e-16) at nw = 128.
+//
+// Bound by the CUDA cores: cutting the operands (about 40 instructions an element), recombining
+// the groups and the conversions run on integer units, since the FP64 pipe (64 times slower than FP32)
+// is what this avoids.  nw = 32, 9 fields, 13 824 k-points: 44.8 ms (CUDA-core FP64, 97% of the pipe)
+// -> 5.7 ms; of the 44 k cycles of a 96-row tile 13 k wait for the products (36 pairs x 4 K steps of
+// M = 128, N = 64: 4.6 k at full rate per GEMM).  nw = 96, 9 fields, 512 k-points: 27.7 ms
+// (double-float) -> 5.1 ms, 53.4 ms (FP64) -> 4.9 ms.
+//
+// Complex products are embedded in real ones as in the TF32 kernel above; operand rows are 128-byte
+// (64-byte) swizzled K-major rows of 64 (32) fp16.  Consecutive B slices are consecutive rows of
+// shared memory and their products consecutive accumulators, so one tcgen05.mma of N = up to 256
+// multiplies A slice i by several B slices: A is read from shared memory once per 256 columns.
+
+constexpr int OZ_FMAX = 256;  // fields of one launch (their selection is kept in shared memory)
+
+template <int DF> struct OzCfg;  // 0: complex128 in and out; 1: double-float complex in, complex64 out
+template <> struct OzCfg<0> {
+  typedef double2 VI;
+  typedef double2 VO;
+  static constexpr int NG = 8, BIAS = 1084, EMAX = 0x7ff;
+};
+template <> struct OzCfg<1> {
+  typedef float4 VI;  // re.hi, re.lo, im.hi, im.lo
+  typedef float2 VO;
+  static constexpr int NG = 7, BIAS = 188, EMAX = 0xff;
+};
+
+// Biased exponents and fixed point of one real number: x = v 2^(emax - BIAS), |v| < 2^62
+WBG_D int oz_exp(double x) { return (int)((unsigned)__double2hiint(x) >> 20) & 0x7ff; }
+WBG_D int oz_exp(float x) { return (int)(__float_as_uint(x) >> 23) & 0xff; }
+WBG_D long long oz_fix(double x, int emax) {
+  const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+  const int e = (int)(u >> 52) & 0x7ff;
+  const int s = emax - e;
+  if (e == 0 || s > 62) return 0;  // zero, subnormal, or below the last digit
+  const long long v = (long long)((((u & 0xfffffffffffffull) | 0x10000000000000ull) << 9) >> s);
+  return (long long)u < 0 ? -v : v;
+}
+WBG_D long long oz_fix(float x, int emax) {
+  const uint32_t u = __float_as_uint(x);
+  const int e = (int)(u >> 23) & 0xff;
+  const int s = emax - e;
+  if (e == 0 || s > 62) return 0;
+  const long long v = (long long)(((unsigned long long)((u & 0x7fffffu) | 0x800000u) << 38) >> s);
+  return (int)u < 0 ? -v : v;
+}
+WBG_D int oz_cexp(double2 a) { return max(oz_exp(a.x), oz_exp(a.y)); }
+WBG_D int oz_cexp(float4 a) { return max(oz_exp(a.x), oz_exp(a.z)); }
+WBG_D long long oz_re(double2 a, int emax) { return oz_fix(a.x, emax); }
+WBG_D long long oz_im(double2 a, int emax) { return oz_fix(a.y, emax); }
+WBG_D long long oz_re(float4 a, int emax) { return oz_fix(a.x, emax) + oz_fix(a.y, emax); }
+WBG_D long long oz_im(float4 a, int emax) { return oz_fix(a.z, emax) + oz_fix(a.w, emax); }
+WBG_D double2 oz_zero(double2) { return make_double2(0.0, 0.0); }
+WBG_D float4 oz_zero(float4) { return make_float4(0.f, 0.f, 0.f, 0.f); }
+WBG_D double2 oz_real(double2 a) { return make_double2(a.x, 0.0); }
+WBG_D float4 oz_real(float4 a) { return make_float4(a.x, a.y, 0.f, 0.f); }
+
+// q 2^E rounded to nearest even, in integer arithmetic (the FP64 pipe converts 64 times slower)
+WBG_D double oz_to_double(long long q, int E) {
+  if (q == 0) return 0.0;
+  const unsigned long long a = q < 0 ? 0ull - (unsigned long long)q : (unsigned long long)q;
+  const int lz = __clzll((long long)a);
+  const unsigned long long m = a << lz;
+  unsigned long long r = m >> 11;
+  const unsigned rem = (unsigned)m & 0x7ffu;
+  r += (rem + ((unsigned)r & 1u)) > 0x400u ? 1u : 0u;
+  const int be = E - lz + 11 + 52 + 1023;  // biased exponent
+  unsigned long long bits;
+  if (be <= 0) bits = 0;                                    // below the normal range
+  else if (be >= 2047) bits = 0x7ff0000000000000ull;
+  else bits = ((unsigned long long)(be - 1) << 52) + r;     // r's leading bit adds the one
+  return __longlong_as_double((long long)(bits | (q < 0 ? 0x8000000000000000ull : 0ull)));
+}
+WBG_D float oz_to_float(long long q, int E) {
+  const float f = __ll2float_rn(q);
+  const int a = max(-126, min(127, E / 2)), b = max(-126, min(127, E - a));  // two exact steps
+  return f * __uint_as_float((uint32_t)(a + 127) << 23) * __uint_as_float((uint32_t)(b + 127) << 23);
+}
+WBG_D double2 oz_pack(double2, long long re, long long im, int E) {
+  return make_double2(oz_to_double(re, E), oz_to_double(im, E));
+}
+WBG_D float2 oz_pack(float2, long long re, long long im, int E) {
+  return make_float2(oz_to_float(re, E), oz_to_float(im, E));
+}
+WBG_D double2 oz_nan(double2) { const double q = __longlong_as_double(0x7ff8000000000000ll); return make_double2(q, q); }
+WBG_D float2 oz_nan(float2) { const float q = __int_as_float(0x7fc00000); return make_float2(q, q); }
+
+// Digits of byte `idx` (3 most significant) of two biased words as fp16 pair: 1024 + byte - 1152
+WBG_D uint32_t oz_dig2(uint32_t a, uint32_t b, int idx) {
+  const uint32_t sel = (uint32_t)idx * 0x0011u | (uint32_t)(4 + idx) * 0x1100u;
+  const uint32_t p = (__byte_perm(a, b, sel) & 0x00ff00ffu) | 0x64006400u;
+  const uint32_t c = 0x64806480u;
+  const __half2 d = __hsub2(*reinterpret_cast<const __half2*>(&p), *reinterpret_cast<const __half2*>(&c));
+  return *reinterpret_cast<const uint32_t*>(&d);
+}
+WBG_D unsigned long long oz_bias(long long v) { return (unsigned long long)v + 0x8080808080808080ull; }
+WBG_D uint32_t oz_word(unsigned long long w, int slice) { return slice < 4 ? (uint32_t)(w >> 32) : (uint32_t)w; }
+
+// Byte offset of the 16-byte chunk c (8 fp16 along K) of operand row r (2 KP bytes, swizzled)
+template <int KP> WBG_D uint32_t oz_off(int r, int c) {
+  if (KP == 64) return (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4));
+  if (KP == 32) return (uint32_t)(r * 64 + ((c ^ ((r >> 1) & 3)) << 4));
+  return (uint32_t)(r * 32 + ((c ^ ((r >> 2) & 1)) << 4));
+}
+// Shared-memory descriptor of a swizzled K-major operand: SBO = 8 rows, version 1, swizzle 128 / 64 / 32 B
+template <int KP> WBG_D uint64_t oz_desc(uint32_t saddr) {
+  return (uint64_t)((saddr & 0x3FFFF) >> 4) | (1ull << 16) | ((uint64_t)(8 * KP * 2 / 16) << 32) | (1ull << 46) |
+         ((KP == 64 ? 2ull : KP == 32 ? 4ull : 6ull) << 61);
+}
+WBG_D void mma_f16(uint32_t dtmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(dtmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
+}
+
+// Every slice product with i + j < NG of one K chunk: accumulators g at d + g ncol.
+template <int KP, int NG>
+WBG_D void oz_issue(uint32_t d, uint32_t a, uint32_t b, int ncol, int ksteps, uint32_t accumulate) {
+  const uint32_t astride = 128 * KP * 2, bstride = (uint32_t)ncol * KP * 2;
+  const int per = 256 / ncol;  // B slices per instruction
+  for (int ks = 0; ks < ksteps; ++ks) {
+    for (int i = 0; i < NG; ++i) {
+      for (int j = 0; j < NG - i; j += per) {
+        const int n = min(per, NG - i - j) * ncol;
+        // D f32 (bits 4-5 = 1), A and B f16, both K-major, N >> 3 at bits 17-22, M >> 4 at 24-28
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
+        mma_f16(d + (uint32_t)((i + j) * ncol), oz_desc<KP>(a + i * astride + ks * 32),
+                oz_desc<KP>(b + j * bstride + ks * 32), idesc, accumulate | (uint32_t)(ks > 0 || i > 0));
+      }
+    }
+  }
+}
+
+// 8 fixed-point values along K as one 16-byte chunk of each of NS slices
+template <int NS> WBG_D void oz_put8(unsigned char* base, uint32_t stride, uint32_t off, const long long (&v)[8]) {
+  unsigned long long w[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) w[q] = oz_bias(v[q]);
+#pragma unroll
+  for (int i = 0; i < NS; ++i) {
+    uint4 o;
+    o.x = oz_dig2(oz_word(w[0], i), oz_word(w[1], i), 3 - (i & 3));
+    o.y = oz_dig2(oz_word(w[2], i), oz_word(w[3], i), 3 - (i & 3));
+    o.z = oz_dig2(oz_word(w[4], i), oz_word(w[5], i), 3 - (i & 3));
+    o.w = oz_dig2(oz_word(w[6], i), oz_word(w[7], i), 3 - (i & 3));
+    *reinterpret_cast<uint4*>(base + i * stride + off) = o;
+  }
+}
+// 4 values along K (half a chunk) to two places, the second one with the sign `flip` applied
+template <int NS>
+WBG_D void oz_put4x2(unsigned char* base, uint32_t stride, uint32_t off0, uint32_t off1, uint32_t flip,
+                     const long long (&v)[4]) {
+  unsigned long long w[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) w[q] = oz_bias(v[q]);
+#pragma unroll
+  for (int i = 0; i < NS; ++i) {
+    uint2 o;
+    o.x = oz_dig2(oz_word(w[0], i), oz_word(w[1], i), 3 - (i & 3));
+    o.y = oz_dig2(oz_word(w[2], i), oz_word(w[3], i), 3 - (i & 3));
+    *reinterpret_cast<uint2*>(base + i * stride + off0) = o;
+    *reinterpret_cast<uint2*>(base + i * stride + off1) = make_uint2(o.x ^ flip, o.y ^ flip);
+  }
+}
+
+// 2 values along K (a quarter chunk) to two places, the second one with the sign `flip` applied
+template <int NS>
+WBG_D void oz_put2x2(unsigned char* base, uint32_t stride, uint32_t off0, uint32_t off1, uint32_t flip, long long a,
+                     long long b) {
+  const unsigned long long wa = oz_bias(a), wb = oz_bias(b);
+#pragma unroll
+  for (int i = 0; i < NS; ++i) {
+    const uint32_t d = oz_dig2(oz_word(wa, i), oz_word(wb, i), 3 - (i & 3));
+    *reinterpret_cast<uint32_t*>(base + i * stride + off0) = d;
+    *reinterpret_cast<uint32_t*>(base + i * stride + off1) = d ^ flip;
+  }
+}
+
+WBG_D void tmem_ld4(uint32_t taddr, uint32_t* r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(taddr));
+}
+// exact integer of an accumulator: |x| <= 2^22 by one addition (its low bits then hold the integer),
+// any |x| < 2^24 by the conversion unit, which runs at a quarter of the rate
+WBG_D int oz_int_small(uint32_t r) { return __float_as_int(__uint_as_float(r) + 12582912.f) - 0x4B400000; }
+WBG_D int oz_int(uint32_t r) { return __float2int_rn(__uint_as_float(r)); }
+// 4 result columns of this thread's row: sum_g acc_g 2^(8 (NG - 1 - g)) >> sh, rounded.  KMAX bounds
+// the contraction: group g sums at most g + 1 pairs, two of them with a leading digit (<= 64).
+template <int NG, int KMAX> WBG_D void oz_cols4(uint32_t taddr, int ncol, int sh, long long* q) {
+  uint32_t r[NG][4];
+#pragma unroll
+  for (int g = 0; g < NG; ++g) tmem_ld4(taddr + (uint32_t)(g * ncol), r[g]);
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int g = 0; g < NG; ++g) asm volatile("" : "+r"(r[g][0]), "+r"(r[g][1]), "+r"(r[g][2]), "+r"(r[g][3])::"memory");
+  constexpr int W = 8 * (NG - 4);  // bits below hi
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    long long hi, lo;
+    if (KMAX <= 64) {  // |acc_0..3| < 2^22, every pair below fits 32 bits
+      const int t1 = oz_int_small(r[0][c]) * 256 + oz_int_small(r[1][c]);
+      const int t2 = oz_int_small(r[2][c]) * 256 + oz_int_small(r[3][c]);
+      const int t3 = oz_int(r[4][c]) * 256 + oz_int(r[5][c]);
+      hi = (long long)t1 * 65536 + t2;
+      if (NG == 8) lo = (long long)t3 * 65536 + (oz_int(r[6][c]) * 256 + oz_int(r[NG - 1][c]));
+      else lo = (long long)t3 * 256 + oz_int(r[6][c]);
+    } else {
+      const int t1 = oz_int_small(r[0][c]) * 256 + oz_int_small(r[1][c]);
+      hi = (long long)t1 * 65536 + ((long long)oz_int(r[2][c]) * 256 + oz_int(r[3][c]));
+      lo = (long long)oz_int(r[4][c]) * 256 + oz_int(r[5][c]);
+      if (NG == 8) lo = lo * 65536 + ((long long)oz_int(r[6][c]) * 256 + oz_int(r[NG - 1][c]));
+      else lo = lo * 256 + oz_int(r[6][c]);
+    }
+    q[c] = (hi << (W - sh)) + ((lo + (1ll << (sh - 1))) >> sh);
+  }
+}
+
+// left shift that brings values whose magnitudes have the largest high word hw just below 2^62
+WBG_D int oz_norm(int hw) { return hw == 0 ? 30 : max(0, __clz(hw) - 2); }
+WBG_D int warp_max(int v) { return __reduce_max_sync(0xffffffffu, v); }
+
+// ---------------------------------------------------------------------------------------
+// nw <= 32: the fields of one k-point stack along M as in rotate_tc_kernel (FPT fields of nw rows
+// in a 128-row tile), both GEMMs share the embedded U.  KP = 16 (nw <= 8), 32 (nw <= 16) or 64 fp16
+// of K; 8 KP threads a CTA and 64 / KP CTAs an SM (512 tensor memory columns in all).
+// ---------------------------------------------------------------------------------------
+template <int KP> constexpr int oz_small_smem() { return 8 * 128 * KP * 2 + 8 * KP * KP * 2 + 1024; }
+
+template <int KP>
+__global__ void __launch_bounds__(8 * KP, 64 / KP)
+    rotate_oz_small(const double2* __restrict__ U, long long strideU, const double2* __restrict__ X, int nFin,
+                    const int* __restrict__ fsel, const int* __restrict__ herm, int nFrot, double2* __restrict__ Xbar,
+                    int nw, int nk, int fpt, int ntiles, int ldf) {
+  typedef OzCfg<0> Cfg;
+  constexpr int NG = Cfg::NG, THR = 8 * KP, NCG = THR / 128;
+  constexpr int SH = KP == 64 ? 12 : KP == 32 ? 11 : 10;  // K <= KP: |sum| <= 2^(68 + log2 KP)
+  constexpr int EP = SH + 112 - 8 * (NG - 1);
+  constexpr uint32_t ASTR = 128 * KP * 2;
+  constexpr uint32_t COLS = 8 * KP;
+  extern __shared__ __align__(1024) unsigned char smo[];
+  unsigned char* As = smo + ((1024u - (smem_u32(smo) & 1023u)) & 1023u);
+  unsigned char* Bs = As + NG * ASTR;
+  __shared__ __align__(8) uint64_t mbar;
+  __shared__ uint32_t tmem_base_s;
+  __shared__ int abort_s, ue_s;
+  __shared__ int code_s[OZ_FMAX];  // per field: -1 invalid selection, else source | herm << 28
+  __shared__ int fe_s[128], qm_s[128];  // per field of the tile: largest exponent of X, high word of max |T|
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t mb = smem_u32(&mbar);
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mb) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    abort_s = 0;
+    ue_s = 1;
+  }
+  if (tid < 128) {
+    fe_s[tid] = 1;
+    qm_s[tid] = 0;
+  }
+  for (int f = tid; f < nFrot; f += THR) {
+    const int fs = fsel[f];
+    code_s[f] = fs >= 0 && fs < nFin ? fs | (herm[f] & 7) << 28 : -1;
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)),
+                 "r"(COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tbase = tmem_base_s;
+  const int nwp = (nw + 7) & ~7, ncol = 2 * nwp, cpr = nwp / 8, nw2 = nw * nw;
+  const int quarter = warp & 3;
+  const int row = 32 * quarter + lane;  // operand / accumulator row of this thread
+  const int ncg = ncol / NCG;           // accumulator columns of this thread: c0 .. c0 + ncg - 1
+  const int c0 = (warp >> 2) * ncg;
+  const uint32_t lane_base = (uint32_t)(32 * quarter) << 16;
+  const uint32_t bstr = (uint32_t)ncol * KP * 2;
+  const int ldst = nwp + 1;  // staging: [row][m'] re plane, then im plane
+  long long* stre = reinterpret_cast<long long*>(As);
+  long long* stim = stre + 128 * ldst;
+  const unsigned long long wait_ns = g_tc_wait_ns;
+  uint32_t phase = 0;
+  // task of the X loads: 8 columns n0.. of row r; 8 lanes take 8 rows (16-byte stores: no conflicts).
+  // The values stay as loaded until their use, so that a prefetch does not wait for them.
+  const int xrow = (tid / (8 * cpr)) * 8 + (tid & 7), xc8 = (tid >> 3) % cpr;
+  const int xfl = xrow / nw, xm = xrow - xfl * nw;
+  const uint32_t magic = 0xffffffffu / (uint32_t)nw + 1;  // r / nw = umulhi(r, magic) for r nw < 2^32
+  double2 xr[8];
+  auto load_x = [&](long long k, int t) {
+    const int f0 = t * fpt, rows = min(fpt, nFrot - f0) * nw;
+    const int code = xrow < rows ? code_s[f0 + xfl] : -1;
+    const double2* src = X + (k * nFin + (code & 0xfffffff)) * (long long)nw2;
+    const bool lower = (code >> 30) & 1;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const int n = 8 * xc8 + c;
+      xr[c] = code >= 0 && n < nw ? src[lower && n > xm ? n * nw + xm : xm * nw + n] : make_double2(0.0, 0.0);
+    }
+  };
+  if (blockIdx.x < nk) load_x(blockIdx.x, 0);
+  for (long long k = blockIdx.x; k < nk && !abort_s; k += gridDim.x) {
+    // ---- embedded U_k (B operand): 4 rows j of one column n per thread
+    const double2* Uk = U + k * strideU;
+    {
+      const int n = tid % nwp, j0 = (tid / nwp) * 4;
+      double2 u[4];
+      int e = 1;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const bool ok = n < nw && j0 + c < nw;
+        u[c] = ok ? Uk[(j0 + c) * nw + n] : make_double2(0.0, 0.0);
+        e = max(e, oz_cexp(u[c]));
+      }
+      e = warp_max(e);
+      if (lane == 0) atomicMax(&ue_s, e);
+      __syncthreads();
+      if (j0 < nwp) {
+        const int eu = ue_s;
+        long long v[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) v[c] = oz_re(u[c], eu);
+        const int cr = j0 >> 3, ci = (nwp + j0) >> 3;  // chunks of K = j and K = nwp + j
+        const uint32_t h = (j0 & 4) << 1;              // second half of the chunk: + 8 bytes
+        oz_put4x2<NG>(Bs, bstr, oz_off<KP>(n, cr) + h, oz_off<KP>(nwp + n, ci) + h, 0u, v);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) v[c] = oz_im(u[c], eu);
+        oz_put4x2<NG>(Bs, bstr, oz_off<KP>(nwp + n, cr) + h, oz_off<KP>(n, ci) + h, 0x80008000u, v);
+      }
+    }
+    const int eu = ue_s;
+    for (int t = 0; t < ntiles; ++t) {
+      const int f0 = t * fpt, nfl = min(fpt, nFrot - f0), rows = nfl * nw;
+      // ---- A1: rows (fl, m), K = [Re X[m][:] | Im X[m][:]]
+      const bool xlow = xrow < rows && ((code_s[f0 + xfl] >> 30) & 1);
+      if (xrow < rows) {
+        int e = 1;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          if (xlow && 8 * xc8 + c == xm) xr[c].y = 0.0;  // a mirrored field's diagonal is real
+          e = max(e, oz_cexp(xr[c]));
+        }
+        atomicMax(&fe_s[xfl], e);
+      }
+      __syncthreads();
+      if (xrow < 128) {
+        const int ex = xrow < rows ? fe_s[xfl] : 1;
+        long long v[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) v[c] = oz_re(xr[c], ex);
+        oz_put8<NG>(As, ASTR, oz_off<KP>(xrow, xc8), v);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          v[c] = oz_im(xr[c], ex);
+          if (xlow && 8 * xc8 + c > xm) v[c] = -v[c];
+        }
+        oz_put8<NG>(As, ASTR, oz_off<KP>(xrow, cpr + xc8), v);
+      }
+      fence_async_smem();
+      __syncthreads();
+      if (tid == 0) {
+        tc_fence_after();
+        oz_issue<KP, NG>(tbase, smem_u32(As), smem_u32(Bs), ncol, ncol / 16, 0u);
+        mma_commit(mb);
+      }
+      if (!wait_all(mb, phase, &abort_s, wait_ns)) break;
+      phase ^= 1;
+      tc_fence_after();
+      // ---- T in fixed point: thread (field, m) holds columns c0.. of [Re T[m][:] | Im T[m][:]]
+      const bool live = 32 * quarter < rows;  // warp-uniform: some row of this warp is in use
+      const int fl = row < rows ? row / nw : 0, m = row - fl * nw;
+      long long q[16];
+      if (live) {
+        int hm = 0;
+#pragma unroll
+        for (int c = 0; c < 16; c += 4) {
+          if (c < ncg) {
+            oz_cols4<NG, KP>(tbase + lane_base + c0 + c, ncol, SH, q + c);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) hm = max(hm, (int)((q[c + i] ^ (q[c + i] >> 63)) >> 32));
+          }
+        }
+        if (row < rows) atomicMax(&qm_s[fl], hm);
+      }
+      __syncthreads();
+      const int nsh = oz_norm(qm_s[fl]);
+      if (live) {  // ---- A2: row (fl, n), K = m: [Re T[m][n] | -Im T[m][n]]
+        const bool even = (nw & 1) == 0;  // rows 2 i, 2 i + 1 belong to one field: exchanged for 4-byte stores
+#pragma unroll
+        for (int c = 0; c < 16; c += 2) {
+          const bool im = c0 + c >= nwp;
+          const int n = c0 + c - (im ? nwp : 0), kk = (im ? nwp : 0) + m;
+          if (c >= ncg || n >= nw) continue;  // warp-uniform
+          long long a = q[c] << nsh, b = q[c + 1] << nsh;
+          if (im) {
+            a = -a;
+            b = -b;
+          }
+          const int r0 = fl * nw + n;
+          if (even) {  // even lanes take column n of rows m, m + 1, odd lanes column n + 1 of rows m - 1, m
+            const bool odd = lane & 1;
+            const long long o = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
+            const unsigned long long wa = oz_bias(odd ? o : a), wb = oz_bias(odd ? b : o);
+            unsigned char* d0 = As + oz_off<KP>(r0 + odd, kk >> 3) + (kk & 6) * 2;
+            if (row < rows) {
+#pragma unroll
+              for (int i = 0; i < NG; ++i)
+                *reinterpret_cast<uint32_t*>(d0 + i * ASTR) = oz_dig2(oz_word(wa, i), oz_word(wb, i), 3 - (i & 3));
+            }
+          } else if (row < rows) {
+            const unsigned long long wa = oz_bias(a), wb = oz_bias(b);
+            unsigned char* d0 = As + oz_off<KP>(r0, kk >> 3) + (kk & 7) * 2;
+            unsigned char* d1 = As + oz_off<KP>(r0 + 1, kk >> 3) + (kk & 7) * 2;
+#pragma unroll
+            for (int i = 0; i < NG; ++i) {
+              const uint32_t d = oz_dig2(oz_word(wa, i), oz_word(wb, i), 3 - (i & 3));
+              *reinterpret_cast<unsigned short*>(d0 + i * ASTR) = (unsigned short)d;
+              if (n + 1 < nw) *reinterpret_cast<unsigned short*>(d1 + i * ASTR) = (unsigned short)(d >> 16);
+            }
+          }
+        }
+      }
+      tc_fence_before();
+      fence_async_smem();
+      __syncthreads();
+      if (tid == 0) {
+        tc_fence_after();
+        oz_issue<KP, NG>(tbase, smem_u32(As), smem_u32(Bs), ncol, ncol / 16, 0u);
+        mma_commit(mb);
+      }
+      {  // the next tile's X while the products run
+        const bool last = t + 1 == ntiles;
+        const long long kn = last ? k + gridDim.x : k;
+        if (kn < nk) {
+          if (last && tid < (nw2 + 7) / 8) prefetch_l2(U + kn * strideU + tid * 8);
+          load_x(kn, last ? 0 : t + 1);
+        }
+      }
+      if (!wait_all(mb, phase, &abort_s, wait_ns)) break;
+      phase ^= 1;
+      tc_fence_after();
+      // ---- D2: thread (fl, n) holds columns c0.. of [Re Y^H[n][:] | Im Y^H[n][:]]; staged, then written
+      if (live) {
+#pragma unroll
+        for (int c = 0; c < 16; c += 4) {
+          if (c < ncg) {
+            long long s[4];
+            oz_cols4<NG, KP>(tbase + lane_base + c0 + c, ncol, SH, s);
+            const bool im = c0 + c >= nwp;
+            long long* p = (im ? stim - nwp : stre) + row * ldst + c0 + c;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) p[i] = s[i];
+          }
+        }
+      }
+      tc_fence_before();
+      __syncthreads();
+#pragma unroll 2
+      for (int e = tid; e < rows * nw; e += THR) {
+        const int r = (int)__umulhi((uint32_t)e, magic), n = e - r * nw;  // row (field, m') and column n
+        const int f = (int)__umulhi((uint32_t)r, magic), mr = r - f * nw;
+        const int code = code_s[f0 + f], hmode = (code >> 28) & 3;
+        const bool bad = code < 0 || fe_s[f] >= Cfg::EMAX || eu >= Cfg::EMAX;
+        if (code >= 0 && hmode == 2 && n != mr) continue;
+        const int E = 2 * EP - oz_norm(qm_s[f]) + fe_s[f] + 2 * eu - 3 * Cfg::BIAS;
+        const int o = (f * nw + n) * ldst + mr;  // Y[m'][n] = conj(Y^H[n][m'])
+        long long re = stre[o], im = -stim[o];
+        if (hmode != 0) {  // + Y^H[m'][n], halved in the exponent
+          const int p = r * ldst + n;
+          re += stre[p];
+          im += stim[p];
+        }
+        Xbar[(k * ldf + f0 + f) * (long long)nw2 + mr * nw + n] =
+            bad ? oz_nan(double2()) : oz_pack(double2(), re, im, hmode != 0 ? E - 1 : E);
+      }
+      __syncthreads();  // TMEM, the operands and the staging are free
+      if (tid < 128) {
+        fe_s[tid] = 1;
+        qm_s[tid] = 0;
+      }
+      if (tid == 0 && t + 1 == ntiles) ue_s = 1;
+      __syncthreads();
+    }
+  }
+  if (abort_s) {  // a wait ran out: let the products already issued finish first
+    if (tid == 0) mbar_wait(mb, phase, DRAIN_NS);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(COLS) : "memory");
+  }
+}
+
+// ---------------------------------------------------------------------------------------
+// 32 < nw <= 128: one field and one panel of PN = 32 columns at a time.
+//   GEMM1  T = X U_P        A = [Re X | Im X] rows m       B = embedded U[:, P]
+//   GEMM2  Y = U^dagger T   A = [Re U^T | Im U^T] rows m'  B = [[Re T, Im T], [Im T, -Re T]]
+// K runs in chunks of 32 complex rows; T stays in registers (fixed point) between the GEMMs, and
+// the warps of TMEM lane quarter c write chunk c of it as operand.  Rows >= nw of A are left as they
+// are: they reach only accumulator rows that nothing reads.  Hermitian-part fields take the
+// Hermitian part on input and write the lower triangle with its mirror, as rotate_panel does, so
+// that the stored matrix is Hermitian bit for bit.
+// ---------------------------------------------------------------------------------------
+constexpr int OZ_PN = 32, OZ_THR = 512;
+template <int DF> constexpr int oz_large_smem() { return OzCfg<DF>::NG * (128 + 64) * 128 + 1024; }
+
+template <int DF>
+__global__ void __launch_bounds__(OZ_THR, 1)
+    rotate_oz_large(const typename OzCfg<DF>::VI* __restrict__ U, long long strideU,
+                    const typename OzCfg<DF>::VI* __restrict__ X, int nFin, const int* __restrict__ fsel,
+                    const int* __restrict__ herm, int nFrot, typename OzCfg<DF>::VO* __restrict__ Xbar, int nw, int nk,
+                    long long per) {
+  typedef OzCfg<DF> Cfg;
+  typedef typename Cfg::VI VI;
+  typedef typename Cfg::VO VO;
+  constexpr int NG = Cfg::NG, KP = 64;
+  constexpr int SH = DF ? 6 : 14;  // K <= 256: |sum| <= 2^76 (FP64), 2^68 (double-float)
+  constexpr int EP = SH + 112 - 8 * (NG - 1);
+  constexpr uint32_t ASTR = 128 * 128, BSTR = 64 * 128;
+  constexpr int LDS = OZ_PN + 1;
+  extern __shared__ __align__(1024) unsigned char smo[];
+  unsigned char* As = smo + ((1024u - (smem_u32(smo) & 1023u)) & 1023u);
+  unsigned char* Bs = As + NG * ASTR;
+  long long* stre = reinterpret_cast<long long*>(As);  // staging: [m'][n] re plane, then im plane
+  long long* stim = stre + 128 * LDS;
+  __shared__ __align__(8) uint64_t mbar;
+  __shared__ uint32_t tmem_base_s;
+  __shared__ int abort_s, ue_s, fe_s, qm_s;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t mb = smem_u32(&mbar);
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mb) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    abort_s = 0;
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)),
+                 "r"(512)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tbase = tmem_base_s;
+  const int nw2 = nw * nw, np = (nw + OZ_PN - 1) / OZ_PN, nch = (nw + 31) / 32;
+  const int quarter = warp & 3, half = warp >> 3, sub = (warp >> 2) & 1;  // columns 32 half + 16 sub ..
+  const uint32_t lane_base = ((uint32_t)(32 * quarter) << 16) + 32 * half + 16 * sub;
+  const int row = 32 * quarter + lane;
+  const unsigned long long wait_ns = g_tc_wait_ns;
+  uint32_t phase = 0;
+  long long kprev = -1, fprev = -1;
+  const long long total = (long long)nk * nFrot * np;
+  const long long u1 = min(total, (blockIdx.x + 1) * per);
+  // task of the A loads: 8 columns of one row; 8 lanes take 8 rows
+  const int am = (tid >> 5) * 8 + (tid & 7), ac8 = (tid >> 3) & 3;
+  VI xr[8];
+  for (long long u = blockIdx.x * per; u < u1 && !abort_s; ++u) {
+    const int P = (int)(u % np), f = (int)((u / np) % nFrot);
+    const long long k = u / ((long long)np * nFrot);
+    const int fs = fsel[f], hm = herm[f];
+    const bool fok = fs >= 0 && fs < nFin;  // selection lives in device memory: validate here
+    const int inmode = (hm & 4) ? 2 : ((hm & 3) != 0 ? 1 : 0);
+    const VI* Xf = X + (k * nFin + (fok ? fs : 0)) * (long long)nw2;
+    const VI* Uk = U + k * strideU;
+    const int n0 = P * OZ_PN;
+    // ---- largest exponents of U_k and of the field (kept while the CTA stays on them)
+    const bool newk = k != kprev, newf = newk || f != fprev;
+    __syncthreads();
+    if (tid == 0) {
+      if (newk) ue_s = 1;
+      if (newf) fe_s = 1;
+      qm_s = 0;
+    }
+    __syncthreads();
+    if (newk) {
+      int e = 1;
+#pragma unroll 4
+      for (int i = tid; i < nw2; i += OZ_THR) e = max(e, oz_cexp(Uk[i]));
+      e = warp_max(e);
+      if (lane == 0) atomicMax(&ue_s, e);
+    }
+    if (newf) {
+      int e = 1;
+#pragma unroll 4
+      for (int i = tid; i < nw2; i += OZ_THR) {
+        const VI v = Xf[i];  // of a lower-triangle field only m >= n counts, of its diagonal the real part
+        const int m = i / nw, n = i - m * nw;
+        if (inmode != 2 || m >= n) e = max(e, oz_cexp(inmode == 2 && m == n ? oz_real(v) : v));
+      }
+      e = warp_max(e);
+      if (lane == 0) atomicMax(&fe_s, e);
+    }
+    kprev = k;
+    fprev = f;
+    auto load_x = [&](int c) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int j = 32 * c + 8 * ac8 + q;
+        xr[q] = oz_zero(VI());
+        if (am < nw && j < nw) {
+          xr[q] = Xf[inmode == 2 && j > am ? j * nw + am : am * nw + j];
+        }
+      }
+    };
+    auto load_uh = [&](int c) {  // row m' of U^H: U[j][m']
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int j = 32 * c + 8 * ac8 + q;
+        xr[q] = am < nw && j < nw ? Uk[j * nw + am] : oz_zero(VI());
+      }
+    };
+    load_x(0);
+    __syncthreads();
+    const int eu = ue_s, ex = fe_s;
+    // ---- GEMM1
+    for (int c = 0; c < nch; ++c) {
+      if (am < nw) {
+        long long v[8];
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {  // re, im
+#pragma unroll
+          for (int q = 0; q < 8; ++q) v[q] = p ? oz_im(xr[q], ex) : oz_re(xr[q], ex);
+          if (inmode == 2 && p) {  // the mirror's conjugate, the real diagonal
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+              const int j = 32 * c + 8 * ac8 + q;
+              v[q] = j > am ? -v[q] : j == am ? 0 : v[q];
+            }
+          }
+          if (inmode == 1) {  // Hermitian part of the input
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+              const int j = 32 * c + 8 * ac8 + q;
+              if (j < nw) {
+                const VI b = Xf[j * nw + am];
+                v[q] = (p ? v[q] - oz_im(b, ex) : v[q] + oz_re(b, ex)) >> 1;
+              }
+            }
+          }
+          oz_put8<NG>(As, ASTR, oz_off<KP>(am, 4 * p + ac8), v);
+        }
+      }
+      {  // embedded U[:, P]: 2 rows j of one column
+        const int jl = warp * 2, j = 32 * c + jl;
+        const bool nok = n0 + lane < nw;
+        const VI a = nok && j < nw ? Uk[j * nw + n0 + lane] : oz_zero(VI());
+        const VI b = nok && j + 1 < nw ? Uk[(j + 1) * nw + n0 + lane] : oz_zero(VI());
+        const int cr = jl >> 3;
+        const uint32_t h = (jl & 7) * 2;
+        oz_put2x2<NG>(Bs, BSTR, oz_off<KP>(lane, cr) + h, oz_off<KP>(32 + lane, 4 + cr) + h, 0u, oz_re(a, eu),
+                      oz_re(b, eu));
+        oz_put2x2<NG>(Bs, BSTR, oz_off<KP>(32 + lane, cr) + h, oz_off<KP>(lane, 4 + cr) + h, 0x80008000u,
+                      oz_im(a, eu), oz_im(b, eu));
+      }
+      fence_async_smem();
+      __syncthreads();
+      if (tid == 0) {
+        tc_fence_after();
+        oz_issue<KP, NG>(tbase, smem_u32(As), smem_u32(Bs), 64, 4, (uint32_t)(c > 0));
+        mma_commit(mb);
+      }
+      if (c + 1 < nch) load_x(c + 1);
+      else load_uh(0);
+      if (!wait_all(mb, phase, &abort_s, wait_ns)) break;
+      phase ^= 1;
+      tc_fence_after();
+    }
+    if (abort_s) break;
+    // ---- T: thread (row j) holds 16 columns n of Re (half 0) or Im (half 1) T[j][n0 + 16 sub ..]
+    long long q[16];
+    const bool live = 32 * quarter < nw;
+    if (live) {
+      int hmx = 0;
+#pragma unroll
+      for (int c = 0; c < 16; c += 4) {
+        oz_cols4<NG, 256>(tbase + lane_base + c, 64, SH, q + c);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if (row >= nw) q[c + i] = 0;
+          hmx = max(hmx, (int)((q[c + i] ^ (q[c + i] >> 63)) >> 32));
+        }
+      }
+      hmx = warp_max(hmx);
+      if (lane == 0) atomicMax(&qm_s, hmx);
+    }
+    tc_fence_before();
+    __syncthreads();
+    const int nsh = oz_norm(qm_s);
+    // ---- GEMM2
+    for (int c = 0; c < nch; ++c) {
+      if (am < nw) {
+        long long v[8];
+#pragma unroll
+        for (int s = 0; s < 8; ++s) v[s] = oz_re(xr[s], eu);
+        oz_put8<NG>(As, ASTR, oz_off<KP>(am, ac8), v);
+#pragma unroll
+        for (int s = 0; s < 8; ++s) v[s] = oz_im(xr[s], eu);
+        oz_put8<NG>(As, ASTR, oz_off<KP>(am, 4 + ac8), v);
+      }
+      if (quarter == c) {  // this quarter's rows j are the chunk's
+        const int k0 = half * 32 + lane, k1 = (1 - half) * 32 + lane;  // K of the n and of the 32 + n rows
+        const uint32_t flip = half ? 0u : 0x80008000u;                 // -Re T at (32 + n, K = 32 + j)
+        const bool odd = lane & 1;  // even lanes write column n of rows j, j + 1, odd lanes column n + 1 of j - 1, j
+        unsigned char* b0 = Bs + (k0 & 6) * 2;
+        unsigned char* b1 = Bs + (k1 & 6) * 2;
+#pragma unroll
+        for (int i = 0; i < 16; i += 2) {
+          const long long a = q[i] << nsh, b = q[i + 1] << nsh;
+          const long long o = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
+          const unsigned long long wa = oz_bias(odd ? o : a), wb = oz_bias(odd ? b : o);
+          const int n = 16 * sub + i + odd;
+          unsigned char* p0 = b0 + oz_off<KP>(n, k0 >> 3);
+          unsigned char* p1 = b1 + oz_off<KP>(32 + n, k1 >> 3);
+#pragma unroll
+          for (int s = 0; s < NG; ++s) {
+            const uint32_t d = oz_dig2(oz_word(wa, s), oz_word(wb, s), 3 - (s & 3));
+            *reinterpret_cast<uint32_t*>(p0 + s * BSTR) = d;
+            *reinterpret_cast<uint32_t*>(p1 + s * BSTR) = d ^ flip;
+          }
+        }
+      }
+      fence_async_smem();
+      __syncthreads();
+      if (tid == 0) {
+        tc_fence_after();
+        oz_issue<KP, NG>(tbase, smem_u32(As), smem_u32(Bs), 64, 4, (uint32_t)(c > 0));
+        mma_commit(mb);
+      }
+      if (c + 1 < nch) load_uh(c + 1);
+      if (!wait_all(mb, phase, &abort_s, wait_ns)) break;
+      phase ^= 1;
+      tc_fence_after();
+    }
+    if (abort_s) break;
+    // ---- Y: thread (row m') holds 16 columns of Re or Im of Y[m'][n0 ..]; staged, then written by rows
+    if (live) {
+#pragma unroll
+      for (int c = 0; c < 16; c += 4) {
+        long long s[4];
+        oz_cols4<NG, 256>(tbase + lane_base + c, 64, SH, s);
+        long long* p = (half ? stim : stre) + row * LDS + 16 * sub + c;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) p[i] = s[i];
+      }
+    }
+    tc_fence_before();
+    __syncthreads();
+    const bool bad = !fok || ex >= Cfg::EMAX || eu >= Cfg::EMAX;
+    const int E = 2 * EP - nsh + ex + 2 * eu - 3 * Cfg::BIAS;
+    VO* dst = Xbar + (k * nFrot + f) * (long long)nw2;
+    const int mode = hm & 3, n = n0 + lane;
+    for (int m = warp; m < nw; m += OZ_THR / 32) {
+      if (n >= nw || (mode != 0 && n > m) || (mode == 2 && n != m)) continue;
+      VO y = oz_pack(VO(), stre[m * LDS + lane], stim[m * LDS + lane], E);
+      if (mode != 0 && m == n) y.y = 0;
+      dst[m * nw + n] = bad ? oz_nan(y) : y;
+    }
+    if (mode == 1) {  // the mirror: row n of the panel, columns m > n
+      for (int nl = warp; nl < OZ_PN && n0 + nl < nw; nl += OZ_THR / 32)
+        for (int m = n0 + nl + 1 + lane; m < nw; m += 32) {
+          const VO y = oz_pack(VO(), stre[m * LDS + nl], -stim[m * LDS + nl], E);
+          dst[(n0 + nl) * nw + m] = bad ? oz_nan(y) : y;
+        }
+    }
+  }
+  if (abort_s) {
+    if (tid == 0) mbar_wait(mb, phase, DRAIN_NS);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(512) : "memory");
+  }
+}

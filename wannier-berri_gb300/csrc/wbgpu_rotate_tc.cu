@@ -20,6 +20,7 @@
 // One thread issues the MMAs; completion is tracked with an mbarrier whose every wait is
 // bounded in time: on timeout the kernel records WBG_DEVICE_FLAG_TC_TIMEOUT in the
 // library's device error word, releases its tensor memory and returns.
+#include <cuda_fp16.h>
 #include "wbgpu_common.cuh"
 #include "wbgpu_band.cuh"
 #include "wbgpu_fixed.cuh"
@@ -1287,6 +1288,8 @@ __global__ void __launch_bounds__(KT_THR, 1)
   }
 }
 
+#include "wbgpu_rotate_oz.cuh"
+
 // A wait that runs out by construction: an mbarrier whose phase never completes, waited on with
 // the kernel's bound; records WBG_DEVICE_FLAG_TC_TIMEOUT exactly as the rotation does.
 __global__ void tc_wait_probe_kernel(int* result) {
@@ -1329,6 +1332,56 @@ int wbg_rotate_tc_run(const void* U, long long strideU, const void* X, int nFin,
   const long long grid = nk < 2ll * sms ? nk : 2ll * sms;
   rotate_tc_kernel<<<(unsigned)grid, NTHR, SMEM_BYTES, stream>>>((const float2*)U, strideU, (const float2*)X, nFin,
                                                                 fsel, herm, nFrot, (float2*)Xbar, nk);
+  return wbg_cuda_status(cudaGetLastError());
+}
+
+// FP64 from nw = 4 (4 096 k-points, 9 fields: 0.086 ms against 0.096 ms for rotate_kernel; 44.8 -> 5.7 ms
+// at nw = 32 and 13 824 k-points), double-float above nw = 32 (nw = 48: 8.1 against 9.9 ms, nw = 96:
+// 5.1 against 27.7 ms; below, the engine rotates in FP32) where the operands allow 16-byte loads.
+bool wbg_rotate_oz_supported(const void* U, const void* X, int nw, int fp64) {
+  if (nw > 128) return false;
+  if (fp64 == 2) return nw > NW && ((reinterpret_cast<uintptr_t>(U) | reinterpret_cast<uintptr_t>(X)) & 15) == 0;
+  return fp64 == 1 && nw >= WBG_OZ_MIN_NW;
+}
+
+int wbg_rotate_oz_run(const void* U, long long strideU, const void* X, int nFin, const int* fsel, const int* herm,
+                      int nFrot, void* Xbar, int nw, int nk, int fp64, cudaStream_t stream) {
+  int dev = 0, sms = 0;
+  if (const cudaError_t e_ = cudaGetDevice(&dev)) return wbg_cuda_status(e_);
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) return WBG_ERR_CUDA;
+  if (nw <= NW) {
+    const int most = TM / nw;  // fields of one 128-row tile; the tiles share the fields evenly
+    const int kp = nw <= 8 ? 16 : nw <= 16 ? 32 : 64;
+    const auto kern = kp == 16 ? rotate_oz_small<16> : kp == 32 ? rotate_oz_small<32> : rotate_oz_small<64>;
+    const int smem = kp == 16 ? oz_small_smem<16>() : kp == 32 ? oz_small_smem<32>() : oz_small_smem<64>();
+    const long long slots = (long long)(64 / kp) * sms, grid = nk < slots ? nk : slots;
+    if (const cudaError_t e_ = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem))
+      return wbg_cuda_status(e_);
+    for (int fb = 0; fb < nFrot; fb += OZ_FMAX) {
+      const int nf = nFrot - fb < OZ_FMAX ? nFrot - fb : OZ_FMAX;
+      const int ntiles = (nf + most - 1) / most, fpt = (nf + ntiles - 1) / ntiles;
+      kern<<<(unsigned)grid, 8 * kp, smem, stream>>>((const double2*)U, strideU, (const double2*)X, nFin, fsel + fb,
+                                                     herm + fb, nf, (double2*)Xbar + (size_t)fb * nw * nw, nw, nk, fpt,
+                                                     (nf + fpt - 1) / fpt, nFrot);
+    }
+    return wbg_cuda_status(cudaGetLastError());
+  }
+  const long long total = (long long)nk * nFrot * ((nw + OZ_PN - 1) / OZ_PN);
+  const long long per = (total + sms - 1) / sms;  // consecutive panels: a CTA stays on a field
+  const unsigned grid = (unsigned)((total + per - 1) / per);
+  if (fp64 == 1) {
+    if (const cudaError_t e_ =
+            cudaFuncSetAttribute(rotate_oz_large<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, oz_large_smem<0>()))
+      return wbg_cuda_status(e_);
+    rotate_oz_large<0><<<grid, OZ_THR, oz_large_smem<0>(), stream>>>((const double2*)U, strideU, (const double2*)X, nFin,
+                                                                     fsel, herm, nFrot, (double2*)Xbar, nw, nk, per);
+  } else {
+    if (const cudaError_t e_ =
+            cudaFuncSetAttribute(rotate_oz_large<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, oz_large_smem<1>()))
+      return wbg_cuda_status(e_);
+    rotate_oz_large<1><<<grid, OZ_THR, oz_large_smem<1>(), stream>>>((const float4*)U, strideU, (const float4*)X, nFin,
+                                                                     fsel, herm, nFrot, (float2*)Xbar, nw, nk, per);
+  }
   return wbg_cuda_status(cudaGetLastError());
 }
 
