@@ -936,6 +936,7 @@ __global__ void berry_scan_kernel(const double* __restrict__ E, const typename C
           }
       } else if (NCM == 27 && formula == WBG_FORMULA_SPIN_OMEGA) {
         KBand<T> kb;
+        kb.pf = nullptr;
         kb.X = Xk;
         kb.E = myE;
         kb.nw = nw;
@@ -1731,17 +1732,47 @@ __global__ void berry_deromega_kernel(const double* __restrict__ E, const VS* __
 }
 
 // cumulative sum over Fermi levels and normalisation: out[ie][c] = scale * sum_{j<=ie} hist[j][c],
-// hist in the fixed-point layout of wbgpu_fixed.cuh; NaN throughout when a contribution was not finite
-__global__ void scan_finalize_kernel(const wbg_u64* __restrict__ hist, int nEF, int ncomp, double scale,
-                                     double* __restrict__ out) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncomp) return;
+// hist in the fixed-point layout of wbgpu_fixed.cuh; NaN throughout when a contribution was not finite.
+// One block per component: every thread adds a run of levels, the block scans the runs, every thread
+// writes its run -- all in the histogram's 128-bit integers, so a level is rounded once whatever the
+// split (a chain of FP64 additions rounds at every level).  Bound by launch latency: 5 us where one
+// thread per component walked 1 001 levels of dependent loads in 360 us.
+constexpr int SCAN_THR = 256;
+WBG_D void add128(wbg_u64& lo, wbg_u64& hi, wbg_u64 l, wbg_u64 h) {
+  const wbg_u64 s = lo + l;
+  hi += h + (s < l ? 1ull : 0ull);
+  lo = s;
+}
+__global__ void __launch_bounds__(SCAN_THR) scan_finalize_kernel(const wbg_u64* __restrict__ hist, int nEF, int ncomp,
+                                                                 double scale, double* __restrict__ out) {
+  __shared__ wbg_u64 tot[SCAN_THR / 32][2];
+  const int c = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool bad = hist[2 * (size_t)nEF * ncomp] != 0ull;
-  double s = 0.0;
-  for (int ie = 0; ie < nEF; ++ie) {
-    const size_t e = (size_t)ie * ncomp + c;
-    s += fx_value(hist[2 * e], hist[2 * e + 1]);
-    out[e] = bad ? nan("") : s * scale;
+  const int run = (nEF + SCAN_THR - 1) / SCAN_THR;
+  const long long i0 = (long long)tid * run, i1 = i0 + run < nEF ? i0 + run : nEF;
+  wbg_u64 lo = 0, hi = 0;
+  for (long long ie = i0; ie < i1; ++ie) add128(lo, hi, hist[2 * (ie * ncomp + c)], hist[2 * (ie * ncomp + c) + 1]);
+  const wbg_u64 lo0 = lo, hi0 = hi;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {  // inclusive scan of the warp's runs
+    const wbg_u64 l = __shfl_up_sync(0xffffffffu, lo, off), h = __shfl_up_sync(0xffffffffu, hi, off);
+    if (lane >= off) add128(lo, hi, l, h);
+  }
+  if (lane == 31) {
+    tot[warp][0] = lo;
+    tot[warp][1] = hi;
+  }
+  __syncthreads();
+  for (int w = 0; w < warp; ++w) add128(lo, hi, tot[w][0], tot[w][1]);
+  add128(lo, hi, ~lo0 + 1ull, ~hi0 + (lo0 == 0 ? 1ull : 0ull));  // exclusive: less the own run
+  for (long long ie = i0; ie < i1; ++ie) {
+    const size_t e = (size_t)(ie * ncomp + c);
+    add128(lo, hi, hist[2 * e], hist[2 * e + 1]);
+    // through the magnitude: of a small negative sum, hi 2^4 and the fraction would cancel
+    const bool neg = (long long)hi < 0;
+    const wbg_u64 ml = neg ? ~lo + 1ull : lo, mh = neg ? ~hi + (lo == 0 ? 1ull : 0ull) : hi;
+    const double v = fx_value(ml, mh);
+    out[e] = bad ? nan("") : (neg ? -v : v) * scale;
   }
 }
 
@@ -2119,6 +2150,6 @@ int wbg_berry_deromega_run(const double* E, const void* Xbar, int nFbar, int iV,
 
 int wbg_scan_finalize_run(const void* hist, int nEF, int ncomp, double scale, double* out, cudaStream_t stream) {
   if (nEF < 1 || ncomp < 1 || !hist || !out) return WBG_ERR_ARG;
-  scan_finalize_kernel<<<(ncomp + 31) / 32, 32, 0, stream>>>((const wbg_u64*)hist, nEF, ncomp, scale, out);
+  scan_finalize_kernel<<<ncomp, SCAN_THR, 0, stream>>>((const wbg_u64*)hist, nEF, ncomp, scale, out);
   return wbg_cuda_status(cudaGetLastError());
 }
