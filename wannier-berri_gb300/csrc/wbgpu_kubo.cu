@@ -22,7 +22,8 @@
 //              FP64 path).
 // kubo_accum:  one thread per frequency, a chunk of levels per block (grid z), a chunk of
 //              k-points per block (grid y): accumulation in shared memory in the records'
-//              precision, fixed-point sums into the result (FP64 path, and JDOS).
+//              precision, fixed-point sums into the result (JDOS).
+// kubo_gemm64: the FP64 path's 9- and 27-component sums as a register-tiled product.
 // kubo_gemm:   the mixed path's 9- and 27-component sums as a register-tiled complex GEMM
 //              (frequencies x (level, component) per k-point, records as the contraction).
 #include <float.h>
@@ -180,6 +181,9 @@ WBG_D void add_element(const KBand<T>& b, int n, int m, typename C2<T>::t* M) {
   }
 }
 
+// doubles of kubo_pairs' energies, group means, borders and flags in shared memory
+__host__ __device__ constexpr size_t pairs_words(int nw) { return 2 * (size_t)nw + ((size_t)(2 * nw + 1) * 4 + 7) / 8; }
+
 // grid: nk blocks of 128 threads.  Records of k-point k occupy slots [k*P, k*P + count[k]).
 template <typename T, int F>
 __global__ void kubo_pairs(const double* __restrict__ E, const typename C2<T>::t* __restrict__ Xbar, int nFbar,
@@ -221,6 +225,16 @@ __global__ void kubo_pairs(const double* __restrict__ E, const typename C2<T>::t
   band.nw = nw;
   band.nw2 = nw2;
   band.f = fs;
+  band.pf = nullptr;
+  if (F == WBG_DYN_SHIFT) {  // nw^2 principal-value factors once, instead of two divisions per pair and band
+    T* pf = reinterpret_cast<T*>(smk + pairs_words(nw));
+    for (int i = threadIdx.x; i < nw * nw; i += blockDim.x) {
+      const double d = Es[i / nw] - Es[i % nw];
+      pf[i] = (T)(-d / (d * d + fs.sc_eta * fs.sc_eta));
+    }
+    band.pf = pf;
+    __syncthreads();
+  }
   const double eocc1max = kp.EFmin - 30.0 * kp.kBT, eocc0min = kp.EFmax + 30.0 * kp.kBT;
   // Records are stored in pair order (slot = number of kept pairs before this one), so the
   // accumulation over them runs in the same order on every run: a block-wide exclusive count of
@@ -482,12 +496,152 @@ __global__ void __launch_bounds__(KG_THR, 1)
     }
 }
 
+// ---------------------------------------------------------------------------------------
+// FP64 path, NC = 9 or 27: the same sums in FP64 as a register-tiled product.  FR: f_w is real
+// (injection, shift current), MR: the elements are real (SHC, shift current) -- the products that are
+// zero by construction are not formed (1, 2 or 4 multiply-adds an output and record).  A block takes
+// K6_TW frequencies x 16 JN columns; sums run over one k-point's records in registers, then over the
+// block's k-points in shared memory, and go to `out` once.  Bound by the FP64 pipe; at 61 frequencies
+// x 3 levels x 27 components, num_wann 12 and 1 680 k-points: 10.8 ms with accumulators read and
+// written in shared memory for every record and flushed per k-point (and four multiply-adds each),
+// now 2.5 ms (the pairs: 1.6 -> 1.4 ms).
+// ---------------------------------------------------------------------------------------
+constexpr int K6_TW = 64, K6_RC = 16, K6_THR = 256;
+template <bool FR, bool MR> struct K6 {
+  static constexpr bool RR = FR && MR;
+  static constexpr int JN = RR ? 8 : 4, TC = 16 * JN;  // columns per thread and per block
+  static constexpr int FW = FR ? 1 : 2, GW = MR ? 1 : 2, AW = RR ? 1 : 2;  // doubles of f, of g, of a sum
+  static constexpr size_t SMEM =
+      8 * ((size_t)4 * JN * AW * K6_THR + (size_t)K6_RC * (K6_TW * FW + TC * GW));
+};
+
+template <int NC, bool FR, bool MR>
+__global__ void __launch_bounds__(K6_THR, 2)
+    kubo_gemm64(const double* __restrict__ rec_dE, const double* __restrict__ rec_fE, const double2* __restrict__ rec_M,
+                const int* __restrict__ count, int P, int nk, int kchunk, const double* __restrict__ omega, WbgKubo kp,
+                int formula, wbg_u64* __restrict__ out) {
+  typedef K6<FR, MR> K;
+  constexpr int JN = K::JN, TC = K::TC, FW = K::FW, GW = K::GW, AW = K::AW;
+  extern __shared__ __align__(16) unsigned char smg[];
+  double* accd = reinterpret_cast<double*>(smg);  // [4 JN AW][K6_THR]
+  double* Fs = accd + 4 * JN * AW * K6_THR;       // [K6_RC][K6_TW][FW]
+  double* Gs = Fs + K6_RC * K6_TW * FW;           // [K6_RC][TC][GW]
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int w0 = blockIdx.x * K6_TW, col0 = blockIdx.z * TC;
+  const int ncol = kp.nEF * NC;
+  const int jn = min(JN, (ncol - col0 + 15) / 16);  // column groups in use
+  const int fgroup = formula >= WBG_DYN_SHC_SIMPLE && formula <= WBG_DYN_SHC_RYOO ? kShcFactor : formula;
+  for (int q = 0; q < 4 * JN * AW; ++q) accd[q * K6_THR + tid] = 0.0;
+  const long long k0 = (long long)blockIdx.y * kchunk;
+  const long long k1 = min((long long)nk, k0 + kchunk);
+  for (long long k = k0; k < k1; ++k) {
+    const int nrec = count[k];
+    if (nrec == 0) continue;
+    const long long rbase = k * (long long)P;
+    double acc[4][JN][AW];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < JN; ++j)
+#pragma unroll
+        for (int a = 0; a < AW; ++a) acc[i][j][a] = 0.0;
+    for (int r0 = 0; r0 < nrec; r0 += K6_RC) {
+      const int rn = min(K6_RC, nrec - r0);
+      __syncthreads();  // the previous chunk's tiles are read
+      for (int idx = tid; idx < rn * K6_TW; idx += K6_THR) {
+        const int r = idx / K6_TW, w = idx % K6_TW;
+        double2 f = make_double2(0.0, 0.0);
+        if (w0 + w < kp.nOmega)
+          f = factor_omega<double>(fgroup, rec_dE[rbase + r0 + r], omega[w0 + w], kp.eta, kp.gaussian);
+        Fs[idx * FW] = f.x;
+        if (!FR) Fs[idx * FW + FW - 1] = f.y;
+      }
+      for (int idx = tid; idx < rn * TC; idx += K6_THR) {
+        const int r = idx / TC, col = col0 + idx % TC;
+        double2 g = make_double2(0.0, 0.0);
+        if (col < ncol) {
+          const int e = col / NC, c = col - e * NC;
+          const long long rr = rbase + r0 + r;
+          const double fe = rec_fE[rr * kp.nEF + e];
+          if (fe != 0.0) {
+            const double2 m = rec_M[rr * NC + c];
+            g = make_double2(fe * m.x, fe * m.y);
+          }
+        }
+        Gs[idx * GW] = g.x;
+        if (!MR) Gs[idx * GW + GW - 1] = g.y;
+      }
+      __syncthreads();
+#pragma unroll 1
+      for (int r = 0; r < rn; ++r) {
+        double fx[4], fy[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int o = (r * K6_TW + ty + 16 * i) * FW;
+          fx[i] = Fs[o];
+          if (!FR) fy[i] = Fs[o + FW - 1];
+        }
+#pragma unroll
+        for (int j = 0; j < JN; ++j) {
+          if (j >= jn) break;
+          const int o = (r * TC + tx + 16 * j) * GW;
+          const double gx = Gs[o], gy = MR ? 0.0 : Gs[o + GW - 1];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            double* a = acc[i][j];
+            a[0] = fma(fx[i], gx, a[0]);
+            if (!FR && !MR) a[0] = fma(-fy[i], gy, a[0]);
+            if (!MR) a[AW - 1] = fma(fx[i], gy, a[AW - 1]);
+            if (!FR) a[AW - 1] = fma(fy[i], gx, a[AW - 1]);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < JN; ++j)
+#pragma unroll
+        for (int a = 0; a < AW; ++a) accd[((i * JN + j) * AW + a) * K6_THR + tid] += acc[i][j][a];
+  }
+  wbg_u64* bad = out + 4 * (long long)kp.nEF * kp.nOmega * NC;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < JN; ++j) {
+      const int w = w0 + ty + 16 * i, col = col0 + tx + 16 * j;
+      if (w >= kp.nOmega || col >= ncol) continue;
+      const int e = col / NC, c = col - e * NC;
+      const double* a = accd + (i * JN + j) * AW * K6_THR + tid;
+      wbg_u64* o = out + 4 * (((long long)e * kp.nOmega + w) * NC + c);
+      fx_add_double(o, a[0], bad);
+      if (AW == 2) fx_add_double(o + 2, a[(AW - 1) * K6_THR], bad);
+    }
+}
+
+template <int NC, bool FR, bool MR>
+void launch_gemm64(int sms, cudaStream_t stream, const double* rec_dE, const void* rec_fE, const void* rec_M,
+                   const int* count, int P, int nk, const double* omega, const WbgKubo& kp, int formula, void* out) {
+  typedef K6<FR, MR> K;
+  const int gw = (kp.nOmega + K6_TW - 1) / K6_TW, gc = (kp.nEF * NC + K::TC - 1) / K::TC;
+  int gk = 2 * sms / (gw * gc);  // one wave of two blocks per SM
+  if (gk < 1) gk = 1;
+  if (gk > nk) gk = nk;
+  const int kc = (nk + gk - 1) / gk;
+  gk = (nk + kc - 1) / kc;
+  cudaFuncSetAttribute(kubo_gemm64<NC, FR, MR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K::SMEM);
+  kubo_gemm64<NC, FR, MR><<<dim3(gw, gk, gc), K6_THR, K::SMEM, stream>>>(
+      rec_dE, (const double*)rec_fE, (const double2*)rec_M, count, P, nk, kc, omega, kp, formula, (wbg_u64*)out);
+}
+
 template <typename T>
 void launch_pairs(int formula, int nk, size_t smp, cudaStream_t stream, const double* E, const void* Xbar, int nFbar,
                   const wbg_dynamic_spec& fs, int nw, const WbgKubo& kp, const double* efermi, double* rec_dE,
                   void* rec_fE, void* rec_M, int* count, int P) {
   typedef typename C2<T>::t V;
   const V* X = (const V*)Xbar;
+  if (formula == WBG_DYN_SHIFT)
+    cudaFuncSetAttribute(kubo_pairs<T, WBG_DYN_SHIFT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
 #define WBG_PAIRS(F) kubo_pairs<T, F><<<nk, 128, smp, stream>>>(E, X, nFbar, fs, nw, kp, efermi, rec_dE, (T*)rec_fE, \
                                                                 (V*)rec_M, count, P)
   switch (formula) {
@@ -549,7 +703,8 @@ int wbg_dynamic_run(const double* E, const void* Xbar, int nFbar, const wbg_dyna
   void* rec_M = w; w += (size_t)nk * P * 16 * nc;
   void* rec_fE = w; w += (size_t)nk * P * 8 * kp->nEF;
   int* count = (int*)w;
-  const size_t smp = (size_t)nw * 16 + (size_t)(2 * nw + 1) * 4;
+  const size_t smp = 8 * pairs_words(nw) + (F == WBG_DYN_SHIFT ? (size_t)nw * nw * (fp64 ? 8 : 4) : 0);
+  if (smp > 220 * 1024) return WBG_ERR_SIZE;
   if (fp64)
     launch_pairs<double>(F, nk, smp, stream, E, Xbar, nFbar, *fs, nw, *kp, efermi, rec_dE, rec_fE, rec_M, count, P);
   else
@@ -585,9 +740,14 @@ int wbg_dynamic_run(const double* E, const void* Xbar, int nFbar, const wbg_dyna
                                                  count, P, nk, kchunk, omega, *kp, F, efc, (wbg_u64*)out);     \
   } while (0)
   if (fp64) {
+#define WBG_GEMM64(NC, FR, MR) \
+  launch_gemm64<NC, FR, MR>(sms, stream, rec_dE, rec_fE, rec_M, count, P, nk, omega, *kp, F, out)
     if (nc == 1) WBG_ACCUM(1, double);
-    else if (nc == 9) WBG_ACCUM(9, double);
-    else WBG_ACCUM(27, double);
+    else if (F == WBG_DYN_OPTCOND) WBG_GEMM64(9, false, false);
+    else if (F == WBG_DYN_SHIFT) WBG_GEMM64(27, true, true);
+    else if (F == WBG_DYN_INJECTION) WBG_GEMM64(27, true, false);
+    else WBG_GEMM64(27, false, true);
+#undef WBG_GEMM64
   } else if (nc == 1) {
     WBG_ACCUM(1, float);
   } else if (wbg_tuned(WBG_TUNE_KUBO_ENGINE, 0, 1) != 2) {  // tensor cores (the built-in choice)

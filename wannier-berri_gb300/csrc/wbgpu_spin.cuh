@@ -13,6 +13,7 @@ struct KBand {
   int nw;
   long long nw2;
   wbg_dynamic_spec f;
+  const T* pf;  // [nw][nw] -(E_p - E_q) / ((E_p - E_q)^2 + sc_eta^2), the shift current's only
   WBG_D V x(int fld, int p, int q) const { return X[fld * nw2 + (long long)p * nw + q]; }
   WBG_D T dinv(int p, int q) const {  // dEig_inv (data_K.py:290-298)
     const double d = E[p] - E[q];
@@ -25,10 +26,7 @@ struct KBand {
     return r;
   }
   // principal-value D of the shift current: -V_pq (E_p - E_q) / ((E_p - E_q)^2 + eta^2)
-  WBG_D V Dp(int a, int p, int q) const {
-    const double d = E[p] - E[q];
-    return cscale(x(f.V + a, p, q), (T)(-d / (d * d + f.sc_eta * f.sc_eta)));
-  }
+  WBG_D V Dp(int a, int p, int q) const { return cscale(x(f.V + a, p, q), pf[p * nw + q]); }
 };
 
 // J'[p][q][a][s] of the spin current before (J' + J'^dagger) / 2 (formula/covariant.py:721-756),
