@@ -1463,11 +1463,33 @@ __global__ void berry_morb_kernel(const double* __restrict__ E, const typename C
 // over (s,a,b) in {(+1, alpha_c, beta_c), (-1, beta_c, alpha_c)}; the group value is
 // sum_{m in G} 2 Re S^{cd}.  hist is [nEF][3][3] (c, d) -- the calculator swaps c and d.
 // ---------------------------------------------------------------------------------------
+template <typename VS> WBG_D bool herm_equal(VS a, VS b) { return (a.x == b.x) & (a.y == -b.y); }
+// Whether thread `i0` of `step` finds V (3 fields) and W (9) Hermitian bit for bit on its rows' lower
+// triangle; every load of an element's twelve pairs is in flight at once
+template <typename VS> WBG_D bool herm_fields(const VS* V, const VS* W, int nw, int i0, int step) {
+  const int nw2 = nw * nw;
+  bool herm = true;
+  for (int i = i0; i < nw2; i += step) {
+    const int x = i / nw, y = i - x * nw, j = y * nw + x;
+    if (x < y) continue;
+    VS a[12], b[12];
+#pragma unroll
+    for (int f = 0; f < 12; ++f) {
+      const VS* F = f < 3 ? V + f * nw2 : W + (f - 3) * nw2;
+      a[f] = F[i];
+      b[f] = F[j];
+    }
+#pragma unroll
+    for (int f = 0; f < 12; ++f) herm &= herm_equal(a[f], b[f]);
+  }
+  return herm;
+}
+
 template <typename T, typename VS = typename C2<T>::t>
 __global__ void berry_deromega_kernel(const double* __restrict__ E, const VS* __restrict__ Xbar,
                                       int nFbar, int iV, int iA, int iO, int iW, int idA, int idO, int nw, int nk,
                                       int L, int G, int table, WbgScan sp, int internal_terms, int external_terms,
-                                      wbg_u64* __restrict__ hist, int shist, BandSel bs) {
+                                      wbg_u64* __restrict__ hist, int shist, BandSel bs, int skip_herm) {
   typedef typename C2<T>::t V;
   extern __shared__ double smb[];
   const int nh = 9 * sp.nEF;  // histogram entries [nEF][9], fixed point (shared or global)
@@ -1516,6 +1538,11 @@ __global__ void berry_deromega_kernel(const double* __restrict__ E, const VS* __
       bandmax = min(below, f0);
     }
     const VS* Xk = Xbar + kk * nFbar * nw2;
+    bool mine = true;  // with skip_herm: not one of berry_deromega_herm's k-points
+    if (skip_herm) {
+      const bool herm = herm_fields(Xk + iV * nw2, Xk + iW * nw2, nw, lane, L);
+      mine = group_sum_i(herm ? 0 : 1, L) > 0;
+    }
 #define XV(a, x, y) ld_c<V>(Xk[(iV + (a)) * nw2 + (x) * nw + (y)])
 #define XA(a, x, y) ld_c<V>(Xk[(iA + (a)) * nw2 + (x) * nw + (y)])
 #define XO(a, x, y) ld_c<V>(Xk[(iO + (a)) * nw2 + (x) * nw + (y)])
@@ -1538,7 +1565,7 @@ __global__ void berry_deromega_kernel(const double* __restrict__ E, const VS* __
       else ingroup = bs.sel ? bs.sel[kk * nw + m] == 1 : (myE[ge - 1] >= sp.EFmin && myE[gs] <= sp.EFmax);
       double val[9];
       for (int i = 0; i < 9; ++i) val[i] = 0.0;
-      if (ingroup) {
+      if (ingroup && mine) {
         for (int l = 0; l < nw; ++l) {
           if (l >= gs && l < ge) continue;
           const T dlm = dinv(l, m);  // 1/(E_l - E_m)
@@ -1695,9 +1722,9 @@ __global__ void berry_deromega_kernel(const double* __restrict__ E, const VS* __
 #undef XdO
 #undef DV
     __syncwarp();
-    if (valid && bs.P) {
+    if (valid && mine && bs.P) {
       emit_band_values(bs.P, k, nw, 9, lane, L, bandmax, bs.sel + k * nw, myS, myT, 9);
-    } else if (valid) {
+    } else if (valid && mine) {
       for (int n = lane; n < nw; n += L) {
         int gs = -1, ge = -1;
         bool sea = false;
@@ -1729,6 +1756,329 @@ __global__ void berry_deromega_kernel(const double* __restrict__ E, const VS* __
   }
   __syncthreads();
   if (hist && shist) fx_flush(sh, nh, hist);
+}
+
+// ---------------------------------------------------------------------------------------
+// The same traces for k-points whose V and W are Hermitian bit for bit (the mixed path's: their
+// inputs are mirrored and the rotation keeps the Hermitian part).  Then dD_ml = -conj(dD_lm), and with
+// D_xy = -V_xy / (E_x - E_y) the sums over intermediate bands become
+//   bracket of dD_lm^{bd} = W^{bd}_lm + t^{bd} + t^{db},  t^{bd} = sum_p V^b_lp (w V^d_pm),
+//   dA_lm^{bd} = dAc^{bd}_lm + sum_p X^b (w Y^d),  w = -1/(E_p - E_m), X = A_lp, Y = V_pm (p notin G)
+//                                                 w = +1/(E_l - E_p), X = A_pm, Y = V_lp (p in G)
+// -- 18 complex multiply-adds per (l, m, p) instead of 27, one instruction stream for both kinds of p,
+// and no access down a column (XV(a, m, p) over lanes m) in the loop.
+// A block takes one k-point: a thread owns band m of the bands that contribute (compacted) and
+// every S-th l outside its group, S = threads / bands, so the lanes are filled whatever num_wann and
+// however many bands the window leaves; the S partial traces add up in order.  Bound by FP32 issue:
+// 44 instructions per double-float multiply-add (11 per real product: exact two-sum, errors collected).
+// AHC + dipole, num_wann 82, 512 k-points: 67.4 -> 11.3 ms; num_wann 21, 4 096 k-points: 12.8 -> 2.3 ms (both with the
+// other kernel's check of the k-points, 0.2-0.3 ms).  One pass over both sums (18 accumulators, 168 registers, 3 blocks
+// an SM) took 12.3 and 2.9 ms, 5 blocks an SM (spills) 15.8 and 2.35 ms.
+// ---------------------------------------------------------------------------------------
+constexpr int DH_THR = 128, DH_OCC = 4;
+
+// w v and acc += r v for a stored element v and a weight / product in the arithmetic
+WBG_D double2 wmul(double w, double2 v) { return make_double2(w * v.x, w * v.y); }
+WBG_D cdf wmul(df64 w, float2 v) {
+  cdf r;
+  float p = w.hi * v.x;
+  r.x = df_quick(p, fmaf(w.lo, v.x, fmaf(w.hi, v.x, -p)));
+  p = w.hi * v.y;
+  r.y = df_quick(p, fmaf(w.lo, v.y, fmaf(w.hi, v.y, -p)));
+  return r;
+}
+WBG_D void df_lazy_fmaf(df64& acc, df64 a, float b) {
+  const float p = a.hi * b;
+  const float e = fmaf(a.lo, b, fmaf(a.hi, b, -p));
+  const float s = acc.hi + p;
+  const float v = s - acc.hi;
+  const float t = (acc.hi - (s - v)) + (p - v);
+  acc.hi = s;
+  acc.lo = acc.lo + (t + e);
+}
+WBG_D void smac(double2& acc, const double2& r, const double2& v) { cfma(acc, r, v); }
+WBG_D void smac(cdf& acc, const cdf& r, const float2& v) {
+  df_lazy_fmaf(acc.x, r.x, v.x);
+  df_lazy_fmaf(acc.x, r.y, -v.y);
+  df_lazy_fmaf(acc.y, r.x, v.y);
+  df_lazy_fmaf(acc.y, r.y, v.x);
+}
+
+template <typename T> size_t deromega_herm_smem(int nw) {
+  return 8 * ((size_t)nw + 9 * (size_t)nw + 9 * DH_THR) + sizeof(T) * (size_t)nw * nw + 4 * (size_t)nw * 4;
+}
+
+template <typename T, typename VS>
+__global__ void __launch_bounds__(DH_THR, DH_OCC)
+    berry_deromega_herm(const double* __restrict__ E, const VS* __restrict__ Xbar, int nFbar, int iV, int iA, int iO,
+                        int iW, int idA, int idO, int nw, int nk, WbgScan sp, int internal_terms, int external_terms,
+                        wbg_u64* __restrict__ hist, BandSel bs) {
+  typedef typename C2<T>::t V;
+  extern __shared__ double smb[];
+  double* Es = smb;                                        // [nw]
+  double* tv = Es + nw;                                    // [nw][9]
+  double* part = tv + 9 * nw;                              // [DH_THR][9]
+  T* dinvS = reinterpret_cast<T*>(part + 9 * DH_THR);      // [nw][M] 1/(E_x - E_m), m contributing
+  int* startS = reinterpret_cast<int*>(dinvS + nw * nw);   // [nw] first band of a group
+  int* gsS = startS + nw;                                  // [nw] group of a band, and the bands that contribute
+  int* geS = gsS + nw;
+  int* act = geS + nw;
+  __shared__ int M_s, bandmax_s;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int nw2 = nw * nw;
+  for (long long k = blockIdx.x; k < nk; k += gridDim.x) {
+    const VS* Xk = Xbar + k * nFbar * (long long)nw2;
+    __syncthreads();  // the previous k-point's shared data is read
+    for (int i = tid; i < nw; i += DH_THR) Es[i] = E[k * nw + i];
+    const bool herm = herm_fields(Xk + (long long)iV * nw2, Xk + (long long)iW * nw2, nw, tid, DH_THR);
+    if (!__syncthreads_and(herm)) continue;  // left to berry_deromega_kernel
+    for (int i = tid; i < nw; i += DH_THR) startS[i] = (i == 0) || (Es[i] - Es[i - 1] > sp.degen_thresh);
+    __syncthreads();
+    if (tid < 32) {
+      int bandmax;
+      if (bs.sel) {
+        bandmax = sel_bandmax(bs.sel + k * nw, nw, lane, 32);
+      } else {
+        int below = 0, f0 = nw;
+        for (int n = lane; n < nw; n += 32) {
+          below += Es[n] < sp.EFmin;
+          if (startS[n]) {
+            int g1 = n + 1;
+            while (g1 < nw && !startS[g1]) ++g1;
+            if (Es[g1 - 1] >= sp.EFmin && Es[n] <= sp.EFmax) f0 = min(f0, n);
+          }
+        }
+        bandmax = min(group_sum_i(below, 32), group_min_i(f0, 32));
+      }
+      int M = 0;
+      for (int base = 0; base < nw; base += 32) {
+        const int m = base + lane;
+        bool in = false;
+        if (m < nw) {
+          int gs = m, ge = m + 1;
+          while (!startS[gs]) --gs;
+          while (ge < nw && !startS[ge]) ++ge;
+          if (m < bandmax) {
+            gs = 0;
+            ge = bandmax;
+            in = true;
+          } else {
+            in = bs.sel ? bs.sel[k * nw + m] == 1 : (Es[ge - 1] >= sp.EFmin && Es[gs] <= sp.EFmax);
+          }
+          gsS[m] = gs;
+          geS[m] = ge;
+        }
+        const unsigned b = __ballot_sync(0xffffffffu, in);
+        if (in) act[M + __popc(b & ((1u << lane) - 1u))] = m;
+        M += __popc(b);
+      }
+      if (lane == 0) {
+        M_s = M;
+        bandmax_s = bandmax;
+      }
+    }
+    __syncthreads();
+    const int M = M_s, bandmax = bandmax_s;
+    for (int i = tid; i < 9 * nw; i += DH_THR) tv[i] = 0.0;
+    for (int i = tid; i < nw * M; i += DH_THR) {
+      const double dE = Es[i / M] - Es[act[i % M]];
+      dinvS[i] = fabs(dE) < 1e-7 ? Arith<T>::from(0.0) : recip_gap<T>(dE);
+    }
+    __syncthreads();
+    const int S = M > 0 ? DH_THR / M : 0;  // slices of the l (and n') loops; M <= nw <= DH_THR
+    if (tid < S * M) {
+      const int im = tid % M, sl = tid / M;
+      const int m = act[im], gs = gsS[m], ge = geS[m], ng = ge - gs;
+      const VS* XV = Xk + (long long)iV * nw2;
+      const VS* XA = Xk + (long long)iA * nw2;
+      const VS* XO = Xk + (long long)iO * nw2;
+      const VS* XW = Xk + (long long)iW * nw2;
+      const VS* XdA = Xk + (long long)idA * nw2;
+      const VS* XdO = Xk + (long long)idO * nw2;
+      double val[9];
+#pragma unroll
+      for (int i = 0; i < 9; ++i) val[i] = 0.0;
+      // the dD terms, then the dA and dO terms: two passes keep 9 accumulators live instead of 18
+      for (int il = sl; il < nw - ng; il += S) {
+        const int l = il < gs ? il : il + ng;  // the bands outside the group
+        V dD[9];
+#pragma unroll
+        for (int i = 0; i < 9; ++i) dD[i] = czero<V>();
+        const T* dl = dinvS + l * M + im - m;  // 1/(E_l - E_p) of a band p of the group at dl[p]
+#pragma unroll 1
+        for (int p = 0; p < nw; ++p) {
+          const T w = p >= gs && p < ge ? dl[p] : -dinvS[p * M + im];
+          VS Vlp[3];
+          V r[3];
+#pragma unroll
+          for (int a = 0; a < 3; ++a) {
+            Vlp[a] = XV[a * nw2 + l * nw + p];
+            r[a] = wmul(w, XV[a * nw2 + p * nw + m]);
+          }
+#pragma unroll
+          for (int b = 0; b < 3; ++b)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) smac(dD[3 * b + d], r[d], Vlp[b]);
+        }
+        const T dlm = dinvS[l * M + im];  // 1/(E_l - E_m)
+#pragma unroll
+        for (int i = 0; i < 9; ++i) dD[i] = cdone(dD[i]);
+#pragma unroll
+        for (int b = 0; b < 3; ++b)
+#pragma unroll
+          for (int d = b; d < 3; ++d) {
+            const V t = cadd(cadd(dD[3 * b + d], dD[3 * d + b]), ld_c<V>(XW[(3 * b + d) * nw2 + l * nw + m]));
+            dD[3 * b + d] = dD[3 * d + b] = cscale(t, -dlm);
+          }
+        // s Im(D^a_ml dD^{bd}_lm) (internal) and, with dD_ml = -conj(dD_lm), s Re(conj(dD^{ad}_lm) A^b_lm)
+        // = -s Re(conj(A^a_lm) dD^{bd}_lm) with a and b exchanged (external): one product with B^a
+        V B[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          B[a] = czero<V>();
+          if (internal_terms) B[a] = cmuli(cscale(ld_c<V>(XV[a * nw2 + m * nw + l]), -dlm));  // -i D^a_ml
+          if (external_terms) B[a] = csub(B[a], cconj(ld_c<V>(XA[a * nw2 + l * nw + m])));
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const int al = (c + 1) % 3, be = (c + 2) % 3;
+#pragma unroll
+          for (int d = 0; d < 3; ++d)
+            val[3 * c + d] += 2.0 * (to_dbl(cmul(B[al], dD[3 * be + d]).x) - to_dbl(cmul(B[be], dD[3 * al + d]).x));
+        }
+      }
+      for (int il = external_terms ? sl : nw; il < nw - ng; il += S) {
+        const int l = il < gs ? il : il + ng;
+        V dA[9];
+#pragma unroll
+        for (int i = 0; i < 9; ++i) dA[i] = czero<V>();
+        const T* dl = dinvS + l * M + im - m;
+#pragma unroll 1
+        for (int p = 0; p < nw; ++p) {
+          const bool inG = p >= gs && p < ge;
+          const T w = inG ? dl[p] : -dinvS[p * M + im];
+          const int ilp = l * nw + p, ipm = p * nw + m;
+          const int ix = inG ? ipm : ilp, iy = inG ? ilp : ipm;
+          VS Xa[3];
+          V r[3];
+#pragma unroll
+          for (int a = 0; a < 3; ++a) {
+            Xa[a] = XA[a * nw2 + ix];
+            r[a] = wmul(w, XV[a * nw2 + iy]);
+          }
+#pragma unroll
+          for (int b = 0; b < 3; ++b)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) smac(dA[3 * b + d], r[d], Xa[b]);
+        }
+        const T dlm = dinvS[l * M + im];
+        V Dml[3];
+#pragma unroll
+        for (int i = 0; i < 9; ++i) dA[i] = cadd(cdone(dA[i]), ld_c<V>(XdA[i * nw2 + l * nw + m]));
+#pragma unroll
+        for (int a = 0; a < 3; ++a) Dml[a] = cscale(ld_c<V>(XV[a * nw2 + m * nw + l]), dlm);  // -V_ml / (E_m - E_l)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const int al = (c + 1) % 3, be = (c + 2) % 3;
+          const V Olm = ld_c<V>(XO[c * nw2 + l * nw + m]), Oml = ld_c<V>(XO[c * nw2 + m * nw + l]);
+#pragma unroll
+          for (int d = 0; d < 3; ++d) {
+            // 1/2 dO_mm: - D^d_ml O^c_lm + O^c_ml D^d_lm, D_lm = -conj(D_ml)
+            const V Dlm = mkc<T>(-Dml[d].x, Dml[d].y);
+            val[3 * c + d] += 2.0 * (to_dbl(cmul(Dml[be], dA[3 * al + d]).x) - to_dbl(cmul(Dml[al], dA[3 * be + d]).x)) +
+                              (to_dbl(cmul(Oml, Dlm).x) - to_dbl(cmul(Dml[d], Olm).x));
+          }
+        }
+      }
+      if (external_terms) {
+        if (sl == 0) {
+#pragma unroll
+          for (int i = 0; i < 9; ++i) val[i] += to_dbl(ld_c<V>(XdO[i * nw2 + m * nw + m]).x);  // 2 Re(1/2 dOc_mm)
+        }
+        // -i s sum_{n' in G} A^a_mn' dA^{bd}_n'm
+        for (int np = gs + sl; np < ge; np += S) {
+          V dAn[9];
+#pragma unroll
+          for (int i = 0; i < 9; ++i) dAn[i] = czero<V>();
+          const int in = im + np - m;
+#pragma unroll 1
+          for (int il = 0; il < nw - ng; ++il) {
+            const int l = il < gs ? il : il + ng;
+            const T wn = -dinvS[l * M + in], wm = -dinvS[l * M + im];
+            V Dn[3], Dm[3];  // -D^d_n'l = -V_n'l / (E_l - E_n') and D^d_lm
+            VS Alm[3], Anl[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+              Dn[a] = wmul(wn, XV[a * nw2 + np * nw + l]);
+              Dm[a] = wmul(wm, XV[a * nw2 + l * nw + m]);
+              Alm[a] = XA[a * nw2 + l * nw + m];
+              Anl[a] = XA[a * nw2 + np * nw + l];
+            }
+#pragma unroll
+            for (int b = 0; b < 3; ++b)
+#pragma unroll
+              for (int d = 0; d < 3; ++d) {
+                smac(dAn[3 * b + d], Dn[d], Alm[b]);
+                smac(dAn[3 * b + d], Dm[d], Anl[b]);
+              }
+          }
+          V Amn[3];
+#pragma unroll
+          for (int a = 0; a < 3; ++a) Amn[a] = ld_c<V>(XA[a * nw2 + m * nw + np]);
+#pragma unroll
+          for (int i = 0; i < 9; ++i) dAn[i] = cadd(cdone(dAn[i]), ld_c<V>(XdA[i * nw2 + np * nw + m]));
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            const int al = (c + 1) % 3, be = (c + 2) % 3;
+#pragma unroll
+            for (int d = 0; d < 3; ++d)  // 2 Re(-i s A dA) = 2 s Im(A dA)
+              val[3 * c + d] += 2.0 * (to_dbl(cmul(Amn[al], dAn[3 * be + d]).y) - to_dbl(cmul(Amn[be], dAn[3 * al + d]).y));
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 9; ++i) part[tid * 9 + i] = val[i];
+    }
+    __syncthreads();
+    for (int i = tid; i < 9 * M; i += DH_THR) {
+      const int im = i / 9, c = i - im * 9;
+      double v = 0.0;
+      for (int s = 0; s < S; ++s) v += part[(s * M + im) * 9 + c];
+      tv[act[im] * 9 + c] = v;
+    }
+    __syncthreads();
+    if (bs.P) {
+      emit_band_values(bs.P, k, nw, 9, tid, DH_THR, bandmax, bs.sel + k * nw, startS, tv, 9);
+      continue;
+    }
+    for (int n = tid; n < nw; n += DH_THR) {
+      int gs = -1, ge = -1;
+      const bool sea = n == 0 && bandmax > 0;
+      if (sea) {
+        gs = 0;
+        ge = bandmax;
+      } else if (n >= bandmax && startS[n] && Es[geS[n] - 1] >= sp.EFmin && Es[n] <= sp.EFmax) {
+        gs = n;
+        ge = geS[n];
+      }
+      if (gs < 0) continue;
+      double v[9], esum = 0.0;
+#pragma unroll
+      for (int i = 0; i < 9; ++i) v[i] = 0.0;
+      for (int q = gs; q < ge; ++q) {
+#pragma unroll
+        for (int i = 0; i < 9; ++i) v[i] += tv[q * 9 + i];
+        esum += Es[q];
+      }
+      int bin = 0;
+      if (!sea) {
+        const double Em = esum / (double)(ge - gs);
+        bin = Em < sp.EFmin ? 0 : Em <= sp.EFmax ? (int)ceil((Em - sp.EFmin) / sp.dEF) : -1;
+      }
+      if (bin >= 0 && bin < sp.nEF)
+        for (int i = 0; i < 9; ++i) fx_add_double(hist + 2 * ((long long)bin * 9 + i), v[i], hist + 2ll * 9 * sp.nEF);
+    }
+  }
 }
 
 // cumulative sum over Fermi levels and normalisation: out[ie][c] = scale * sum_{j<=ie} hist[j][c],
@@ -2128,22 +2478,32 @@ int wbg_berry_deromega_run(const double* E, const void* Xbar, int nFbar, int iV,
   long long nblk = (nk + G - 1) / G;
   const long long cap = (long long)sms * 8;
   if (nblk > cap) nblk = cap;
+  // double-float: the Hermitian k-points (every one of the mixed path's) take the kernel made for them
+  const int split = fp64 == 2 && nw <= DH_THR;
+  if (split) {
+    const size_t smh = deromega_herm_smem<df64>(nw);
+    cudaFuncSetAttribute(berry_deromega_herm<df64, float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+    const int nb = nk < DH_OCC * sms ? nk : DH_OCC * sms;
+    berry_deromega_herm<df64, float2><<<nb, DH_THR, smh, stream>>>(E, (const float2*)Xbar, nFbar, iV, iA, iO, iW, idA,
+                                                                   idO, nw, nk, *sp, internal_terms, external_terms,
+                                                                   (wbg_u64*)hist, bs);
+  }
   if (fp64 == 1) {
     cudaFuncSetAttribute(berry_deromega_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
     berry_deromega_kernel<double><<<(int)nblk, G * L, sm, stream>>>(E, (const double2*)Xbar, nFbar, iV, iA, iO, iW,
                                                                     idA, idO, nw, nk, L, G, table, *sp, internal_terms,
-                                                                    external_terms, (wbg_u64*)hist, shist, bs);
+                                                                    external_terms, (wbg_u64*)hist, shist, bs, 0);
   } else if (fp64 == 2) {  // complex64 Xbar, double-float arithmetic
     cudaFuncSetAttribute(berry_deromega_kernel<df64, float2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          220 * 1024);
     berry_deromega_kernel<df64, float2><<<(int)nblk, G * L, sm, stream>>>(
         E, (const float2*)Xbar, nFbar, iV, iA, iO, iW, idA, idO, nw, nk, L, G, table, *sp, internal_terms,
-        external_terms, (wbg_u64*)hist, shist, bs);
+        external_terms, (wbg_u64*)hist, shist, bs, split);
   } else {
     cudaFuncSetAttribute(berry_deromega_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
     berry_deromega_kernel<float><<<(int)nblk, G * L, sm, stream>>>(E, (const float2*)Xbar, nFbar, iV, iA, iO, iW, idA,
                                                                    idO, nw, nk, L, G, table, *sp, internal_terms,
-                                                                   external_terms, (wbg_u64*)hist, shist, bs);
+                                                                   external_terms, (wbg_u64*)hist, shist, bs, 0);
   }
   return wbg_cuda_status(cudaGetLastError());
 }
