@@ -74,3 +74,16 @@ def test_hermitian_and_other_kpoints_in_one_batch():
                         for s in (slice(None), slice(0, None, 2), slice(1, None, 2)))
     assert any(even) and any(odd)
     assert whole == [(a + b) % 2 ** 128 for a, b in zip(even, odd)]
+
+
+@pytest.mark.parametrize("nw,nk", [(5, 60), (21, 9), (33, 4), (82, 2)])
+def test_fp64_hermitian_kpoints(nw, nk):
+    """The same split in FP64: the two FP64 kernels differ by 2^-53 where the double-float one differs by 2^-47
+    through the same gaps -- 2^-6 of its distance, with a factor 8 for the different order of the sums."""
+    E, X = _fields(nw, nk, 7 * nw + nk, True)
+    other = X.astype(np.complex128)
+    other[:, IV, 0, 0] += 1e-30j
+    general = _hist(E, other, 1, 1, 1)
+    got = _hist(E, X.astype(np.complex128), 1, 1, 1)
+    df = _hist(E, other.astype(np.complex64), 2, 1, 1)
+    assert np.abs(got - general).max() <= 2.0 ** -3 * np.abs(df - general).max() + 2.0 ** -50 * np.abs(general).max()

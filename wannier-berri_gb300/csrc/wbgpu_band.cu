@@ -2478,21 +2478,29 @@ int wbg_berry_deromega_run(const double* E, const void* Xbar, int nFbar, int iV,
   long long nblk = (nk + G - 1) / G;
   const long long cap = (long long)sms * 8;
   if (nblk > cap) nblk = cap;
-  // double-float: the Hermitian k-points (every one of the mixed path's) take the kernel made for them
-  const int split = fp64 == 2 && nw <= DH_THR;
+  // FP64 and double-float: the Hermitian k-points (every one whose fields come from lower triangles)
+  // take the kernel made for them
+  const int split = fp64 != 0 && nw <= DH_THR;
   if (split) {
-    const size_t smh = deromega_herm_smem<df64>(nw);
-    cudaFuncSetAttribute(berry_deromega_herm<df64, float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
     const int nb = nk < DH_OCC * sms ? nk : DH_OCC * sms;
-    berry_deromega_herm<df64, float2><<<nb, DH_THR, smh, stream>>>(E, (const float2*)Xbar, nFbar, iV, iA, iO, iW, idA,
-                                                                   idO, nw, nk, *sp, internal_terms, external_terms,
-                                                                   (wbg_u64*)hist, bs);
+    if (fp64 == 1) {
+      cudaFuncSetAttribute(berry_deromega_herm<double, double2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           220 * 1024);
+      berry_deromega_herm<double, double2><<<nb, DH_THR, deromega_herm_smem<double>(nw), stream>>>(
+          E, (const double2*)Xbar, nFbar, iV, iA, iO, iW, idA, idO, nw, nk, *sp, internal_terms, external_terms,
+          (wbg_u64*)hist, bs);
+    } else {
+      cudaFuncSetAttribute(berry_deromega_herm<df64, float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+      berry_deromega_herm<df64, float2><<<nb, DH_THR, deromega_herm_smem<df64>(nw), stream>>>(
+          E, (const float2*)Xbar, nFbar, iV, iA, iO, iW, idA, idO, nw, nk, *sp, internal_terms, external_terms,
+          (wbg_u64*)hist, bs);
+    }
   }
   if (fp64 == 1) {
     cudaFuncSetAttribute(berry_deromega_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
     berry_deromega_kernel<double><<<(int)nblk, G * L, sm, stream>>>(E, (const double2*)Xbar, nFbar, iV, iA, iO, iW,
                                                                     idA, idO, nw, nk, L, G, table, *sp, internal_terms,
-                                                                    external_terms, (wbg_u64*)hist, shist, bs, 0);
+                                                                    external_terms, (wbg_u64*)hist, shist, bs, split);
   } else if (fp64 == 2) {  // complex64 Xbar, double-float arithmetic
     cudaFuncSetAttribute(berry_deromega_kernel<df64, float2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          220 * 1024);

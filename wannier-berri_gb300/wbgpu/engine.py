@@ -215,25 +215,26 @@ class DeviceSystem:
 
     def hermitian_bases(self, rtol=1e-12):
         """Base matrices whose R-space data are Hermitian, X_R = X_{-R}^dagger within rtol of
-        max |X| with every -R present: for them the k-space fields are exactly Hermitian and the
-        mixed path transforms only lower triangles.  Other bases keep the full-matrix path with
-        the reference's symmetrisation.  The verdict is a property of the host matrices: it is
-        computed on the device once and kept with the system's pinned upload copies (dropped
+        max |X| with every -R present: for them the k-space fields are exactly Hermitian and
+        only lower triangles are transformed (the mixed path; with rtol 0, equality bit for bit, the FP64
+        path too).  Other bases keep the full-matrix path with the reference's symmetrisation.  The
+        verdict is a property of the host matrices: it is computed once (on the device, on the host
+        where the matrices are small) and kept with the system's pinned upload copies (dropped
         when set_R_mat or do_ws_dist change the matrices)."""
-        if 'herm_bases' not in self._cache:
+        if ('herm_bases', rtol) not in self._cache:
             verdicts = self.system.__dict__.setdefault('_herm_cache', {})
             out = set()
             for key in ('Ham', 'AA', 'SS'):
                 if not self.system.has_R_mat(key):
                     continue
                 if (key, rtol) not in verdicts:
-                    verdicts[(key, rtol)] = self._hermitian_on_device(key, rtol)
+                    verdicts[(key, rtol)] = self._is_hermitian(key, rtol)
                 if verdicts[(key, rtol)]:
                     out.add(key)
-            self._cache['herm_bases'] = frozenset(out)
-        return self._cache['herm_bases']
+            self._cache[('herm_bases', rtol)] = frozenset(out)
+        return self._cache[('herm_bases', rtol)]
 
-    def _hermitian_on_device(self, key, rtol):
+    def _is_hermitian(self, key, rtol):
         R = self.geom.R  # sorted by (R0, R1, R2): -R found by a binary search on the packed keys
         span = 2 * int(np.abs(R).max()) + 1
         pack = lambda a: ((a[:, 0] * span) + a[:, 1]) * span + a[:, 2]
@@ -241,10 +242,18 @@ class DeviceSystem:
         pos = np.minimum(np.searchsorted(keys, pack(-R)), len(keys) - 1)
         if not np.array_equal(keys[pos], pack(-R)):
             return False
-        neg = torch.from_numpy(pos).to(self.device)
         nw = self.nw
+        if len(R) * nw * nw <= 1 << 16:  # a few hundred microseconds on the host, no synchronisation
+            X = host_pinned(self.system, key, self.geom.order).numpy().reshape(-1, len(R), nw, nw)
+            Xd = X[:, pos].conj().swapaxes(2, 3)
+            if rtol == 0:
+                return bool(np.array_equal(X, Xd))
+            return bool(np.abs(X - Xd).max() <= rtol * max(float(np.abs(X).max()), 1e-300))
+        neg = torch.from_numpy(pos).to(self.device)
         X = self._key_fp64(key).reshape(-1, len(R), nw, nw)  # device, sorted R order
         Xd = X[:, neg].conj().transpose(2, 3)
+        if rtol == 0:
+            return bool((X == Xd).all())
         diff, mx = (X - Xd).abs().max(), X.abs().max()
         return float(diff) <= rtol * max(float(mx), 1e-300)
 
@@ -402,13 +411,14 @@ def hermitian_fields(quantities, with_H, herm_bases=('Ham', 'AA')):
     return [d[1] not in nonherm for d in desc]
 
 
-def column_list(dev, quantities, with_H, lower):
+def column_list(dev, quantities, with_H, lower, rtol=1e-12):
     """Device int32 list of the elements f*nw2 + m*nw + n that wbg_r2k_columns computes: the
-    lower triangle (m >= n) of the Hermitian fields when ``lower``, every element otherwise."""
-    key = ('cols', tuple(sorted(quantities)), with_H, bool(lower))
+    lower triangle (m >= n) of the Hermitian fields (hermitian_bases(rtol)) when ``lower``, every
+    element otherwise."""
+    key = ('cols', tuple(sorted(quantities)), with_H, bool(lower), rtol)
     if key not in dev._cache:
         nw = dev.nw
-        herm = hermitian_fields(quantities, with_H, dev.hermitian_bases())
+        herm = hermitian_fields(quantities, with_H, dev.hermitian_bases(rtol))
         m, n = np.meshgrid(np.arange(nw), np.arange(nw), indexing='ij')
         full = (m * nw + n).reshape(-1)
         tril = (m * nw + n)[m >= n]
@@ -416,6 +426,14 @@ def column_list(dev, quantities, with_H, lower):
         dev._cache[key] = (torch.tensor(cols.astype(np.int32), device=dev.device),
                            [bool(lower and h) for h in herm])
     return dev._cache[key]
+
+
+def fp64_columns(dev, quantities, nkt):
+    """Column list of an FP64 batch of `nkt` k-points (H and the quantities' fields) and the fields given by
+    their lower triangle; (None, all False): every element."""
+    if nkt >= FP64_LOWER_MIN_K and dev.hermitian_bases(0.0):
+        return column_list(dev, quantities, True, True, 0.0)
+    return None, [False] * len(field_plan(quantities, True, extra_keys_for(quantities))[0])
 
 
 def split_columns(dev, quantities, with_H, lower, first):
@@ -544,6 +562,11 @@ MIXED_EIGH_REFINE_NW = (24, 32)
 # Berry-curvature dipole on two 12^3 blocks: 1.9e-6 and 4.8e-7).
 MIXED_FIELDS_PREC = 3  # PREC_FP32S
 MIXED_DF64_QUANTITIES = {'V'}
+# From this many k-points a batch's FP64 transform writes only the lower triangles of the fields whose
+# R-space matrices are Hermitian bit for bit (half the transform: 18.9 -> 9.6 ms per 13 824 k-points at
+# num_wann 32, 5.0 ms on conjugate pairs of R); below, building the column list on a
+# fresh system (0.1 ms) costs more than it saves.
+FP64_LOWER_MIN_K = 64
 # Arithmetic of the mixed path's Berry-curvature dipole (wbg_berry_deromega fp64 argument): 2 =
 # double-float on the complex64 band-basis fields.  Its sums over intermediate bands of V D terms
 # cancel strongly near degeneracies; in FP32 they put the BCD of a num_wann = 82 system 3.9e-6 from
@@ -732,10 +755,12 @@ def band_data(dev, dKs, NKFFT, quantities, precision='fp64', phases=None, block_
     _lib.check(_lib.load().wbg_eigh_workspace_size(nw, nkt, ctypes.byref(ews)), "wbg_eigh_workspace_size")
     ework = arena.buffer('eigh_ws', (int(ews.value),), torch.uint8)
     if precision == 'fp64':
-        fields, index, nF, k1 = fields_for(quantities, True, PREC_FP64, 'fields')
+        cols, lower_in = fp64_columns(dev, quantities, nkt)
+        fields, index, nF, k1 = fields_for(quantities, True, PREC_FP64, 'fields', cols=cols)
         keep.append(k1)
         U = arena.buffer('U', (nkt, nw, nw), torch.complex128)
-        E, U, flag = eigh(fields, nF * nw * nw, nw, nkt, E=E, U=U, mode=1, work=ework, flag=flag)
+        mode = 1 | (EIGH_LOWER if lower_in[0] else 0)
+        E, U, flag = eigh(fields, nF * nw * nw, nw, nkt, E=E, U=U, mode=mode, work=ework, flag=flag)
         fp64_fields = True
     elif precision == 'mixed':
         # lower triangles of the Hermitian fields only: exactly Hermitian, half the transform
@@ -807,10 +832,9 @@ def band_data(dev, dKs, NKFFT, quantities, precision='fp64', phases=None, block_
             n = QUANTITIES[q]['ncomp']
             sel += list(range(index[q], index[q] + n))
             herm += [QUANTITIES[q]['herm']] * n
-    if not fp64_fields:
-        # mirrored (exactly Hermitian) inputs: flag them, and keep the Hermitian part of their
-        # rotation, which drops only the FP32 rounding noise of U^dagger X U
-        herm = [(h or 1) | 4 if lower_in[f] else h for f, h in zip(sel, herm)]
+    # mirrored (exactly Hermitian) inputs: flag them, and keep the Hermitian part of their
+    # rotation, which drops only the rounding noise of U^dagger X U
+    herm = [(h or 1) | 4 if lower_in[f] else h for f, h in zip(sel, herm)]
     if sel:
         Xb = arena.buffer('Xbar', (nkt, len(sel), nw, nw), torch.complex128 if fp64_fields else torch.complex64)
         Xbar, k2 = rotate(U, fields, nF, sel, herm, nw, nkt, 1 if fp64_fields else rot_prec, out=Xb)
@@ -944,9 +968,10 @@ def energies(dev, dKs, NKFFT, precision='fp64', out=None, phases=None, block_sta
     flag = arena.buffer('flag_E', (1,), torch.int32)
     flag.zero_()
     if precision == 'fp64':
-        prec, lower, mode = PREC_FP64, False, 1
+        cols, lower_in = fp64_columns(dev, set(), nkt)
+        lower, prec, mode = False, PREC_FP64, 1 | (EIGH_LOWER if lower_in[0] else 0)
     elif precision == 'mixed':
-        lower = 'Ham' in dev.hermitian_bases()
+        lower, cols = 'Ham' in dev.hermitian_bases(), None
         prec, mode = PREC_DF64, 3 | (EIGH_LOWER if lower else 0)
     else:
         raise ValueError(f"unknown precision mode {precision!r}")
@@ -958,7 +983,8 @@ def energies(dev, dKs, NKFFT, precision='fp64', out=None, phases=None, block_sta
                "wbg_r2k_workspace_size")
     work = arena.buffer('r2k_ws', (int(wsz.value),), torch.uint8)
     Hf, _, _, keep = r2k(dev, dKs, NKFFT, set(), True, prec, out=Hf, workspace=work,
-                         phases=None if phases is None else phases.get(prec), block_start=block_start, lower=lower)
+                         phases=None if phases is None else phases.get(prec), block_start=block_start, lower=lower,
+                         cols=cols)
     ews = ctypes.c_size_t(0)
     _lib.check(_lib.load().wbg_eigh_workspace_size(nw, nkt, ctypes.byref(ews)), "wbg_eigh_workspace_size")
     ework = arena.buffer('eigh_ws', (int(ews.value),), torch.uint8)
