@@ -112,9 +112,18 @@ __global__ void rotate_kernel(const typename C2<T>::t* __restrict__ U, long long
   }
 }
 
-// Register-tiled rotation for nw % 4 == 0: each thread owns a 4x4 tile of the nw x nw
-// output; KB k-points per CTA.  X rows are padded (stride nw+1) so the column reads of
-// different tile rows fall in different banks.  Same math as rotate_kernel.
+// Register-tiled rotation: each thread owns a 4x4 tile of the nw x nw output (rows and columns up to
+// nwp = 4 ceil(nw / 4), zeros beyond nw); KB k-points per CTA.  X rows are padded (stride nwp+1) so the
+// column reads of different tile rows fall in different banks; the next field's tile is loaded while
+// this one is rotated.  Same sums in the same order as rotate_kernel, which needs two loads per
+// multiply-add and serves only num_wann < 5.  FP32: num_wann 21, 36 fields, 4 096 k-points 1.61 (rotate_kernel)
+// -> 1.13 ms; num_wann 31, 9 fields 1.09 -> 0.55 ms; num_wann 8, 9 fields, 110 592 k-points 0.64 -> 0.57 ms.
+// X kept transposed, with 16-byte shared-memory loads for every operand, gained nothing (1.14, 0.61, 0.67 ms).
+// complex words of one k-point in shared memory: U, X and T
+WBG_HD size_t tiled_words(int nw) {
+  const int nwp = (nw + 3) & ~3;
+  return (size_t)nw * nwp + (size_t)nwp * (nwp + 1) + (size_t)nwp * nwp;
+}
 template <typename T, typename VO>
 __global__ void rotate_tiled(const typename C2<T>::t* __restrict__ U, long long strideU,
                              const typename C2<T>::t* __restrict__ X, int nFin, const int* __restrict__ fsel,
@@ -122,30 +131,58 @@ __global__ void rotate_tiled(const typename C2<T>::t* __restrict__ U, long long 
                              int nk, int KB) {
   typedef typename C2<T>::t V;
   extern __shared__ unsigned char smr[];
-  const int nt = nw / 4;                 // tiles per dimension
-  const int tpk = nt * nt;               // threads per k-point
+  const int nt = (nw + 3) / 4, nwp = 4 * nt;  // tiles per dimension
+  const int tpk = nt * nt;                    // threads per k-point
   const int kl = threadIdx.x / tpk, tid = threadIdx.x % tpk;
   const int ty = tid / nt, tx = tid % nt;
-  const int ldx = nw + 1;
-  V* base = reinterpret_cast<V*>(smr) + (size_t)kl * (nw * nw + nw * ldx + nw * nw);
-  V* Us = base;                          // [nw][nw]
-  V* Xs = Us + nw * nw;                  // [nw][nw+1]
-  V* Ts = Xs + nw * ldx;                 // [nw][nw]
+  V* base = reinterpret_cast<V*>(smr) + (size_t)kl * tiled_words(nw);
+  V* Us = base;                          // [nw][nwp]
+  V* Xs = Us + nw * nwp;                 // [nwp][nwp+1] X, then the Hermitian part's staging
+  V* Ts = Xs + nwp * (nwp + 1);          // [nwp][nwp]
   long long k = (long long)blockIdx.x * KB + kl;
   const bool valid = k < nk;
   if (!valid) k = nk - 1;
   const int nw2 = nw * nw;
-  for (int i = tid; i < nw2; i += tpk) Us[i] = U[k * strideU + i];
-  const int m0 = 4 * ty, n0 = 4 * tx;
-  for (int f = 0; f < nFrot; ++f) {
+  const int m0 = 4 * ty, n0 = 4 * tx, ldx = nwp + 1;
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+      if (m0 + a < nw)
+        Us[(m0 + a) * nwp + n0 + b] = n0 + b < nw ? U[k * strideU + (m0 + a) * nw + n0 + b] : czero<V>();
+  // a field's tile of this thread: loaded one field ahead, while the previous one is rotated, and taken
+  // as it is in memory (a use of the values would wait for them)
+  V xn[4][4];
+  auto load_tile = [&](int f) {
     const int fs = fsel[f];
     const bool fok = fs >= 0 && fs < nFin;  // selection lives in device memory: validate here
     const V* src = X + (k * nFin + (fok ? fs : 0)) * (long long)nw2;
-    const T nan = rnan<T>();
     const bool lower = (herm[f] & 4) != 0;
-    for (int i = tid; i < nw2; i += tpk)
-      Xs[(i / nw) * ldx + (i % nw)] = fok ? load_field(src, i, nw, lower) : mkc<T>(nan, nan);
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const int m = m0 + a, n = n0 + b;
+        xn[a][b] = m < nw && n < nw && fok ? src[lower && m < n ? n * nw + m : m * nw + n] : czero<V>();
+      }
+  };
+  load_tile(0);
+  for (int f = 0; f < nFrot; ++f) {
+    const bool fbad = fsel[f] < 0 || fsel[f] >= nFin, lower = (herm[f] & 4) != 0;
+    const T nan = rnan<T>();
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const int m = m0 + a, n = n0 + b;
+        V v = xn[a][b];
+        if (lower && m < n) v.y = -v.y;
+        if (lower && m == n) v = real_only(v);
+        if (fbad && m < nw && n < nw) v = mkc<T>(nan, nan);
+        Xs[m * ldx + n] = v;
+      }
     __syncthreads();
+    if (f + 1 < nFrot) load_tile(f + 1);
     V acc[4][4];
 #pragma unroll
     for (int a = 0; a < 4; ++a)
@@ -156,7 +193,7 @@ __global__ void rotate_tiled(const typename C2<T>::t* __restrict__ U, long long 
 #pragma unroll
       for (int a = 0; a < 4; ++a) xa[a] = Xs[(m0 + a) * ldx + j];
 #pragma unroll
-      for (int b = 0; b < 4; ++b) ub[b] = Us[j * nw + n0 + b];
+      for (int b = 0; b < 4; ++b) ub[b] = Us[j * nwp + n0 + b];
 #pragma unroll
       for (int a = 0; a < 4; ++a)
 #pragma unroll
@@ -165,18 +202,17 @@ __global__ void rotate_tiled(const typename C2<T>::t* __restrict__ U, long long 
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
-      for (int b = 0; b < 4; ++b) Ts[(m0 + a) * nw + n0 + b] = acc[a][b];
+      for (int b = 0; b < 4; ++b) Ts[(m0 + a) * nwp + n0 + b] = acc[a][b];
     __syncthreads();
     const int hmode = herm[f] & 3;
+    VO* dst = Xbar + (k * nFrot + f) * (long long)nw2;
     if (hmode == 2) {  // diagonal only: Y_mm = sum_j conj(U_jm) T_jm, Hermitian part = Re
-      VO* dstd = Xbar + (k * nFrot + f) * (long long)nw2;
       for (int m = tid; m < nw; m += tpk) {
         V y = czero<V>();
-        for (int j = 0; j < nw; ++j) cfmac(y, Us[j * nw + m], Ts[j * nw + m]);
-        if (valid) dstd[m * nw + m] = rstore<VO>(real_only(y));
+        for (int j = 0; j < nw; ++j) cfmac(y, Us[j * nwp + m], Ts[j * nwp + m]);
+        if (valid) dst[m * nw + m] = rstore<VO>(real_only(y));
       }
-      __syncthreads();
-      continue;
+      continue;  // the next field's X has its own buffer; its barrier comes before T is written again
     }
 #pragma unroll
     for (int a = 0; a < 4; ++a)
@@ -185,30 +221,33 @@ __global__ void rotate_tiled(const typename C2<T>::t* __restrict__ U, long long 
     for (int j = 0; j < nw; ++j) {  // Y = U^dagger T
       V ua[4], tb[4];
 #pragma unroll
-      for (int a = 0; a < 4; ++a) ua[a] = Us[j * nw + m0 + a];
+      for (int a = 0; a < 4; ++a) ua[a] = Us[j * nwp + m0 + a];
 #pragma unroll
-      for (int b = 0; b < 4; ++b) tb[b] = Ts[j * nw + n0 + b];
+      for (int b = 0; b < 4; ++b) tb[b] = Ts[j * nwp + n0 + b];
 #pragma unroll
       for (int a = 0; a < 4; ++a)
 #pragma unroll
         for (int b = 0; b < 4; ++b) cfmac(acc[a][b], ua[a], tb[b]);
     }
+    if (hmode != 0) {  // Hermitian part: the transposed tile comes from shared memory (X is read)
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+      for (int a = 0; a < 4; ++a)
 #pragma unroll
-      for (int b = 0; b < 4; ++b) Xs[(m0 + a) * ldx + n0 + b] = acc[a][b];
-    __syncthreads();
-    VO* dst = Xbar + (k * nFrot + f) * (long long)nw2;
-    const bool h = hmode != 0;
-    if (valid) {
-      for (int i = tid; i < nw2; i += tpk) {
-        const int m = i / nw, n = i % nw;
-        V y = Xs[m * ldx + n];
-        if (h) y = herm_pair(y, Xs[n * ldx + m]);
-        dst[i] = rstore<VO>(y);
-      }
+        for (int b = 0; b < 4; ++b) Xs[(m0 + a) * ldx + n0 + b] = acc[a][b];
+      __syncthreads();
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) acc[a][b] = herm_pair(acc[a][b], Xs[(n0 + b) * ldx + m0 + a]);
+      __syncthreads();
     }
-    __syncthreads();
+    if (valid) {
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+          if (m0 + a < nw && n0 + b < nw) dst[(m0 + a) * nw + n0 + b] = rstore<VO>(acc[a][b]);
+    }
   }
 }
 
@@ -2165,11 +2204,12 @@ int launch_rotate(const void* U, long long strideU, const void* X, int nFin, con
                                                                    herm, nFrot, (VO*)Xbar, nw, nk);
     return wbg_cuda_status(cudaGetLastError());
   }
-  if (nw % 4 == 0 && nw >= 8) {
-    const int tpk = (nw / 4) * (nw / 4);
-    const size_t per_k = ((size_t)nw * nw * 2 + (size_t)nw * (nw + 1)) * sizeof(V);
+  if (nw >= 5) {
+    const int tpk = ((nw + 3) / 4) * ((nw + 3) / 4);
+    const size_t per_k = tiled_words(nw) * sizeof(V);
+    // k-points per block: up to 256 threads and 64 KB, but no fewer blocks than two per SM (152)
     int KB = 1;
-    while (KB * 2 * tpk <= 256 && (KB * 2) * per_k <= 64 * 1024) KB *= 2;
+    while (KB * 2 * tpk <= 256 && (KB * 2) * per_k <= 64 * 1024 && nk / (KB * 2) >= 304) KB *= 2;
     if (KB * per_k <= 200 * 1024) {
       const int t = wbg_tuned(WBG_TUNE_ROTATE_KPOINTS, sizeof(T) == 8 ? 1 : 0, nw);
       if (t > 0 && tiled_kpoints_fit(t, tpk, per_k)) KB = t;
@@ -2220,7 +2260,7 @@ int wbg_rotate_tune_candidates(int param, int nw, int variant, int* values, int 
   if (param != WBG_TUNE_ROTATE_KPOINTS || nw % 4 != 0 || nw < 8 || nw > 64) return 0;
   // the tiled kernel serves this (nw, precision) when its built-in block fits (launch_rotate)
   const int tpk = (nw / 4) * (nw / 4);
-  const size_t per_k = ((size_t)nw * nw * 2 + (size_t)nw * (nw + 1)) * (variant ? 16 : 8);
+  const size_t per_k = tiled_words(nw) * (variant ? 16 : 8);
   int KB = 1;
   while (KB * 2 * tpk <= 256 && (KB * 2) * per_k <= 64 * 1024) KB *= 2;
   if (KB * per_k > 200 * 1024) return 0;
