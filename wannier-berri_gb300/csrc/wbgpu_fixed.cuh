@@ -17,17 +17,32 @@
 
 typedef unsigned long long wbg_u64;
 
-// (lo, hi) of floor(v 2^60) for finite v
+// (lo, hi) of floor(v 2^60) for finite v, from the bits of v: the FP64 pipe issues 64 times slower than the
+// integer one, and its v 2^-4 - floor(v 2^-4) would round the fraction of a negative v
 WBG_D void fx_split(double v, wbg_u64& lo, wbg_u64& hi) {
-  const double t = v * 0x1p-4;  // v 2^60 / 2^64: exact scaling
-  double h = floor(t);
-  double f = (t - h) * 0x1p64;  // fraction in units of 2^-60, exact, in [0, 2^64]
-  if (f >= 0x1p64) {             // t - h rounded up to 1 (|t| far below one ulp of 1)
-    f = 0.0;
-    h += 1.0;
+  const wbg_u64 u = (wbg_u64)__double_as_longlong(v);
+  const int e = (int)(u >> 52) & 0x7ff;
+  const wbg_u64 m = (u & 0xfffffffffffffull) | (e ? 0x10000000000000ull : 0ull);
+  const int s = (e ? e : 1) - 1015;  // |v| 2^60 = m 2^s
+  bool frac = false;                 // a fraction was cut off |v| 2^60
+  if (s >= 128) {
+    lo = hi = 0;
+  } else if (s >= 64) {
+    lo = 0;
+    hi = m << (s - 64);
+  } else if (s > 0) {
+    lo = m << s;
+    hi = m >> (64 - s);
+  } else {
+    hi = 0;
+    lo = s > -64 ? m >> -s : 0;
+    frac = s > -64 ? (lo << -s) != m : m != 0;
   }
-  hi = (wbg_u64)(long long)h;
-  lo = (wbg_u64)f;
+  if ((long long)u < 0) {  // floor: minus the magnitude, one less where a fraction was cut off
+    lo = ~lo;
+    hi = ~hi;
+    if (!frac && ++lo == 0) ++hi;
+  }
 }
 
 // entry += (lo, hi): the carry of the low word is taken from the value the low word held right

@@ -245,35 +245,42 @@ WBG_D TetF make_tetf(float2 a, float2 b, float2 c, float2 d) {
   return q;
 }
 
+// Products and sums of the weights are written out: which of them the compiler fuses would otherwise depend on
+// the code around the call, and the weights' last bits with it.
 WBG_D float tetf_occ(const TetF& q, float x) {
   if (x >= q.g4) return 1.0f;
   if (x < 0.0f) return 0.0f;
   if (x >= q.g3) {
     const float y = q.g4 - x;
-    return 1.0f - (y * q.r41) * (y * q.r42) * (y * q.r43);
+    return __fmaf_rn(-__fmul_rn(__fmul_rn(y, q.r41), __fmul_rn(y, q.r42)), __fmul_rn(y, q.r43), 1.0f);
   }
   if (x >= q.g2) {
     const float x2 = x - q.g2;
-    const float a13 = x * q.r31, a14 = x * q.r41, a23 = x2 * q.r32, a24 = x2 * q.r42;
-    return a23 * a24 + a13 * (a14 * (1.0f - a24) + a24 * (1.0f - a23));
+    const float a13 = __fmul_rn(x, q.r31), a14 = __fmul_rn(x, q.r41);
+    const float a23 = __fmul_rn(x2, q.r32), a24 = __fmul_rn(x2, q.r42);
+    const float in = __fmaf_rn(a14, __fadd_rn(1.0f, -a24), __fmul_rn(a24, __fadd_rn(1.0f, -a23)));
+    return __fmaf_rn(a23, a24, __fmul_rn(a13, in));
   }
-  return (x * q.r21) * (x * q.r31) * (x * q.r41);
+  return __fmul_rn(__fmul_rn(__fmul_rn(x, q.r21), __fmul_rn(x, q.r31)), __fmul_rn(x, q.r41));
 }
 
 WBG_D float tetf_dos(const TetF& q, float x) {
   if (x >= q.g4 || x < 0.0f) return 0.0f;
   if (x >= q.g3) {
     const float y = q.g4 - x;
-    return 3.0f * y * y * (q.r41 * q.r42 * q.r43);
+    return __fmul_rn(__fmul_rn(__fmul_rn(3.0f, y), y), __fmul_rn(__fmul_rn(q.r41, q.r42), q.r43));
   }
   if (x >= q.g2) {
     const float x2 = x - q.g2;
-    const float a13 = x * q.r31, a14 = x * q.r41, a23 = x2 * q.r32, a24 = x2 * q.r42;
-    const float B = a14 * (1.0f - a24) + a24 * (1.0f - a23);
-    const float dB = q.r41 * (1.0f - a24) - a14 * q.r42 + q.r42 * (1.0f - a23) - a24 * q.r32;
-    return q.r32 * a24 + a23 * q.r42 + q.r31 * B + a13 * dB;
+    const float a13 = __fmul_rn(x, q.r31), a14 = __fmul_rn(x, q.r41);
+    const float a23 = __fmul_rn(x2, q.r32), a24 = __fmul_rn(x2, q.r42);
+    const float o24 = __fadd_rn(1.0f, -a24), o23 = __fadd_rn(1.0f, -a23), ra = __fmul_rn(q.r32, a24);
+    // B = a14 (1 - a24) + a24 (1 - a23), dB its derivative; r32 a24 + a23 r42 + r31 B + a13 dB
+    const float B = __fmaf_rn(a14, o24, __fmul_rn(a24, o23));
+    const float dB = __fadd_rn(__fmaf_rn(q.r42, o23, __fmaf_rn(q.r41, o24, -__fmul_rn(a14, q.r42))), -ra);
+    return __fmaf_rn(a13, dB, __fmaf_rn(q.r31, B, __fmaf_rn(a23, q.r42, ra)));
   }
-  return 3.0f * x * x * (q.r21 * q.r31 * q.r41);
+  return __fmul_rn(__fmul_rn(__fmul_rn(3.0f, x), x), __fmul_rn(__fmul_rn(q.r21, q.r31), q.r41));
 }
 
 // s += v, compensated (error-free two-sum into s.y)
@@ -300,127 +307,184 @@ WBG_D int lower_bound(const double* __restrict__ EF, int n, double x) {
   return lo;
 }
 
-constexpr int kWin = 32;  // Fermi levels per window chunk (per-lane column of shared memory)
-// shared memory per warp: window sums [kWin][32], level offsets [kWin][32] (FP32 weights only),
-// band energies [9][32]; 8 bytes each
-constexpr int kWarpSmem = (2 * kWin + 9) * 32;
+// a / 12 correctly rounded: Markstein's quotient correction with the rounded reciprocal of 12
+WBG_D double div12(double a) {
+  constexpr double r12 = 1.0 / 12.0;
+  const double q = a * r12;
+  return fma(fma(-12.0, q, a), r12, q);
+}
+
+constexpr int kLv = 8;        // lanes per band: one per corner, then one per Fermi level
+constexpr int kAccThr = 512;  // threads per block: 64 bands at a time
+// Shared data of one band: 9 energies, then its 12 tetrahedra in 16-byte pieces.  The stride puts the
+// pieces that a warp's four bands read at the same time into different banks.
+template <bool F32> struct BandTet;
+template <> struct BandTet<true> {
+  typedef TetF Q;
+  float2 e[9];
+  float pad0[2];
+  float4 q[12][3];
+  float pad1[4];
+};
+template <> struct BandTet<false> {
+  typedef Tet Q;
+  double e[9];
+  double pad0;
+  double2 q[12][5];
+  double pad1[2];
+};
+static_assert(sizeof(BandTet<true>) % 128 == 32 && sizeof(BandTet<false>) % 128 == 32, "four bands, four bank groups");
+WBG_D void put_tet(BandTet<true>& b, int t, const TetF& q) {
+  b.q[t][0] = make_float4(q.c_hi, q.c_lo, q.g2, q.g3);
+  b.q[t][1] = make_float4(q.g4, q.r21, q.r31, q.r41);
+  b.q[t][2] = make_float4(q.r32, q.r42, q.r43, 0.f);
+}
+WBG_D TetF get_tet(const BandTet<true>& b, int t) {
+  const float4 x = b.q[t][0], y = b.q[t][1], z = b.q[t][2];
+  TetF q;
+  q.c_hi = x.x; q.c_lo = x.y; q.g2 = x.z; q.g3 = x.w;
+  q.g4 = y.x; q.r21 = y.y; q.r31 = y.z; q.r41 = y.w;
+  q.r32 = z.x; q.r42 = z.y; q.r43 = z.z;
+  return q;
+}
+WBG_D void put_tet(BandTet<false>& b, int t, const Tet& q) {
+  b.q[t][0] = make_double2(q.e1, q.e2);
+  b.q[t][1] = make_double2(q.e3, q.e4);
+  b.q[t][2] = make_double2(q.r21, q.r31);
+  b.q[t][3] = make_double2(q.r41, q.r32);
+  b.q[t][4] = make_double2(q.r42, q.r43);
+}
+WBG_D Tet get_tet(const BandTet<false>& b, int t) {
+  const double2 x = b.q[t][0], y = b.q[t][1], z = b.q[t][2], u = b.q[t][3], v = b.q[t][4];
+  Tet q;
+  q.e1 = x.x; q.e2 = x.y; q.e3 = y.x; q.e4 = y.y;
+  q.r21 = z.x; q.r31 = z.y; q.r41 = u.x; q.r32 = u.y; q.r42 = v.x; q.r43 = v.y;
+  return q;
+}
 
 // ---------------------------------------------------------------------------------------
-// Weighted accumulation.  Lane n takes band n of its warp's k-point: for sel 1 the band weight
-// w(E_F) = (1/12) sum over the 12 tetrahedra, evaluated on the levels between the band's
-// smallest and largest corner energy (0 below, 1 (der 0) / 0 (der 1) above); for sel 2 the
-// weight is 1 everywhere (the Fermi sea, der 0).  hist gets the contribution P[k][n] w(E_F) in
-// difference form -- hist[i] += P (w(i) - w(i-1)) -- so that the cumulative scan of
-// wbg_scan_finalize returns sum P w.  F32: weights in FP32 (mixed precision, see TetF); else
-// the reference's FP64 arithmetic.  smem: the block's [nEF][nc] histogram when it fits (else
-// atomics go to hist directly) + kWarpSmem doubles per warp.
+// Weighted accumulation.  For sel 1 the band weight w(E_F) = (1/12) sum over the 12 tetrahedra,
+// evaluated on the levels between the band's smallest and largest corner energy (0 below, 1 (der 0) /
+// 0 (der 1) above); for sel 2 the weight is 1 everywhere (the Fermi sea, der 0).  hist gets the
+// contribution P[k][n] w(E_F) in difference form -- hist[i] += P (w(i) - w(i-1)) -- so that the
+// cumulative scan of wbg_scan_finalize returns sum P w.  F32: weights in FP32 (mixed precision, see
+// TetF); else the reference's FP64 arithmetic.
+// A warp takes 32 bands, keeps those with sel 1 and works on four at a time: 8 lanes read a band's 8
+// corners, build its 12 tetrahedra in shared memory and then take a level each, summing over the
+// tetrahedra in order in registers.  Bound by instruction issue and the histogram's integer atomics;
+// with a lane per band (window sums in shared memory, 75 KB a block of 4 warps and one block an SM) the
+// same levels took 6.0 ms at num_wann 32, 13 824 k-points, 1 001 levels; now 0.34 ms, the same weights
+// bit for bit.  smem: the block's [nEF][nc] histogram when it fits (else atomics go to hist directly).
 // ---------------------------------------------------------------------------------------
 template <bool F32>
-__global__ void tetra_accumulate_kernel(const double* __restrict__ E, const double* __restrict__ Ec,
-                                        const int* __restrict__ slot, const int* __restrict__ blocks,
-                                        wbg_tetra_grid g, int nw, long long nkt, const signed char* __restrict__ sel,
-                                        const double* __restrict__ P, int nc, const double* __restrict__ EF, int nEF,
-                                        int der, int ascending, int smem_hist, wbg_u64* __restrict__ hist) {
-  extern __shared__ double sm[];
-  const int G = blockDim.x / 32, w = threadIdx.x / 32, lane = threadIdx.x % 32;
+__global__ void __launch_bounds__(kAccThr, F32 ? 2 : 1)
+    tetra_accumulate_kernel(const double* __restrict__ E, const double* __restrict__ Ec, const int* __restrict__ slot,
+                            const int* __restrict__ blocks, wbg_tetra_grid g, int nw, long long nkt,
+                            const signed char* __restrict__ sel, const double* __restrict__ P, int nc,
+                            const double* __restrict__ EF, int nEF, int der, int ascending, int smem_hist,
+                            wbg_u64* __restrict__ hist) {
+  extern __shared__ __align__(16) unsigned char smt[];
+  BandTet<F32>* bands = reinterpret_cast<BandTet<F32>*>(smt);
+  const int lane = threadIdx.x % 32, l8 = lane % kLv, g4 = lane / kLv;
   const int nh = nEF * nc;  // fixed-point histogram entries (wbgpu_fixed.cuh)
-  wbg_u64* acc = smem_hist ? reinterpret_cast<wbg_u64*>(sm) : hist;
+  wbg_u64* acc = smem_hist ? reinterpret_cast<wbg_u64*>(bands + kAccThr / kLv) : hist;
   wbg_u64* bad = acc + 2 * nh;  // count of non-finite contributions
-  double* win = sm + (smem_hist ? fx_words(nh) : 0) + (size_t)w * kWarpSmem;
-  float2* winf = reinterpret_cast<float2*>(win);            // F32: compensated window sums
-  float2* xs = reinterpret_cast<float2*>(win + kWin * 32);  // F32: E_F - eb per level
-  double* ek = win + 2 * kWin * 32;                         // [9][32]: corner s at s * 32 + lane
-  float2* ekf = reinterpret_cast<float2*>(ek);              // F32: e - eb as (hi, lo)
+  BandTet<F32>& my = bands[threadIdx.x / kLv];
   if (smem_hist) {
     fx_zero(acc, nh);
     __syncthreads();
   }
   const double wend = der == 0 ? 1.0 : 0.0;
-  for (long long kk = (long long)blockIdx.x * G + w; kk < nkt; kk += (long long)gridDim.x * G) {
-    for (int n = lane; n < nw; n += 32) {
-      const int s = sel[kk * nw + n];
-      if (s == 0) continue;
-      const double* Pn = P + (kk * nw + n) * nc;
-      if (s == 2) {  // Fermi sea: weight 1 at every level
-        if (der == 0)
-          for (int c = 0; c < nc; ++c) {
-            fx_add_double(acc + 2 * c, Pn[c], bad);
-          }
-        continue;
-      }
-      double pv[9];  // the band's values in registers; more than 9 components are read from P
-      for (int c = 0; c < nc && c < 9; ++c) pv[c] = Pn[c];
-      const double e0 = E[kk * nw + n];
-      double lo = e0, hi = e0;
-      double ev[8];
+  const long long total = nkt * nw;
+  const long long step = (long long)gridDim.x * kAccThr;
+  for (long long base = (long long)blockIdx.x * kAccThr + (threadIdx.x & ~31); base < total; base += step) {
+    const int s = base + lane < total ? sel[base + lane] : 0;
+    if (s == 2 && der == 0) {  // Fermi sea: weight 1 at every level
+      const double* Pn = P + (base + lane) * nc;
+      for (int c = 0; c < nc; ++c) fx_add_double(acc + 2 * c, Pn[c], bad);
+    }
+    unsigned todo = __ballot_sync(0xffffffffu, s == 1);
+    while (todo) {  // warp-uniform
+      // the g4-th of the next four bands
+      unsigned mine = todo;
+      for (int q = 0; q < g4; ++q) mine &= mine - 1;
+      for (int q = 0; q < 4; ++q) todo &= todo - 1;
+      const bool has = mine != 0;
+      const long long kn = base + (has ? __ffs(mine) - 1 : 0);
+      const long long kk = kn / nw;
+      const int n = (int)(kn - kk * nw);
+      const double e0 = E[kn], ev = Ec[corner_row(g, blocks, slot, kk, l8) * nw + n];
+      double lo = fmin(e0, ev), hi = fmax(e0, ev);
 #pragma unroll
-      for (int s8 = 0; s8 < 8; ++s8) {
-        ev[s8] = Ec[corner_row(g, blocks, slot, kk, s8) * nw + n];
-        lo = fmin(lo, ev[s8]);
-        hi = fmax(hi, ev[s8]);
+      for (int off = 1; off < kLv; off <<= 1) {
+        lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, off));
+        hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, off));
       }
+      __syncwarp();  // the previous four bands' data is read
       if constexpr (F32) {
-#pragma unroll
-        for (int s8 = 0; s8 < 8; ++s8) ekf[s8 * 32 + lane] = split_df(ev[s8] - lo);
-        ekf[8 * 32 + lane] = split_df(e0 - lo);
+        my.e[l8] = split_df(ev - lo);
+        if (l8 == 0) my.e[8] = split_df(e0 - lo);
       } else {
-#pragma unroll
-        for (int s8 = 0; s8 < 8; ++s8) ek[s8 * 32 + lane] = ev[s8];
+        my.e[l8] = ev;
+        if (l8 == 0) my.e[8] = e0;
       }
+      __syncwarp();
+      for (int t = l8; t < 12; t += kLv) {
+        if constexpr (F32)
+          put_tet(my, t, make_tetf(my.e[8], my.e[kTetra[t][0]], my.e[kTetra[t][1]], my.e[kTetra[t][2]]));
+        else
+          put_tet(my, t, make_tet(my.e[8], my.e[kTetra[t][0]], my.e[kTetra[t][1]], my.e[kTetra[t][2]]));
+      }
+      __syncwarp();
       // below lo every weight is 0; from i1 on, E_F exceeds every (separated) tetrahedron top
       int i0 = 0, i1 = nEF;
       if (ascending) {
         i0 = lower_bound(EF, nEF, lo);
         i1 = lower_bound(EF, nEF, hi + 4e-12);
       }
-      double wprev = 0.0;
-      for (int c0 = i0; c0 < i1; c0 += kWin) {
-        const int cn = min(kWin, i1 - c0);
+      if (!has) i0 = i1 = nEF;
+      const double* Pn = P + kn * nc;
+      double wprev = 0.0;  // weight of the level before this chunk
+      const int nchunk = (max(i1 - i0, 0) + kLv - 1) / kLv;
+      const int rounds = __reduce_max_sync(0xffffffffu, nchunk);
+      for (int r = 0; r < rounds; ++r) {
+        const int i = i0 + r * kLv + l8;
+        const bool on = i < i1;
+        const double ef = on ? __ldg(EF + i) : 0.0;
+        double wi;
         if constexpr (F32) {
-          for (int i = 0; i < cn; ++i) {
-            winf[i * 32 + lane] = make_float2(0.0f, 0.0f);
-            xs[i * 32 + lane] = split_df(__ldg(EF + c0 + i) - lo);
-          }
-        } else {
-          for (int i = 0; i < cn; ++i) win[i * 32 + lane] = 0.0;
-        }
-#pragma unroll 1
-        for (int t = 0; t < 12; ++t) {
-          if constexpr (F32) {
-            const TetF q = make_tetf(ekf[8 * 32 + lane], ekf[kTetra[t][0] * 32 + lane], ekf[kTetra[t][1] * 32 + lane],
-                                     ekf[kTetra[t][2] * 32 + lane]);
-            for (int i = 0; i < cn; ++i) {
-              const float2 xb = xs[i * 32 + lane];
+          const float2 xb = split_df(ef - lo);
+          float2 sum = make_float2(0.0f, 0.0f);
+          if (on) {
+#pragma unroll 2
+            for (int t = 0; t < 12; ++t) {
+              const TetF q = get_tet(my, t);
               const float x = (xb.x - q.c_hi) + (xb.y - q.c_lo);
-              two_sum_add(winf[i * 32 + lane], der == 0 ? tetf_occ(q, x) : tetf_dos(q, x));
+              two_sum_add(sum, der == 0 ? tetf_occ(q, x) : tetf_dos(q, x));
             }
-          } else {
-            const Tet q = make_tet(e0, ek[kTetra[t][0] * 32 + lane], ek[kTetra[t][1] * 32 + lane],
-                                   ek[kTetra[t][2] * 32 + lane]);
-            if (der == 0)
-              for (int i = 0; i < cn; ++i) win[i * 32 + lane] += tet_occ(q, __ldg(EF + c0 + i));
-            else
-              for (int i = 0; i < cn; ++i) win[i * 32 + lane] += tet_dos(q, __ldg(EF + c0 + i));
           }
-        }
-        for (int i = 0; i < cn; ++i) {
-          double wi;
-          if constexpr (F32) {
-            const float2 v = winf[i * 32 + lane];
-            wi = ((double)v.x + (double)v.y) / 12.0;
-          } else {
-            wi = win[i * 32 + lane] / 12.0;
+          wi = div12((double)sum.x + (double)sum.y);
+        } else {
+          double sum = 0.0;
+          if (on) {
+            for (int t = 0; t < 12; ++t) {
+              const Tet q = get_tet(my, t);
+              sum += der == 0 ? tet_occ(q, ef) : tet_dos(q, ef);
+            }
           }
-          const double d = wi - wprev;
-          wprev = wi;
-          if (d != 0.0)
-            for (int c = 0; c < nc; ++c)
-              fx_add_double(acc + 2 * ((c0 + i) * nc + c), (nc <= 9 ? pv[c] : Pn[c]) * d, bad);
+          wi = div12(sum);
         }
+        const double before = __shfl_up_sync(0xffffffffu, wi, 1, kLv);
+        const double d = wi - (l8 == 0 ? wprev : before);
+        // the last level of the chunk (of the window) is the next chunk's predecessor
+        const int last = min(kLv, i1 - i0 - r * kLv) - 1;
+        const double wl = __shfl_sync(0xffffffffu, wi, last < 0 ? 0 : last, kLv);
+        if (last >= 0) wprev = wl;
+        if (on && d != 0.0)
+          for (int c = 0; c < nc; ++c) fx_add_double(acc + 2 * (i * nc + c), Pn[c] * d, bad);
       }
-      if (i1 < nEF && wend != wprev)
-        for (int c = 0; c < nc; ++c)
-          fx_add_double(acc + 2 * (i1 * nc + c), (nc <= 9 ? pv[c] : Pn[c]) * (wend - wprev), bad);
+      if (has && l8 == 0 && i1 < nEF && wend != wprev)
+        for (int c = 0; c < nc; ++c) fx_add_double(acc + 2 * (i1 * nc + c), Pn[c] * (wend - wprev), bad);
     }
   }
   if (smem_hist) {
@@ -468,20 +532,19 @@ int wbg_tetra_accumulate_run(const double* E, const double* Ec, const int* slot,
     return WBG_ERR_ARG;
   if (ncomp < 1 || ncomp > 81 || der < 0 || der > 1 || fp64 < 0 || fp64 > 1) return WBG_ERR_ARG;
   const long long nkt = (long long)nblocks * g->fft[0] * g->fft[1] * g->fft[2];
-  const int G = 4;
-  const size_t wsm = (size_t)G * kWarpSmem * 8;
   const size_t hsm = fx_words((size_t)nEF * ncomp) * 8;
+  const size_t wsm = (size_t)(kAccThr / kLv) * (fp64 ? sizeof(BandTet<false>) : sizeof(BandTet<true>));
   const int smem_hist = wsm + hsm <= 200 * 1024;
   const size_t sm = wsm + (smem_hist ? hsm : 0);
-  const int nblk = grid_cap(G, nkt, 4);
+  const int nblk = grid_cap(kAccThr, nkt * nw, fp64 ? 1 : 2);
   if (fp64) {
     cudaFuncSetAttribute(tetra_accumulate_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    tetra_accumulate_kernel<false><<<nblk, 32 * G, sm, stream>>>(E, Ec, slot, blocks, *g, nw, nkt, sel, P, ncomp, EF,
-                                                                 nEF, der, ascending, smem_hist, (wbg_u64*)hist);
+    tetra_accumulate_kernel<false><<<nblk, kAccThr, sm, stream>>>(E, Ec, slot, blocks, *g, nw, nkt, sel, P, ncomp, EF,
+                                                                  nEF, der, ascending, smem_hist, (wbg_u64*)hist);
   } else {
     cudaFuncSetAttribute(tetra_accumulate_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    tetra_accumulate_kernel<true><<<nblk, 32 * G, sm, stream>>>(E, Ec, slot, blocks, *g, nw, nkt, sel, P, ncomp, EF,
-                                                                nEF, der, ascending, smem_hist, (wbg_u64*)hist);
+    tetra_accumulate_kernel<true><<<nblk, kAccThr, sm, stream>>>(E, Ec, slot, blocks, *g, nw, nkt, sel, P, ncomp, EF,
+                                                                 nEF, der, ascending, smem_hist, (wbg_u64*)hist);
   }
   return wbg_cuda_status(cudaGetLastError());
 }
