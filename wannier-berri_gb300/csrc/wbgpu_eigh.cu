@@ -16,6 +16,7 @@
 // df64 (double-float on the FP32 pipe, 48-bit significand) for the mixed-precision path.
 // The back-transform runs in precision TU (double or float).
 #include <float.h>
+#include <type_traits>
 #include "wbgpu_common.cuh"
 #include "wbgpu_df64.cuh"
 #include "wbgpu_eigh.cuh"
@@ -294,10 +295,178 @@ __global__ void eigh_tridiag(const HIn* __restrict__ H, long long strideK, int n
 }
 
 // ---------------------------------------------------------------------------------------
+// The same reduction for n > 32: one matrix per block of 4 n threads.  A batch of large matrices is
+// small (512 of 96 x 96) and two or three fit an SM's shared memory, so a group of 16 lanes a matrix
+// leaves an SM with a warp or two.  Here a row's matrix-vector product takes four threads (one for each of
+// its accumulators) and the rank-2 update a thread per element; the short sums over rows (norm,
+// w^dagger v) stay with 16 lanes in eigh_tridiag's order, so the double-float result has the same bits.
+// Bound by its dependent steps: five block barriers a column.  512 matrices in double-float: 96 x 96 6.15 ->
+// 1.93 ms, 82 x 82 2.5 -> 1.42 ms.
+// ---------------------------------------------------------------------------------------
+constexpr int TW_THR = 512, TW_L = 16;  // most threads a block; lanes of the sums over rows
+
+template <typename R, typename HIn, typename TV>
+__global__ void __launch_bounds__(TW_THR, 2)
+    eigh_tridiag_wide(const HIn* __restrict__ H, long long strideK, int n, int lowerIn,
+                      typename C2<TV>::t* __restrict__ Vh, typename C2<TV>::t* __restrict__ tauOut,
+                      R* __restrict__ dOut, R* __restrict__ eOut) {
+  typedef typename C2<R>::t CR;
+  typedef typename C2<TV>::t CV;
+  typedef Arith<R> A;
+  extern __shared__ __align__(16) unsigned char smt[];
+  const long long k = blockIdx.x;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  CR* Am = reinterpret_cast<CR*>(smt);  // packed lower triangle
+  CR* vs = Am + tri(n);
+  CR* ws = vs + n;
+  CR* sh = ws + n;  // tau, scale, -1/2 tau w^dagger v, (beta, 0)
+  const HIn* Hk = H + k * strideK;
+  for (int idx = tid; idx < n * n; idx += blockDim.x) {
+    const int i = idx / n, j = idx - i * n;
+    if (j <= i)
+      Am[tri(i) + j] = lowerIn ? lower_elem<R>(Hk[i * n + j], i == j) : herm_avg<R>(Hk[i * n + j], Hk[j * n + i]);
+  }
+  __syncthreads();
+  const R zero = A::from(0.0), one = A::from(1.0), mhalf = A::from(-0.5);
+  const int T = (n + 2 * TW_L - 1) / (2 * TW_L);
+  for (int c = 0; c < n - 1; ++c) {
+    if (warp == 0) {
+      R xn = zero;
+      if (lane < TW_L)
+        for (int t = 0; t < T; ++t)
+          for (int h = 0; h < 2; ++h) {
+            const int i = owned_row(t, h, lane, TW_L);
+            if (i < n && i >= c + 2) { const CR x = Am[tri(i) + c]; xn = fma(x.x, x.x, fma(x.y, x.y, xn)); }
+          }
+      xn = group_sum(xn, TW_L);
+      const CR alpha = Am[tri(c + 1) + c];
+      CR tau = czero<CR>(), scale = czero<CR>(), b = czero<CR>();
+      if (xn == zero && alpha.y == zero) {
+        b.x = alpha.x;  // H = I
+      } else {
+        const R nrm = sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xn);
+        const R beta = alpha.x >= zero ? -nrm : nrm;
+        b.x = beta;
+        const R rb = one / beta;
+        tau.x = (beta - alpha.x) * rb;
+        tau.y = -alpha.y * rb;
+        const R ar = alpha.x - beta, ai = alpha.y;  // scale = 1 / (alpha - beta)
+        const R rden = one / (ar * ar + ai * ai);
+        scale.x = ar * rden;
+        scale.y = -ai * rden;
+      }
+      if (lane == 0) {
+        sh[0] = tau;
+        sh[1] = scale;
+        sh[3] = b;
+      }
+    }
+    __syncthreads();
+    const CR tau = sh[0];
+    if (tid >= c + 1 && tid < n) {
+      const int i = tid;
+      CR v;
+      v.x = one;
+      v.y = zero;
+      if (i >= c + 2) v = cmul(Am[tri(i) + c], sh[1]);
+      vs[i] = v;
+      Am[tri(i) + c] = v;
+    }
+    __syncthreads();
+    {  // p = tau A v: thread q of a row's four takes every second element of the lower (0, 1) or upper (2, 3) part
+      const int i = c + 1 + (tid >> 2), q = tid & 3;
+      CR acc = czero<CR>();
+      if (i < n) {
+        if (q < 2) {
+          const CR* Ai = Am + tri(i);
+          for (int j = c + 1 + q; j <= i; j += 2) lz_cfma(acc, Ai[j], vs[j]);
+        } else {
+          for (int j = i + q - 1; j < n; j += 2) lz_cfmac(acc, Am[tri(j) + i], vs[j]);
+        }
+        acc = lz_cdone(acc);
+      }
+      acc.x = acc.x + shfl_xor(acc.x, 1);
+      acc.y = acc.y + shfl_xor(acc.y, 1);
+      acc.x = acc.x + shfl_xor(acc.x, 2);
+      acc.y = acc.y + shfl_xor(acc.y, 2);
+      if (i < n && q == 0) ws[i] = cmul(tau, acc);
+    }
+    __syncthreads();
+    if (warp == 0) {
+      R dr = zero, di = zero;
+      if (lane < TW_L)
+        for (int t = 0; t < T; ++t)
+          for (int h = 0; h < 2; ++h) {
+            const int i = owned_row(t, h, lane, TW_L);
+            if (i < n && i >= c + 1) {
+              const CR p = ws[i], v = vs[i];
+              dr = fma(p.x, v.x, fma(p.y, v.y, dr));  // conj(p) v
+              di = fma(p.x, v.y, fma(-p.y, v.x, di));
+            }
+          }
+      dr = group_sum(dr, TW_L);
+      di = group_sum(di, TW_L);
+      CR dd;
+      dd.x = dr;
+      dd.y = di;
+      if (lane == 0) sh[2] = cscale(cmul(tau, dd), mhalf);
+    }
+    __syncthreads();
+    if (tid >= c + 1 && tid < n) {
+      CR w = ws[tid];
+      cfma(w, sh[2], vs[tid]);
+      ws[tid] = w;
+    }
+    __syncthreads();
+    // lower-triangle rank-2 update: A[i][j] -= v_i conj(w_j) + w_i conj(v_j), c+1 <= j <= i
+    for (int i = c + 1 + warp; i < n; i += blockDim.x / 32) {
+      const CR vi = vs[i], wi = ws[i];
+      CR* Ai = Am + tri(i);
+      for (int j = c + 1 + lane; j <= i; j += 32) {
+        CR a = Ai[j];
+        const CR vj = vs[j], wj = ws[j];
+        lz_fma(a.x, -vi.x, wj.x);
+        lz_fma(a.x, -vi.y, wj.y);
+        lz_fma(a.x, -wi.x, vj.x);
+        lz_fma(a.x, -wi.y, vj.y);
+        lz_fma(a.y, -vi.y, wj.x);
+        lz_fma(a.y, vi.x, wj.y);
+        lz_fma(a.y, -wi.y, vj.x);
+        lz_fma(a.y, wi.x, vj.y);
+        Ai[j] = lz_cdone(a);
+      }
+    }
+    const bool refl = (tau.x != zero || tau.y != zero);
+    if (tid < n) Vh[(k * n + c) * n + tid] = (refl && tid >= c + 1) ? to_tu_c<TV>(Am[tri(tid) + c]) : czero<CV>();
+    if (tid == 0) {
+      tauOut[k * n + c] = to_tu_c<TV>(tau);
+      eOut[k * n + c] = sh[3].x;
+      dOut[k * n + c] = Am[tri(c) + c].x;
+    }
+    __syncthreads();
+  }
+  if (tid == 0) {
+    dOut[k * n + n - 1] = Am[tri(n - 1) + n - 1].x;
+    eOut[k * n + n - 1] = zero;
+    tauOut[k * n + n - 1] = czero<CV>();
+  }
+  if (tid < n) Vh[(k * n + n - 1) * n + tid] = czero<CV>();
+}
+
+// ---------------------------------------------------------------------------------------
 // 2. Implicit QL eigenvalues of the real symmetric tridiagonal (d, e), thread per matrix.
 // d and e of thread t live in shared memory at [i * blockDim + t] (conflict-free, no
 // local-memory traffic).
 // ---------------------------------------------------------------------------------------
+// a b, a b + c d and a b - c of the QL rotations.  FP64 names its roundings, so that the two kernels below
+// give the same bits whatever the compiler would fuse in each.
+template <typename R> WBG_D R ql_mul(R a, R b) { return a * b; }
+template <typename R> WBG_D R ql_lin(R a, R b, R c, R d) { return a * b + c * d; }
+template <typename R> WBG_D R ql_mulsub(R a, R b, R c) { return a * b - c; }
+template <> WBG_D double ql_mul(double a, double b) { return __dmul_rn(a, b); }
+template <> WBG_D double ql_lin(double a, double b, double c, double d) { return __fma_rn(a, b, __dmul_rn(c, d)); }
+template <> WBG_D double ql_mulsub(double a, double b, double c) { return __fma_rn(a, b, -c); }
+
 template <typename R>
 __global__ void eigh_ql(const R* __restrict__ dIn, const R* __restrict__ eIn, int n, int nk, double* __restrict__ Eout,
                         int* __restrict__ errflag) {
@@ -329,20 +498,20 @@ __global__ void eigh_ql(const R* __restrict__ dIn, const R* __restrict__ eIn, in
         R s = one, c = one, p = zero;
         bool underflow = false;
         for (int i = m - 1; i >= l; --i) {
-          const R f = s * e(i);
-          const R b = c * e(i);
+          const R f = ql_mul(s, e(i));
+          const R b = ql_mul(c, e(i));
           // Givens rotation: one sqrt and one reciprocal (f, g are O(|T|): no overflow concern)
-          r = sqrt(fma(f, f, g * g));
+          r = sqrt(fma(f, f, ql_mul(g, g)));
           e(i + 1) = r;
           if (r == zero) { d(i + 1) = d(i + 1) - p; e(m) = zero; underflow = true; break; }
           const R rinv = one / r;
-          s = f * rinv;
-          c = g * rinv;
+          s = ql_mul(f, rinv);
+          c = ql_mul(g, rinv);
           g = d(i + 1) - p;
-          r = (d(i) - g) * s + two * c * b;
-          p = s * r;
+          r = ql_lin(d(i) - g, s, two * c, b);
+          p = ql_mul(s, r);
           d(i + 1) = g + p;
-          g = c * r - b;
+          g = ql_mulsub(c, r, b);
         }
         if (underflow) continue;
         d(l) = d(l) - p;
@@ -363,6 +532,99 @@ __global__ void eigh_ql(const R* __restrict__ dIn, const R* __restrict__ eIn, in
   for (int i = 0; i < n; ++i) Eout[k * n + i] = A::to(d(i));
 }
 
+// The same sweep with a warp per matrix, for batches too small to fill the SMs otherwise: every lane runs
+// the (serial) rotations on the same values, the search for a negligible off-diagonal element and the
+// final sort, a third of the time in one thread, are shared by the lanes.  The same comparisons and
+// rotations: the same bits.  512 double-float matrices of 96 x 96: 4.7 (a thread each) -> 3.7 ms.
+constexpr int QW_WARPS = 4;  // matrices per block
+template <typename R>
+__global__ void __launch_bounds__(32 * QW_WARPS)
+    eigh_ql_warp(const R* __restrict__ dIn, const R* __restrict__ eIn, int n, int nk, double* __restrict__ Eout,
+                 int* __restrict__ errflag) {
+  typedef Arith<R> A;
+  extern __shared__ unsigned char smq[];
+  const int lane = threadIdx.x & 31;
+  const long long k = (long long)blockIdx.x * QW_WARPS + (threadIdx.x >> 5);
+  if (k >= nk) return;
+  R* ds = reinterpret_cast<R*>(smq) + (size_t)(threadIdx.x >> 5) * 2 * n;
+  R* es = ds + n;
+  auto d = [&](int i) -> R& { return ds[i]; };
+  auto e = [&](int i) -> R& { return es[i]; };
+  const R zero = A::from(0.0), one = A::from(1.0), two = A::from(2.0), eps = A::eps();
+  for (int i = lane; i < n; i += 32) {
+    ds[i] = dIn[k * n + i];
+    es[i] = i < n - 1 ? eIn[k * n + i] : zero;
+  }
+  __syncwarp();
+  bool ok = true;
+  for (int l = 0; l < n; ++l) {
+    int iter = 0, m;
+    do {
+      __syncwarp();
+      m = n - 1;
+      for (int base = l; base < n - 1; base += 32) {  // the first m >= l with |e(m)| negligible
+        const int i = base + lane;
+        const bool hit = i < n - 1 && fabs(es[i]) <= eps * (fabs(ds[i]) + fabs(ds[i + 1]));
+        const unsigned hits = __ballot_sync(0xffffffffu, hit);
+        if (hits) {
+          m = base + __ffs(hits) - 1;
+          break;
+        }
+      }
+      __syncwarp();
+      if (m != l) {
+        if (iter++ >= 60) { ok = false; break; }
+        R g = (d(l + 1) - d(l)) / (two * e(l));
+        R r = sqrt(fma(g, g, one));
+        g = d(m) - d(l) + e(l) / (g + copysign(r, g));
+        R s = one, c = one, p = zero;
+        bool underflow = false;
+        // d(i + 1) is the value read as d(i) one step before; the next step's e and d are read ahead of
+        // this one's stores, off the chain of dependent operations
+        R di1 = d(m), en = e(m - 1), dn = d(m - 1);
+        for (int i = m - 1; i >= l; --i) {
+          const R ei = en, di = dn;
+          if (i > l) {
+            en = e(i - 1);
+            dn = d(i - 1);
+          }
+          const R f = ql_mul(s, ei);
+          const R b = ql_mul(c, ei);
+          // Givens rotation: one sqrt and one reciprocal (f, g are O(|T|): no overflow concern)
+          r = sqrt(fma(f, f, ql_mul(g, g)));
+          e(i + 1) = r;
+          if (r == zero) { d(i + 1) = di1 - p; e(m) = zero; underflow = true; break; }
+          const R rinv = one / r;
+          s = ql_mul(f, rinv);
+          c = ql_mul(g, rinv);
+          g = di1 - p;
+          r = ql_lin(di - g, s, two * c, b);
+          p = ql_mul(s, r);
+          d(i + 1) = g + p;
+          g = ql_mulsub(c, r, b);
+          di1 = di;
+        }
+        if (underflow) continue;
+        d(l) = d(l) - p;
+        e(l) = g;
+        e(m) = zero;
+      }
+    } while (m != l);
+    if (!ok) break;
+  }
+  if (!ok && lane == 0) atomicOr(errflag, WBG_FLAG_QL_NOCONV);
+  __syncwarp();
+  bool nan = false;
+  for (int i = lane; i < n; i += 32) nan |= ds[i] != ds[i];
+  nan = __any_sync(0xffffffffu, nan);  // not ordered: left as it is
+  for (int i = lane; i < n; i += 32) {
+    const R x = ds[i];
+    int r = 0;
+    for (int j = 0; j < n; ++j) r += ds[j] < x || (ds[j] == x && j < i);
+    Eout[k * n + (nan ? i : r)] = A::to(x);
+  }
+}
+
 WBG_D double hash_uniform(unsigned int a, unsigned int b) {
   unsigned int h = a * 2654435761u ^ (b + 0x9e3779b9u + (a << 6) + (a >> 2));
   h ^= h >> 16; h *= 0x7feb352du; h ^= h >> 15; h *= 0x846ca68bu; h ^= h >> 16;
@@ -372,7 +634,10 @@ WBG_D double hash_uniform(unsigned int a, unsigned int b) {
 // ---------------------------------------------------------------------------------------
 // 3. Eigenvectors: inverse iteration on T (real type R, two solves from a pseudo-random
 //    start), clusters re-orthogonalised, U = Q Z.
-// grid: ceil(nk/G) blocks of G*L threads; lane j computes eigenvectors j, j+L, ...
+// grid: ceil(nk/G) blocks of G*L threads; lane j computes eigenvectors j, j+L, ...  For n > 32 a
+// matrix takes a block of its own with a thread per column (L = 32 ceil(n / 32), G = 1): with one warp a
+// matrix, 96 x 96 left three columns to a lane and a warp to an SM (512 matrices in double-float: 10.3 ->
+// 3.74 ms; every column's arithmetic is its own, so the bits are the same).
 // The back-transform by the Householder reflectors runs in precision TU, one reflector at a
 // time staged in shared memory for all lanes.  Shared memory per group: Z [n][n], d, e,
 // lam [n] (type R), then U[n][n] and the staged reflector [n], complex(TU).  The iterate of
@@ -388,6 +653,12 @@ constexpr bool kUOverlaysZ = sizeof(typename C2<TU>::t) == sizeof(R);
 // rows 2i and 2i+1 of Z, which are read by then), so the group needs U's region only
 template <typename R, typename TU>
 constexpr bool kUWideOverlay = sizeof(typename C2<TU>::t) == 2 * sizeof(R);
+
+// barrier of a group of L lanes: within a warp, or the whole block (L > 32, one group a block)
+WBG_D void group_sync(int L) {
+  if (L > 32) __syncthreads();
+  else __syncwarp();
+}
 
 template <typename R, typename TU, typename VO>
 __global__ void eigh_vectors(const typename C2<TU>::t* __restrict__ Vh, const typename C2<TU>::t* __restrict__ tauIn,
@@ -414,7 +685,7 @@ __global__ void eigh_vectors(const typename C2<TU>::t* __restrict__ Vh, const ty
                                          : reinterpret_cast<VU*>(gbase + zbytes);  // [i][j-c0]
   VU* vsh = reinterpret_cast<VU*>(gbase + regbytes);
   for (int i = lane; i < n; i += L) { ds[i] = dIn[k * n + i]; es[i] = eIn[k * n + i]; lam[i] = A::from(E[k * n + i]); }
-  __syncwarp();
+  group_sync(L);
   const R zero = A::from(0.0), one = A::from(1.0);
   R tnorm = zero;
   for (int i = 0; i < n; ++i) tnorm = fmax(tnorm, fabs(ds[i]) + fabs(es[i]) + (i > 0 ? fabs(es[i - 1]) : zero));
@@ -479,7 +750,7 @@ __global__ void eigh_vectors(const typename C2<TU>::t* __restrict__ Vh, const ty
       for (int i = 0; i < n; ++i) x[i * n] = x[i * n] * nrm;
     }
   }
-  __syncwarp();
+  group_sync(L);
   // modified Gram-Schmidt inside clusters (eigenvalues closer than ortol), in eigenvalue order
   bool anyc = false;
   for (int j = 1; j < n; ++j) anyc |= (lam[j] - lam[j - 1] < ortol);
@@ -503,7 +774,7 @@ __global__ void eigh_vectors(const typename C2<TU>::t* __restrict__ Vh, const ty
           }
         }
       }
-      __syncwarp();
+      group_sync(L);
     }
   }
   // back-transform: u = H_0 H_1 ... H_{n-2} z  (precision TU), in chunks of CW columns (every
@@ -517,7 +788,7 @@ __global__ void eigh_vectors(const typename C2<TU>::t* __restrict__ Vh, const ty
 #pragma unroll
         for (int q = 0; q < kQ; ++q)
           if (lane + q * L < n) zr[q] = Zs[i * n + lane + q * L];
-        __syncwarp();
+        group_sync(L);
 #pragma unroll
         for (int q = 0; q < kQ; ++q)
           if (lane + q * L < n) {
@@ -525,7 +796,7 @@ __global__ void eigh_vectors(const typename C2<TU>::t* __restrict__ Vh, const ty
             z.x = to_tu<TU>(zr[q]);
             Us[i * n + lane + q * L] = z;
           }
-        __syncwarp();
+        group_sync(L);
       }
     } else {
       for (int jj = lane; jj < cw; jj += L)
@@ -540,7 +811,7 @@ __global__ void eigh_vectors(const typename C2<TU>::t* __restrict__ Vh, const ty
       const VU tau = tauIn[k * n + c];
       const bool act = cnonzero(tau);
       for (int i = c + 1 + lane; i < n; i += L) vsh[i] = Vh[(k * n + c) * n + i];
-      __syncwarp();
+      group_sync(L);
       if (act)
         for (int jj = lane; jj < cw; jj += L) {
           // v^H u as two lazy chains (even and odd rows): in double-float a chain step costs one
@@ -565,14 +836,14 @@ __global__ void eigh_vectors(const typename C2<TU>::t* __restrict__ Vh, const ty
             Us[i * CW + jj] = u;
           }
         }
-      __syncwarp();
+      group_sync(L);
     }
     if (valid)
       for (int idx = lane; idx < n * cw; idx += L) {
         const int i = idx / cw, jj = idx % cw;
         Uout[k * strideU + i * n + c0 + jj] = store_u<VO, VU>(Us[i * CW + jj]);
       }
-    __syncwarp();
+    group_sync(L);
   }
 }
 
@@ -1039,7 +1310,7 @@ int pick_group(size_t smem, int threads, int gmax) {
 // the built-in choices, and which other group sizes fit (the autotuner's candidates).
 template <typename R, typename TU>
 struct EighShape {
-  int L, LT, CW, gmaxT, gmaxV;
+  int L, LT, LV, CW, gmaxT, gmaxV;
   size_t smT, smQ1, smV;  // shared memory per matrix: tridiagonalisation, QL (d and e), vectors
   explicit EighShape(int n) {
     typedef typename C2<R>::t CR;
@@ -1061,15 +1332,23 @@ struct EighShape {
       if (!kUOverlaysZ<R, TU> && zbytes + ub(n) + vbytes > kMaxBlockSmem) CW = 32;
       smV = zbytes + ub(CW) + vbytes;
     }
-    gmaxV = 64 / L;
+    LV = n > 32 ? (n + 31) / 32 * 32 : L;  // n > 32: a block per matrix, a thread per column
+    gmaxV = n > 32 ? 1 : 64 / L;
   }
   int tridiag_default() const { return pick_group(smT, LT, gmaxT); }
-  int ql_default() const {
-    int BQ = 128;  // threads (matrices) per block
+  // Matrices (threads) per block of the QL sweep, a power of two up to 128: as few as spread the batch over
+  // the SMs (152) with `warps` warps each, since a warp takes as long as the longest and most divergent of
+  // its matrices.  An FP64 warp instruction takes the SM's FP64 pipe for 17 cycles whatever its active
+  // lanes, so 3 FP64 warps fill it; 4 warps hide the FP32 and double-float chains.
+  // 512 double-float matrices of 96 x 96: 6.7 ms (32 a warp) -> 4.7 ms (one a warp).
+  int ql_default(int nk) const {
+    const int warps = std::is_same<R, double>::value ? 3 : 4;
+    int BQ = 1;
+    while (BQ < 128 && (long long)BQ * 152 * warps < nk) BQ *= 2;
     while (BQ > 32 && (size_t)BQ * smQ1 > 64 * 1024) BQ /= 2;
     return BQ;
   }
-  int vectors_default() const { return pick_group(smV, L, gmaxV); }
+  int vectors_default() const { return pick_group(smV, LV, gmaxV); }
   // a group size fits: power of two up to gmax whose shared memory fits one block, and whole
   // warps unless it is the largest size that fits (the heuristic's choice when memory-bound)
   static bool group_fits(int g, size_t smem, int lanes, int gmax) {
@@ -1079,7 +1358,7 @@ struct EighShape {
   }
   bool fits(int param, int v) const {
     if (param == WBG_TUNE_EIGH_TRIDIAG_GROUP) return group_fits(v, smT, LT, gmaxT);
-    if (param == WBG_TUNE_EIGH_VECTORS_GROUP) return group_fits(v, smV, L, gmaxV);
+    if (param == WBG_TUNE_EIGH_VECTORS_GROUP) return group_fits(v, smV, LV, gmaxV);
     if (param == WBG_TUNE_EIGH_QL_BLOCK)
       return v >= 32 && v <= 256 && !(v & (v - 1)) && (size_t)v * smQ1 <= kMaxBlockSmem;
     return false;
@@ -1108,21 +1387,39 @@ int launch_eigh(const void* H, long long strideH, int n, int nk, void* E, void* 
   R* d = (R*)w; w += (size_t)nk * n * 8;
   R* e = (R*)w;
   const EighShape<R, TU> sh(n);
-  const int L = sh.L, LT = sh.LT;
+  const int LV = sh.LV, LT = sh.LT;
   if (stage != 2) {  // stage 1 (or both): the tridiagonalisation into the workspace
     const size_t smT = sh.smT;
+    if constexpr (!std::is_same<R, float>::value) {  // the FP32 solve serves n <= 32 only
+      if (n > 32) {
+        const size_t smW = smT + 4 * sizeof(CR);
+        cudaFuncSetAttribute(eigh_tridiag_wide<R, HIn, TU>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
+        const int thr = (4 * n + 31) / 32 * 32;
+        eigh_tridiag_wide<R, HIn, TU><<<nk, thr, smW, stream>>>((const HIn*)H, strideH, n, lowerIn, Vh, tau, d, e);
+      }
+    }
     const int G0 = sh.tridiag_default();
     if (G0 == 0) return WBG_ERR_SIZE;
     const int G = sh.choose(WBG_TUNE_EIGH_TRIDIAG_GROUP, variant, n, G0);
-    cudaFuncSetAttribute(eigh_tridiag<R, HIn, TU>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
-    eigh_tridiag<R, HIn, TU><<<(nk + G - 1) / G, G * LT, G * smT, stream>>>((const HIn*)H, strideH, n, nk, LT, G,
-                                                                             lowerIn, Vh, tau, d, e);
+    if (n <= 32) {
+      cudaFuncSetAttribute(eigh_tridiag<R, HIn, TU>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
+      eigh_tridiag<R, HIn, TU><<<(nk + G - 1) / G, G * LT, G * smT, stream>>>((const HIn*)H, strideH, n, nk, LT, G,
+                                                                               lowerIn, Vh, tau, d, e);
+    }
     if (stage == 1) return wbg_cuda_status(cudaGetLastError());
   }
-  const int BQ = sh.choose(WBG_TUNE_EIGH_QL_BLOCK, variant, n, sh.ql_default());
+  const int BQ = sh.choose(WBG_TUNE_EIGH_QL_BLOCK, variant, n, sh.ql_default(nk));
   const size_t smQ = (size_t)BQ * sh.smQ1;
-  cudaFuncSetAttribute(eigh_ql<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
-  eigh_ql<R><<<(nk + BQ - 1) / BQ, BQ, smQ, stream>>>(d, e, n, nk, (double*)E, errflag);
+  // up to four matrices an SM: a warp each (unless the tuner chose a block of matrices).  Not the FP32 solve,
+  // whose last bits depend on which products the compiler fuses in this very loop, and the refined
+  // eigenvectors on them (3e-8 of an AHC at num_wann 32).
+  if (!std::is_same<R, float>::value && wbg_tuned(WBG_TUNE_EIGH_QL_BLOCK, variant, n) == 0 && nk <= 4 * 152) {
+    eigh_ql_warp<R><<<(nk + QW_WARPS - 1) / QW_WARPS, 32 * QW_WARPS, QW_WARPS * sh.smQ1, stream>>>(d, e, n, nk,
+                                                                                                  (double*)E, errflag);
+  } else {
+    cudaFuncSetAttribute(eigh_ql<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
+    eigh_ql<R><<<(nk + BQ - 1) / BQ, BQ, smQ, stream>>>(d, e, n, nk, (double*)E, errflag);
+  }
   if (valuesOnly) return wbg_cuda_status(cudaGetLastError());
   const int CW = sh.CW;
   const size_t smV = sh.smV;
@@ -1130,7 +1427,7 @@ int launch_eigh(const void* H, long long strideH, int n, int nk, void* E, void* 
   if (GV0 == 0) return WBG_ERR_SIZE;
   const int GV = sh.choose(WBG_TUNE_EIGH_VECTORS_GROUP, variant, n, GV0);
   cudaFuncSetAttribute(eigh_vectors<R, TU, VO>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
-  eigh_vectors<R, TU, VO><<<(nk + GV - 1) / GV, GV * L, GV * smV, stream>>>(Vh, tau, d, e, (const double*)E, n, nk, L,
+  eigh_vectors<R, TU, VO><<<(nk + GV - 1) / GV, GV * LV, GV * smV, stream>>>(Vh, tau, d, e, (const double*)E, n, nk, LV,
                                                                             GV, CW, (VO*)U, strideU);
   return wbg_cuda_status(cudaGetLastError());
 }
