@@ -470,6 +470,8 @@ int wbg_scan_finalize(const void* hist, int nEF, int ncomp, double scale, double
  *   WBG_TUNE_EIGH_QL_BLOCK       matrices (threads) per block of the QL sweep   variant: eigh mode & 3
  *   WBG_TUNE_EIGH_VECTORS_GROUP  matrices per block of the inverse iteration and
  *                                back-transform                                variant: eigh mode & 3
+ *                                (above nw = 32 both groups are listed and kept for saved tables:
+ *                                those kernels take one matrix a block)
  *   WBG_TUNE_ROTATE_KPOINTS      k-points per block of the CUDA-core tiled U^dagger X U  variant: fp64
  *                                (FP64: listed and kept for saved tables; the tensor-core
  *                                rotation that serves FP64 does not read it)

@@ -1333,7 +1333,7 @@ struct EighShape {
       smV = zbytes + ub(CW) + vbytes;
     }
     LV = n > 32 ? (n + 31) / 32 * 32 : L;  // n > 32: a block per matrix, a thread per column
-    gmaxV = n > 32 ? 1 : 64 / L;
+    gmaxV = 64 / L;
   }
   int tridiag_default() const { return pick_group(smT, LT, gmaxT); }
   // Matrices (threads) per block of the QL sweep, a power of two up to 128: as few as spread the batch over
@@ -1348,7 +1348,7 @@ struct EighShape {
     while (BQ > 32 && (size_t)BQ * smQ1 > 64 * 1024) BQ /= 2;
     return BQ;
   }
-  int vectors_default() const { return pick_group(smV, LV, gmaxV); }
+  int vectors_default() const { return pick_group(smV, LV, LV > L ? 1 : gmaxV); }
   // a group size fits: power of two up to gmax whose shared memory fits one block, and whole
   // warps unless it is the largest size that fits (the heuristic's choice when memory-bound)
   static bool group_fits(int g, size_t smem, int lanes, int gmax) {
@@ -1358,12 +1358,13 @@ struct EighShape {
   }
   bool fits(int param, int v) const {
     if (param == WBG_TUNE_EIGH_TRIDIAG_GROUP) return group_fits(v, smT, LT, gmaxT);
-    if (param == WBG_TUNE_EIGH_VECTORS_GROUP) return group_fits(v, smV, LV, gmaxV);
+    if (param == WBG_TUNE_EIGH_VECTORS_GROUP) return group_fits(v, smV, L, gmaxV);
     if (param == WBG_TUNE_EIGH_QL_BLOCK)
       return v >= 32 && v <= 256 && !(v & (v - 1)) && (size_t)v * smQ1 <= kMaxBlockSmem;
     return false;
   }
-  // the tuned value of `param` when one is set and fits, else the built-in choice
+  // the tuned value of `param` when one is set and fits, else the built-in choice (n > 32: the
+  // reduction and the vectors take a matrix a block whatever group is set)
   int choose(int param, int variant, int n, int dflt) const {
     const int t = wbg_tuned(param, variant, n);
     return (t > 0 && fits(param, t)) ? t : dflt;
@@ -1390,6 +1391,8 @@ int launch_eigh(const void* H, long long strideH, int n, int nk, void* E, void* 
   const int LV = sh.LV, LT = sh.LT;
   if (stage != 2) {  // stage 1 (or both): the tridiagonalisation into the workspace
     const size_t smT = sh.smT;
+    const int G0 = sh.tridiag_default();
+    if (G0 == 0) return WBG_ERR_SIZE;
     if constexpr (!std::is_same<R, float>::value) {  // the FP32 solve serves n <= 32 only
       if (n > 32) {
         const size_t smW = smT + 4 * sizeof(CR);
@@ -1398,10 +1401,8 @@ int launch_eigh(const void* H, long long strideH, int n, int nk, void* E, void* 
         eigh_tridiag_wide<R, HIn, TU><<<nk, thr, smW, stream>>>((const HIn*)H, strideH, n, lowerIn, Vh, tau, d, e);
       }
     }
-    const int G0 = sh.tridiag_default();
-    if (G0 == 0) return WBG_ERR_SIZE;
-    const int G = sh.choose(WBG_TUNE_EIGH_TRIDIAG_GROUP, variant, n, G0);
     if (n <= 32) {
+      const int G = sh.choose(WBG_TUNE_EIGH_TRIDIAG_GROUP, variant, n, G0);
       cudaFuncSetAttribute(eigh_tridiag<R, HIn, TU>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
       eigh_tridiag<R, HIn, TU><<<(nk + G - 1) / G, G * LT, G * smT, stream>>>((const HIn*)H, strideH, n, nk, LT, G,
                                                                                lowerIn, Vh, tau, d, e);
@@ -1425,7 +1426,7 @@ int launch_eigh(const void* H, long long strideH, int n, int nk, void* E, void* 
   const size_t smV = sh.smV;
   const int GV0 = sh.vectors_default();
   if (GV0 == 0) return WBG_ERR_SIZE;
-  const int GV = sh.choose(WBG_TUNE_EIGH_VECTORS_GROUP, variant, n, GV0);
+  const int GV = n > 32 ? 1 : sh.choose(WBG_TUNE_EIGH_VECTORS_GROUP, variant, n, GV0);
   cudaFuncSetAttribute(eigh_vectors<R, TU, VO>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBlockSmem);
   eigh_vectors<R, TU, VO><<<(nk + GV - 1) / GV, GV * LV, GV * smV, stream>>>(Vh, tau, d, e, (const double*)E, n, nk, LV,
                                                                             GV, CW, (VO*)U, strideU);
