@@ -107,3 +107,32 @@ def test_many_fields_and_strided_u():
     assert st == 0
     Y = _exact(np.ascontiguousarray(Up[:, :nw]), X)
     assert float(np.abs(out.cpu().numpy() - Y).max() / np.abs(Y).max()) < 2.0 ** -53 * (1 + 2 * np.sqrt(2 * nw))
+
+
+@pytest.mark.parametrize("nw,fp", [(32, 1), (48, 1), (82, 2)])
+def test_waits_that_run_out(nw, fp):
+    """With a 0 ns bound on every wait the blocks that find a barrier incomplete give up together, drain their
+    products and return; with the normal bound the same call then gives the same bits as before."""
+    import ctypes
+    lib, nk = engine._lib.load(), 400
+    U, X = _case(nw, 4, 5, nw)
+    X[:, 1:3] = X[:, 3:5]  # double-float holds the range of floats
+    conv = lambda a: torch.from_numpy(a if fp == 1 else engine._df64_pairs(a)).contiguous().view(torch.complex128)
+    Ut = conv(U).reshape(U.shape).repeat(nk // 4, 1, 1).cuda()
+    Xt = conv(X).reshape(X.shape).repeat(nk // 4, 1, 1, 1).cuda()
+    run = lambda: engine.rotate(Ut, Xt, 5, [0, 1, 2, 3, 4], MODES, nw, nk, fp)[0].clone()
+    diag = lambda a: torch.view_as_real(a.diagonal(dim1=-2, dim2=-1).contiguous())
+    before = run()
+    engine.device_flags()
+    try:
+        assert lib.wbg_tc_wait_limit(ctypes.c_ulonglong(0)) == 0
+        run()
+        torch.cuda.synchronize()
+        engine.device_flags()  # whether a block gave up depends on timing
+    finally:
+        assert lib.wbg_tc_wait_limit(ctypes.c_ulonglong(1_000_000_000)) == 0
+    after = run()
+    torch.cuda.synchronize()
+    assert engine.device_flags() == 0
+    assert torch.equal(torch.view_as_real(before[:, [0, 1, 3]]), torch.view_as_real(after[:, [0, 1, 3]]))
+    assert torch.equal(diag(before), diag(after))

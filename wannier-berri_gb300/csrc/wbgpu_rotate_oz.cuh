@@ -21,7 +21,7 @@
 // is what this avoids.  nw = 32, 9 fields, 13 824 k-points: 44.8 ms (CUDA-core FP64, 97% of the pipe)
 // -> 5.7 ms; of the 44 k cycles of a 96-row tile 13 k wait for the products (36 pairs x 4 K steps of
 // M = 128, N = 64: 4.6 k at full rate per GEMM).  nw = 96, 9 fields, 512 k-points: 27.7 ms
-// (double-float) -> 5.1 ms, 53.4 ms (FP64) -> 4.9 ms.
+// (double-float) -> 4.5 ms, 53.4 ms (FP64) -> 4.6 ms.
 //
 // Complex products are embedded in real ones as in the TF32 kernel above; operand rows are 128-byte
 // (64-byte) swizzled K-major rows of 64 (32) fp16.  Consecutive B slices are consecutive rows of
@@ -34,11 +34,13 @@ template <int DF> struct OzCfg;  // 0: complex128 in and out; 1: double-float co
 template <> struct OzCfg<0> {
   typedef double2 VI;
   typedef double2 VO;
+  typedef double PI;  // one part (re or im) of VI
   static constexpr int NG = 8, BIAS = 1084, EMAX = 0x7ff;
 };
 template <> struct OzCfg<1> {
   typedef float4 VI;  // re.hi, re.lo, im.hi, im.lo
   typedef float2 VO;
+  typedef float2 PI;
   static constexpr int NG = 7, BIAS = 188, EMAX = 0xff;
 };
 
@@ -61,14 +63,22 @@ WBG_D long long oz_fix(float x, int emax) {
   const long long v = (long long)(((unsigned long long)((u & 0x7fffffu) | 0x800000u) << 38) >> s);
   return (int)u < 0 ? -v : v;
 }
+// the same of the low half of a double-float: the multiplication by 2^(BIAS - emax), exact in two steps, and a
+// truncating conversion.  It runs on the FP64 pipe, which is idle here: nw = 82 as below takes 15.2 ms with both
+// halves on the integer pipe, 15.9 ms with both here, 14.7 ms with one on each.
+WBG_D long long oz_fix_lo(float x, int emax) {
+  const int t = 188 - emax, ta = t / 2;
+  return __float2ll_rz(x * __int_as_float((ta + 127) << 23) * __int_as_float((t - ta + 127) << 23));
+}
 WBG_D int oz_cexp(double2 a) { return max(oz_exp(a.x), oz_exp(a.y)); }
 WBG_D int oz_cexp(float4 a) { return max(oz_exp(a.x), oz_exp(a.z)); }
 WBG_D long long oz_re(double2 a, int emax) { return oz_fix(a.x, emax); }
 WBG_D long long oz_im(double2 a, int emax) { return oz_fix(a.y, emax); }
-WBG_D long long oz_re(float4 a, int emax) { return oz_fix(a.x, emax) + oz_fix(a.y, emax); }
-WBG_D long long oz_im(float4 a, int emax) { return oz_fix(a.z, emax) + oz_fix(a.w, emax); }
+WBG_D long long oz_part(double a, int emax) { return oz_fix(a, emax); }
+WBG_D long long oz_part(float2 a, int emax) { return oz_fix(a.x, emax) + oz_fix_lo(a.y, emax); }
+WBG_D double oz_zero(double) { return 0.0; }
+WBG_D float2 oz_zero(float2) { return make_float2(0.f, 0.f); }
 WBG_D double2 oz_zero(double2) { return make_double2(0.0, 0.0); }
-WBG_D float4 oz_zero(float4) { return make_float4(0.f, 0.f, 0.f, 0.f); }
 WBG_D double2 oz_real(double2 a) { return make_double2(a.x, 0.0); }
 WBG_D float4 oz_real(float4 a) { return make_float4(a.x, a.y, 0.f, 0.f); }
 
@@ -147,6 +157,25 @@ WBG_D void oz_issue(uint32_t d, uint32_t a, uint32_t b, int ncol, int ksteps, ui
       }
     }
   }
+}
+
+// The same with the loops unrolled (NCOL columns a slice, all K steps): a few instructions a product
+template <int KP, int NG, int NCOL>
+WBG_D void oz_issue_all(uint32_t d, uint32_t a, uint32_t b, uint32_t accumulate) {
+  constexpr uint32_t astride = 128 * KP * 2, bstride = NCOL * KP * 2;
+  constexpr int per = 256 / NCOL;
+  const uint64_t ad = oz_desc<KP>(a), bd = oz_desc<KP>(b);
+#pragma unroll
+  for (int ks = 0; ks < KP / 16; ++ks)
+#pragma unroll
+    for (int i = 0; i < NG; ++i)
+#pragma unroll
+      for (int j = 0; j < NG - i; j += per) {
+        const int n = (per < NG - i - j ? per : NG - i - j) * NCOL;
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
+        mma_f16(d + (uint32_t)((i + j) * NCOL), ad + ((i * astride + ks * 32) >> 4), bd + ((j * bstride + ks * 32) >> 4),
+                idesc, ks > 0 || i > 0 ? 1u : accumulate);
+      }
 }
 
 // 8 fixed-point values along K as one 16-byte chunk of each of NS slices
@@ -518,14 +547,19 @@ __global__ void __launch_bounds__(8 * KP, 64 / KP)
 // 32 < nw <= 128: one field and one panel of PN = 32 columns at a time.
 //   GEMM1  T = X U_P        A = [Re X | Im X] rows m       B = embedded U[:, P]
 //   GEMM2  Y = U^dagger T   A = [Re U^T | Im U^T] rows m'  B = [[Re T, Im T], [Im T, -Re T]]
-// K runs in chunks of 32 complex rows; T stays in registers (fixed point) between the GEMMs, and
-// the warps of TMEM lane quarter c write chunk c of it as operand.  Rows >= nw of A are left as they
+// K runs in stages of 16 complex rows ([16 Re | 16 Im]) through two operand buffers: while the tensor cores
+// multiply one, all threads cut the next.  T stays in registers (fixed point) between the GEMMs, and the
+// warps of TMEM lane quarter c write stages 2c and 2c + 1 of it as operand.  Rows >= nw of A are left as they
 // are: they reach only accumulator rows that nothing reads.  Hermitian-part fields take the
 // Hermitian part on input and write the lower triangle with its mirror, as rotate_panel does, so
 // that the stored matrix is Hermitian bit for bit.
 // ---------------------------------------------------------------------------------------
-constexpr int OZ_PN = 32, OZ_THR = 512;
-template <int DF> constexpr int oz_large_smem() { return OzCfg<DF>::NG * (128 + 64) * 128 + 1024; }
+// Bound by the cutting: issue slots 46% active, the tensor pipe 27%.  One buffer of 32 rows, every product waited
+// for: 17.3 ms at nw = 82 (double-float, 36 fields, 512 k-points) and 8.1 ms at nw = 48 (9 fields, 2 048);
+// two buffers with all threads meeting at each stage: 17.7 and 7.0 ms; this, with a warp for the products and
+// full / done barriers a stage, so that no cutting warp waits for another one: 14.7 and 6.2 ms.
+constexpr int OZ_PN = 32, OZ_WK = 512, OZ_THR = OZ_WK + 32;  // 16 warps at the operands, one for the products
+template <int DF> constexpr int oz_large_smem() { return 2 * OzCfg<DF>::NG * (128 + 64) * 64 + 1024; }
 
 template <int DF>
 __global__ void __launch_bounds__(OZ_THR, 1)
@@ -536,23 +570,27 @@ __global__ void __launch_bounds__(OZ_THR, 1)
   typedef OzCfg<DF> Cfg;
   typedef typename Cfg::VI VI;
   typedef typename Cfg::VO VO;
-  constexpr int NG = Cfg::NG, KP = 64;
+  typedef typename Cfg::PI PI;
+  constexpr int NG = Cfg::NG, KP = 32;
   constexpr int SH = DF ? 6 : 14;  // K <= 256: |sum| <= 2^76 (FP64), 2^68 (double-float)
   constexpr int EP = SH + 112 - 8 * (NG - 1);
-  constexpr uint32_t ASTR = 128 * 128, BSTR = 64 * 128;
+  constexpr uint32_t ASTR = 128 * 64, BSTR = 64 * 64, STAGE = NG * (ASTR + BSTR);  // A slices, then B slices
   constexpr int LDS = OZ_PN + 1;
+  static_assert(2 * STAGE >= 2 * 128 * LDS * 8, "the staging overlays the operand buffers");
   extern __shared__ __align__(1024) unsigned char smo[];
   unsigned char* As = smo + ((1024u - (smem_u32(smo) & 1023u)) & 1023u);
-  unsigned char* Bs = As + NG * ASTR;
   long long* stre = reinterpret_cast<long long*>(As);  // staging: [m'][n] re plane, then im plane
   long long* stim = stre + 128 * LDS;
-  __shared__ __align__(8) uint64_t mbar;
+  __shared__ __align__(8) uint64_t mbar[4];  // full[2]: an arrival a warp; done[2]: the products' commit
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s, ue_s, fe_s, qm_s;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t mb = smem_u32(&mbar);
+  const uint32_t full = smem_u32(mbar), done = full + 16;
   if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mb) : "memory");
+    for (int i = 0; i < 2; ++i) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(full + 8 * i), "r"(OZ_WK / 32) : "memory");
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(done + 8 * i) : "memory");
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     abort_s = 0;
   }
@@ -566,19 +604,54 @@ __global__ void __launch_bounds__(OZ_THR, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tbase = tmem_base_s;
-  const int nw2 = nw * nw, np = (nw + OZ_PN - 1) / OZ_PN, nch = (nw + 31) / 32;
+  const int nw2 = nw * nw, np = (nw + OZ_PN - 1) / OZ_PN, nst = (nw + 15) / 16;
   const int quarter = warp & 3, half = warp >> 3, sub = (warp >> 2) & 1;  // columns 32 half + 16 sub ..
   const uint32_t lane_base = ((uint32_t)(32 * quarter) << 16) + 32 * half + 16 * sub;
   const int row = 32 * quarter + lane;
   const unsigned long long wait_ns = g_tc_wait_ns;
-  uint32_t phase = 0;
+  volatile int* ab = &abort_s;
+  uint32_t g = 0;  // stages so far: stage g in buffer g & 1, phase g >> 1 of its barriers
   long long kprev = -1, fprev = -1;
   const long long total = (long long)nk * nFrot * np;
   const long long u1 = min(total, (blockIdx.x + 1) * per);
-  // task of the A loads: 8 columns of one row; 8 lanes take 8 rows
-  const int am = (tid >> 5) * 8 + (tid & 7), ac8 = (tid >> 3) & 3;
-  VI xr[8];
-  for (long long u = blockIdx.x * per; u < u1 && !abort_s; ++u) {
+  // task of the A operand: 8 columns of one part (0 re, 1 im) of one row (8 lanes take 8 rows); of the embedded
+  // U panel: rows bj, bj + 1 of one part of column n0 + lane
+  const int am = (tid >> 5) * 8 + (tid & 7), akc = (tid >> 3) & 3, apart = akc >> 1, aj = 8 * (akc & 1);
+  const int bj = 2 * (warp & 7), bpart = warp >> 3;
+  PI xr[8], br[2];
+  // A wait that runs out sets abort_s: the warps then skip operands and accumulators, but meet at every barrier
+  // until the next unit, where all leave together.
+  bool ok = true;
+  auto wait_stage = [&](uint32_t x) {  // all products of stage x are done (x < g)
+    if (lane == 0) ok = ok && kt_wait(done + 8 * (x & 1), (x >> 1) & 1u, ab, wait_ns);
+    ok = __shfl_sync(0xffffffffu, ok, 0);
+  };
+  auto stage_full = [&]() {  // this warp's part of the stage is written
+    fence_async_smem();
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0 && ok) mbar_arrive(full + 8 * (g & 1));
+    ++g;
+  };
+  auto wsync = [&]() { named_sync(1, OZ_WK); };
+  if (warp == OZ_WK / 32) {
+    // ---- products: two GEMMs of nst stages a unit
+    if (lane == 0) {
+      const long long nu = u1 - blockIdx.x * per;
+      for (long long u = 0; u < 2 * nu && ok; ++u)
+        for (int i = 0; i < nst; ++i, ++g) {
+          ok = kt_wait(full + 8 * (g & 1), (g >> 1) & 1u, ab, wait_ns);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t st = smem_u32(As + (g & 1) * STAGE);
+          oz_issue_all<KP, NG, 64>(tbase, st, st + NG * ASTR, (uint32_t)(i > 0));
+          mma_commit(done + 8 * (g & 1));
+        }
+      if (g > 0) mbar_wait(done + 8 * ((g - 1) & 1), ((g - 1) >> 1) & 1u, DRAIN_NS);  // no product in flight at exit
+    }
+    __syncwarp();
+  } else {
+  for (long long u = blockIdx.x * per; u < u1; ++u) {
     const int P = (int)(u % np), f = (int)((u / np) % nFrot);
     const long long k = u / ((long long)np * nFrot);
     const int fs = fsel[f], hm = herm[f];
@@ -589,111 +662,120 @@ __global__ void __launch_bounds__(OZ_THR, 1)
     const int n0 = P * OZ_PN;
     // ---- largest exponents of U_k and of the field (kept while the CTA stays on them)
     const bool newk = k != kprev, newf = newk || f != fprev;
-    __syncthreads();
+    if (named_any(1, OZ_WK, !ok || *ab)) break;
     if (tid == 0) {
       if (newk) ue_s = 1;
       if (newf) fe_s = 1;
       qm_s = 0;
     }
-    __syncthreads();
+    wsync();
     if (newk) {
       int e = 1;
 #pragma unroll 4
-      for (int i = tid; i < nw2; i += OZ_THR) e = max(e, oz_cexp(Uk[i]));
+      for (int i = tid; i < nw2; i += OZ_WK) e = max(e, oz_cexp(Uk[i]));
       e = warp_max(e);
       if (lane == 0) atomicMax(&ue_s, e);
     }
     if (newf) {
       int e = 1;
-#pragma unroll 4
-      for (int i = tid; i < nw2; i += OZ_THR) {
-        const VI v = Xf[i];  // of a lower-triangle field only m >= n counts, of its diagonal the real part
-        const int m = i / nw, n = i - m * nw;
-        if (inmode != 2 || m >= n) e = max(e, oz_cexp(inmode == 2 && m == n ? oz_real(v) : v));
-      }
+#pragma unroll 2
+      for (int m = warp; m < nw; m += OZ_WK / 32)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {  // of a lower-triangle field only m >= n counts, of its diagonal the real part
+          const int n = 32 * c + lane;
+          if (n < nw && (inmode != 2 || m >= n)) {
+            const VI v = Xf[m * nw + n];
+            e = max(e, oz_cexp(inmode == 2 && m == n ? oz_real(v) : v));
+          }
+        }
       e = warp_max(e);
       if (lane == 0) atomicMax(&fe_s, e);
     }
     kprev = k;
     fprev = f;
-    auto load_x = [&](int c) {
+    const PI* Xp = reinterpret_cast<const PI*>(Xf) + apart;
+    const PI* Up = reinterpret_cast<const PI*>(Uk);
+    const PI* Xa = Xp + 2 * (am * nw + aj);
+    auto load_x = [&](int i) {  // stage i of GEMM1: X and the rows of U[:, P]
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
-        const int j = 32 * c + 8 * ac8 + q;
-        xr[q] = oz_zero(VI());
-        if (am < nw && j < nw) {
-          xr[q] = Xf[inmode == 2 && j > am ? j * nw + am : am * nw + j];
-        }
+        const int j = 16 * i + aj + q;
+        xr[q] = oz_zero(PI());
+        if (am < nw && j < nw) xr[q] = inmode == 2 && j > am ? Xp[2 * (j * nw + am)] : Xa[2 * (16 * i + q)];
+      }
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int j = 16 * i + bj + q;
+        br[q] = n0 + lane < nw && j < nw ? Up[2 * (j * nw + n0 + lane) + bpart] : oz_zero(PI());
       }
     };
-    auto load_uh = [&](int c) {  // row m' of U^H: U[j][m']
+    auto load_uh = [&](int i) {  // stage i of GEMM2: row m' of U^H: U[j][m']
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
-        const int j = 32 * c + 8 * ac8 + q;
-        xr[q] = am < nw && j < nw ? Uk[j * nw + am] : oz_zero(VI());
+        const int j = 16 * i + aj + q;
+        xr[q] = am < nw && j < nw ? Up[2 * (j * nw + am) + apart] : oz_zero(PI());
+      }
+    };
+    auto put_uh = [&](int eu) {
+      if (am < nw && ok) {
+        long long v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = oz_part(xr[q], eu);
+        oz_put8<NG>(As + (g & 1) * STAGE, ASTR, oz_off<KP>(am, akc), v);
       }
     };
     load_x(0);
-    __syncthreads();
+    wsync();
     const int eu = ue_s, ex = fe_s;
     // ---- GEMM1
-    for (int c = 0; c < nch; ++c) {
-      if (am < nw) {
+    for (int i = 0; i < nst; ++i) {
+      if (i >= 2) wait_stage(g - 2);  // (the previous unit's stages are done)
+      unsigned char* A = As + (g & 1) * STAGE;
+      unsigned char* B = A + NG * ASTR;
+      if (am < nw && ok) {
         long long v[8];
 #pragma unroll
-        for (int p = 0; p < 2; ++p) {  // re, im
+        for (int q = 0; q < 8; ++q) v[q] = oz_part(xr[q], ex);
+        if (inmode == 2 && apart) {  // the mirror's conjugate, the real diagonal
 #pragma unroll
-          for (int q = 0; q < 8; ++q) v[q] = p ? oz_im(xr[q], ex) : oz_re(xr[q], ex);
-          if (inmode == 2 && p) {  // the mirror's conjugate, the real diagonal
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-              const int j = 32 * c + 8 * ac8 + q;
-              v[q] = j > am ? -v[q] : j == am ? 0 : v[q];
-            }
+          for (int q = 0; q < 8; ++q) {
+            const int j = 16 * i + aj + q;
+            v[q] = j > am ? -v[q] : j == am ? 0 : v[q];
           }
-          if (inmode == 1) {  // Hermitian part of the input
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-              const int j = 32 * c + 8 * ac8 + q;
-              if (j < nw) {
-                const VI b = Xf[j * nw + am];
-                v[q] = (p ? v[q] - oz_im(b, ex) : v[q] + oz_re(b, ex)) >> 1;
-              }
-            }
-          }
-          oz_put8<NG>(As, ASTR, oz_off<KP>(am, 4 * p + ac8), v);
         }
+        if (inmode == 1) {  // Hermitian part of the input
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const int j = 16 * i + aj + q;
+            if (j < nw) {
+              const long long o = oz_part(Xp[2 * (j * nw + am)], ex);
+              v[q] = (apart ? v[q] - o : v[q] + o) >> 1;
+            }
+          }
+        }
+        oz_put8<NG>(A, ASTR, oz_off<KP>(am, akc), v);
       }
-      {  // embedded U[:, P]: 2 rows j of one column
-        const int jl = warp * 2, j = 32 * c + jl;
-        const bool nok = n0 + lane < nw;
-        const VI a = nok && j < nw ? Uk[j * nw + n0 + lane] : oz_zero(VI());
-        const VI b = nok && j + 1 < nw ? Uk[(j + 1) * nw + n0 + lane] : oz_zero(VI());
-        const int cr = jl >> 3;
-        const uint32_t h = (jl & 7) * 2;
-        oz_put2x2<NG>(Bs, BSTR, oz_off<KP>(lane, cr) + h, oz_off<KP>(32 + lane, 4 + cr) + h, 0u, oz_re(a, eu),
-                      oz_re(b, eu));
-        oz_put2x2<NG>(Bs, BSTR, oz_off<KP>(32 + lane, cr) + h, oz_off<KP>(lane, 4 + cr) + h, 0x80008000u,
-                      oz_im(a, eu), oz_im(b, eu));
+      if (ok) {  // embedded U[:, P]: Re at (n, re K) and (32 + n, im K), Im at (32 + n, re K) and, negated, at (n, im K)
+        const int rc = bj >> 3;
+        const uint32_t h = (bj & 7) * 2;
+        oz_put2x2<NG>(B, BSTR, oz_off<KP>(bpart ? 32 + lane : lane, rc) + h,
+                      oz_off<KP>(bpart ? lane : 32 + lane, 2 + rc) + h, bpart ? 0x80008000u : 0u, oz_part(br[0], eu),
+                      oz_part(br[1], eu));
       }
-      fence_async_smem();
-      __syncthreads();
-      if (tid == 0) {
-        tc_fence_after();
-        oz_issue<KP, NG>(tbase, smem_u32(As), smem_u32(Bs), 64, 4, (uint32_t)(c > 0));
-        mma_commit(mb);
-      }
-      if (c + 1 < nch) load_x(c + 1);
+      stage_full();
+      if (i + 1 < nst) load_x(i + 1);
       else load_uh(0);
-      if (!wait_all(mb, phase, &abort_s, wait_ns)) break;
-      phase ^= 1;
-      tc_fence_after();
     }
-    if (abort_s) break;
+    // the first stage of U^H while the last products run
+    wait_stage(g - 2);
+    put_uh(eu);
+    load_uh(1);
+    wait_stage(g - 1);
+    tc_fence_after();
     // ---- T: thread (row j) holds 16 columns n of Re (half 0) or Im (half 1) T[j][n0 + 16 sub ..]
     long long q[16];
     const bool live = 32 * quarter < nw;
-    if (live) {
+    if (live && ok) {
       int hmx = 0;
 #pragma unroll
       for (int c = 0; c < 16; c += 4) {
@@ -707,34 +789,39 @@ __global__ void __launch_bounds__(OZ_THR, 1)
       hmx = warp_max(hmx);
       if (lane == 0) atomicMax(&qm_s, hmx);
     }
-    tc_fence_before();
-    __syncthreads();
+    wsync();
     const int nsh = oz_norm(qm_s);
+    // lanes l and l + 16 exchange half of their columns, so that the 16 rows of a stage lie on all lanes: lane l
+    // then holds columns 16 sub + 8 (l >> 4) .. + 7 of rows l & 15 (q[0 .. 7]) and 16 + (l & 15) (q[8 .. 15])
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const long long o = __shfl_xor_sync(0xffffffffu, lane < 16 ? q[8 + i] : q[i], 16);
+      if (lane < 16) q[8 + i] = o;
+      else q[i] = o;
+    }
     // ---- GEMM2
-    for (int c = 0; c < nch; ++c) {
-      if (am < nw) {
-        long long v[8];
-#pragma unroll
-        for (int s = 0; s < 8; ++s) v[s] = oz_re(xr[s], eu);
-        oz_put8<NG>(As, ASTR, oz_off<KP>(am, ac8), v);
-#pragma unroll
-        for (int s = 0; s < 8; ++s) v[s] = oz_im(xr[s], eu);
-        oz_put8<NG>(As, ASTR, oz_off<KP>(am, 4 + ac8), v);
+    const int jl = lane & 15;
+    const int ka = half * 16 + jl, kb = (1 - half) * 16 + jl;  // K of the n and of the 32 + n rows
+    const uint32_t flip = half ? 0u : 0x80008000u;             // -Re T at (32 + n, im K)
+    const bool odd = lane & 1;  // even lanes write column n of rows j, j + 1, odd lanes column n + 1 of j - 1, j
+    for (int i = 0; i < nst; ++i) {
+      if (i > 0) {
+        if (i >= 2) wait_stage(g - 2);
+        put_uh(eu);
+        if (i + 1 < nst) load_uh(i + 1);
       }
-      if (quarter == c) {  // this quarter's rows j are the chunk's
-        const int k0 = half * 32 + lane, k1 = (1 - half) * 32 + lane;  // K of the n and of the 32 + n rows
-        const uint32_t flip = half ? 0u : 0x80008000u;                 // -Re T at (32 + n, K = 32 + j)
-        const bool odd = lane & 1;  // even lanes write column n of rows j, j + 1, odd lanes column n + 1 of j - 1, j
-        unsigned char* b0 = Bs + (k0 & 6) * 2;
-        unsigned char* b1 = Bs + (k1 & 6) * 2;
+      if (quarter == i >> 1 && ok) {  // this quarter's rows j
+        unsigned char* B = As + (g & 1) * STAGE + NG * ASTR;
+        unsigned char* b0 = B + (ka & 6) * 2;
+        unsigned char* b1 = B + (kb & 6) * 2;
 #pragma unroll
-        for (int i = 0; i < 16; i += 2) {
-          const long long a = q[i] << nsh, b = q[i + 1] << nsh;
+        for (int c = 0; c < 8; c += 2) {
+          const long long a = (i & 1 ? q[8 + c] : q[c]) << nsh, b = (i & 1 ? q[9 + c] : q[c + 1]) << nsh;
           const long long o = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
           const unsigned long long wa = oz_bias(odd ? o : a), wb = oz_bias(odd ? b : o);
-          const int n = 16 * sub + i + odd;
-          unsigned char* p0 = b0 + oz_off<KP>(n, k0 >> 3);
-          unsigned char* p1 = b1 + oz_off<KP>(32 + n, k1 >> 3);
+          const int n = 16 * sub + 8 * (lane >> 4) + c + odd;
+          unsigned char* p0 = b0 + oz_off<KP>(n, ka >> 3);
+          unsigned char* p1 = b1 + oz_off<KP>(32 + n, kb >> 3);
 #pragma unroll
           for (int s = 0; s < NG; ++s) {
             const uint32_t d = oz_dig2(oz_word(wa, s), oz_word(wb, s), 3 - (s & 3));
@@ -743,21 +830,13 @@ __global__ void __launch_bounds__(OZ_THR, 1)
           }
         }
       }
-      fence_async_smem();
-      __syncthreads();
-      if (tid == 0) {
-        tc_fence_after();
-        oz_issue<KP, NG>(tbase, smem_u32(As), smem_u32(Bs), 64, 4, (uint32_t)(c > 0));
-        mma_commit(mb);
-      }
-      if (c + 1 < nch) load_uh(c + 1);
-      if (!wait_all(mb, phase, &abort_s, wait_ns)) break;
-      phase ^= 1;
-      tc_fence_after();
+      stage_full();
     }
-    if (abort_s) break;
+    wait_stage(g - 2);
+    wait_stage(g - 1);
+    tc_fence_after();
     // ---- Y: thread (row m') holds 16 columns of Re or Im of Y[m'][n0 ..]; staged, then written by rows
-    if (live) {
+    if (live && ok) {
 #pragma unroll
       for (int c = 0; c < 16; c += 4) {
         long long s[4];
@@ -768,27 +847,25 @@ __global__ void __launch_bounds__(OZ_THR, 1)
       }
     }
     tc_fence_before();
-    __syncthreads();
+    wsync();
     const bool bad = !fok || ex >= Cfg::EMAX || eu >= Cfg::EMAX;
     const int E = 2 * EP - nsh + ex + 2 * eu - 3 * Cfg::BIAS;
     VO* dst = Xbar + (k * nFrot + f) * (long long)nw2;
     const int mode = hm & 3, n = n0 + lane;
-    for (int m = warp; m < nw; m += OZ_THR / 32) {
+    for (int m = warp; m < nw && ok; m += OZ_WK / 32) {
       if (n >= nw || (mode != 0 && n > m) || (mode == 2 && n != m)) continue;
       VO y = oz_pack(VO(), stre[m * LDS + lane], stim[m * LDS + lane], E);
       if (mode != 0 && m == n) y.y = 0;
       dst[m * nw + n] = bad ? oz_nan(y) : y;
     }
-    if (mode == 1) {  // the mirror: row n of the panel, columns m > n
-      for (int nl = warp; nl < OZ_PN && n0 + nl < nw; nl += OZ_THR / 32)
+    if (mode == 1 && ok) {  // the mirror: row n of the panel, columns m > n
+      for (int nl = warp; nl < OZ_PN && n0 + nl < nw; nl += OZ_WK / 32)
         for (int m = n0 + nl + 1 + lane; m < nw; m += 32) {
           const VO y = oz_pack(VO(), stre[m * LDS + nl], -stim[m * LDS + nl], E);
           dst[(n0 + nl) * nw + m] = bad ? oz_nan(y) : y;
         }
     }
   }
-  if (abort_s) {
-    if (tid == 0) mbar_wait(mb, phase, DRAIN_NS);
   }
   tc_fence_before();
   __syncthreads();
