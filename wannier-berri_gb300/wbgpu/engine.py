@@ -9,6 +9,7 @@ without the library every entry point raises.
 """
 import copy
 import ctypes
+import math
 import warnings
 
 import numpy as np
@@ -96,7 +97,7 @@ def _ptr(t):
 
 
 def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return ctypes.c_void_p(torch.cuda.current_stream(torch.cuda.current_device()).cuda_stream)  # (an index: a third of the time)
 
 
 class RGeometry:
@@ -167,7 +168,7 @@ class Workspace:
 
     def buffer(self, name, shape, dtype):
         """Buffer `name` viewed as dtype[shape], grown when too small (old contents dropped)."""
-        nbytes = int(np.prod(shape)) * torch.empty((), dtype=dtype).element_size()
+        nbytes = math.prod(shape) * dtype.itemsize
         buf = self._bufs.get(name)
         if buf is None or buf.numel() < nbytes:
             self._bufs.pop(name, None)
@@ -287,11 +288,26 @@ class DeviceSystem:
         return self._cache[ck]
 
     def geom_tensors(self):
+        """Device tables of the R-vector structure (int32) and the Wannier centers 'wcc' (float64), uploaded
+        in one copy that has completed on return (every stream may read them); a table starts on a multiple
+        of 256 bytes."""
         if 'geom' not in self._cache:
             g = self.geom
-            mk = lambda a: torch.from_numpy(np.ascontiguousarray(a, dtype=np.int32)).to(self.device)
-            self._cache['geom'] = dict(pair_start=mk(g.pair_start), r2=mk(g.r2), slice_start=mk(g.slice_start),
-                                       pair_r1=mk(g.pair_r1), slice_r0=mk(g.slice_r0), iR=mk(g.R))
+            parts = {k: np.ascontiguousarray(a, dtype=np.int32) for k, a in
+                     (('pair_start', g.pair_start), ('r2', g.r2), ('slice_start', g.slice_start),
+                      ('pair_r1', g.pair_r1), ('slice_r0', g.slice_r0), ('iR', g.R))}
+            parts['wcc'] = np.ascontiguousarray(self.wcc, dtype=np.float64)
+            offs, n = [], 0
+            for a in parts.values():
+                offs.append(n)
+                n += (a.nbytes + 255) // 256 * 256
+            host = np.zeros(n, dtype=np.uint8)
+            for a, o in zip(parts.values(), offs):
+                host[o:o + a.nbytes] = a.reshape(-1).view(np.uint8)
+            flat = torch.from_numpy(host).to(self.device)
+            self._cache['geom'] = {
+                k: flat[o:o + a.nbytes].view(torch.float64 if k == 'wcc' else torch.int32).view(a.shape)
+                for (k, a), o in zip(parts.items(), offs)}
         return self._cache['geom']
 
     def buffer(self, name, shape, dtype):
@@ -328,7 +344,7 @@ class DeviceSystem:
             self._cache[key + ('staging',)] = host  # page-locked source of the in-flight copy
         return self._cache[key]
 
-    def _upload_phases(self, tables, prec):
+    def _upload_phases(self, tables, prec, pin=False):
         parts = []
         for p in tables:
             if prec == PREC_DF64:
@@ -339,8 +355,8 @@ class DeviceSystem:
         # table starts on a multiple of its element size
         words = [a.reshape(-1).view(np.float64 if a.dtype == np.complex128 else np.float32) for a in parts]
         host = torch.from_numpy(np.concatenate(words))
-        if torch.cuda.is_available() and host.numel() * host.element_size() > (4 << 20):
-            host = host.pin_memory()  # large tables: asynchronous copy from page-locked memory
+        if pin or (torch.cuda.is_available() and host.numel() * host.element_size() > (4 << 20)):
+            host = host.pin_memory()  # large tables, tables of one call: asynchronous copy from page-locked memory
         dev_flat = host.to(self.device, non_blocking=host.is_pinned())
         tabs, off = [], 0
         for a, w in zip(parts, words):
@@ -350,13 +366,6 @@ class DeviceSystem:
                 t = torch.view_as_complex(t.view(-1, 2))
             tabs.append(t.view(a.shape))
         return tabs, host
-
-    def wcc_tensor(self, fp64):
-        k = ('wcc', fp64)
-        if k not in self._cache:
-            self._cache[k] = torch.tensor(self.wcc, dtype=torch.float64 if fp64 else torch.float32,
-                                          device=self.device).contiguous()
-        return self._cache[k]
 
 
 def field_plan(quantities, with_H, extra_keys):
@@ -512,7 +521,7 @@ def r2k_geometry(dev, NKFFT):
     g = dev.geom
     nw = dev.nw
     return _lib.R2KGeom(nR=len(g.R), nw=nw, nw2=nw * nw, nBase=0, nP=g.nP, nU=g.nU,
-                        N0=NKFFT[0], N1=NKFFT[1], N2=NKFFT[2], nk=int(np.prod(NKFFT)),
+                        N0=NKFFT[0], N1=NKFFT[1], N2=NKFFT[2], nk=math.prod(int(n) for n in NKFFT),
                         nr0=int(g.nr[0]), nr1=int(g.nr[1]), nr2=int(g.nr[2]),
                         rmin0=int(g.rmin[0]), rmin1=int(g.rmin[1]), rmin2=int(g.rmin[2]),
                         maxPairLen=g.maxPairLen, maxSliceLen=g.maxSliceLen)
@@ -615,7 +624,7 @@ def field_arrays(dev, quantities, with_H, prec):
         fd = torch.tensor(np.array(desc, dtype=np.int32).reshape(-1), dtype=torch.int32, device=dev.device)
         XF = _complex_tensor(((2 if prec == PREC_FP32S else 1) * len(desc), nR, nw * nw), prec, dev.device)
         st = _lib.load().wbg_r2k_fields(_ptr(X), len(names), _ptr(dev.geom_tensors()['iR']), nR, nw, _ptr(fd),
-                                        len(desc), _ptr(dev.wcc_tensor(True)), ctypes.byref(lat), prec, _ptr(XF),
+                                        len(desc), _ptr(dev.geom_tensors()['wcc']), ctypes.byref(lat), prec, _ptr(XF),
                                         _stream())
         _lib.check(st, "wbg_r2k_fields")
         dev._cache[ck] = (XF, index, len(desc), fd)
@@ -634,7 +643,7 @@ def r2k(dev, dKs, NKFFT, quantities, with_H, prec, out=None, workspace=None, pha
     XF, index, nF, _ = field_arrays(dev, quantities, with_H, prec)
     nb = len(dKs)
     nw = dev.nw
-    nk = int(np.prod(NKFFT))
+    nk = math.prod(NKFFT)
     geo = r2k_geometry(dev, NKFFT)
     lib = _lib.load()
     ws = ctypes.c_size_t(0)
@@ -650,13 +659,11 @@ def r2k(dev, dKs, NKFFT, quantities, with_H, prec, out=None, workspace=None, pha
             sub = t[block_start:block_start + nb]
             ph += [sub, sub]
     else:
-        for p in dev.geom.phases(dKs, NKFFT):  # page-locked staging so the upload does not stall the host
-            if prec in DF64_PRECS:
-                host = torch.from_numpy(_df64_pairs(p)).pin_memory()
-            else:
-                host = torch.from_numpy(p.astype(np.complex128 if prec == PREC_FP64 else np.complex64)).pin_memory()
-            ph.append(host.to(dev.device, non_blocking=True))
-            ph.append(host)  # keep the staging buffer alive until the copy has run
+        # one upload from page-locked staging, so that it does not stall the host; the staging buffer is kept
+        # alive until the copy has run
+        tabs, host = dev._upload_phases(dev.geom.phases(dKs, NKFFT), _input_prec(prec), pin=True)
+        for t in tabs:
+            ph += [t, host]
     gt = dev.geom_tensors()
     name = {PREC_FP32: 'r2k_fp32', PREC_FP32S: 'r2k_fp32', PREC_FP64: 'r2k_fp64', PREC_DF64: 'r2k_df64',
             PREC_DF64C: 'r2k_df64c'}[prec]
@@ -730,7 +737,7 @@ def band_data(dev, dKs, NKFFT, quantities, precision='fp64', phases=None, block_
         quantities.discard('Od')  # a full rotation also serves diagonal-only readers
     nw = dev.nw
     NKFFT = [int(n) for n in NKFFT]
-    nk = int(np.prod(NKFFT))
+    nk = math.prod(NKFFT)
     nb = len(dKs)
     nkt = nb * nk
     keep = []
@@ -1110,7 +1117,11 @@ def _flag_word(v):
 
 
 def check_flag(bd):
-    _flag_word(int(bd._flag.item()))
+    check_flag_word(bd._flag)
+
+
+def check_flag_word(flag):
+    _flag_word(int(flag.item()))
 
 
 def check_flags(flags):

@@ -44,7 +44,7 @@ class Grid:
 
     def block_shifts(self):
         """dK = K/NKFFT for every K of the division grid (Kpoint.Kp_fullBZ), C order."""
-        g = np.stack(np.meshgrid(*[np.arange(n) for n in self.div], indexing='ij'), axis=-1).reshape(-1, 3)
+        g = np.ascontiguousarray(np.indices(self.div).reshape(3, -1).T)
         return (g / self.div[None, :]) / self.FFT[None, :]
 
     @property

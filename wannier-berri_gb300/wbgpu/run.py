@@ -361,8 +361,10 @@ def run(system, grid, calculators, precision='fp64', blocks_per_batch=None, devi
             c.accumulate(bd, system)
         flags.append(bd._flag.clone())  # the batch's QL flag (its buffer is reused by the next batch)
         del bd
+    # the results' scans are queued before the host waits for the flags
+    factor = 1.0 / grid.nblocks
+    results = ResultDict({k: c.result(system.cell_volume, nk, factor) for k, c in calculators.items()})
     engine.check_flags(flags)
     if tetra is not None:
         tetra.check()
-    factor = 1.0 / grid.nblocks
-    return ResultDict({k: c.result(system.cell_volume, nk, factor) for k, c in calculators.items()})
+    return results

@@ -40,7 +40,7 @@ def _band_quantities(system, quantities):
 
 
 def _tab_batch(dev, system, dKs, NKFFT, quantities, precision, degen_thresh, phases=None, block_start=0):
-    """Per-k, per-band values of `quantities` for a batch of blocks: dict q -> device tensor."""
+    """Per-k, per-band values of `quantities` for a batch of blocks: dict q -> array."""
     bd = engine.band_data(dev, dKs, NKFFT, _band_quantities(system, quantities), precision, phases=phases,
                           block_start=block_start)
     nkt, nw = bd.nk_total, bd.nw
@@ -59,11 +59,34 @@ def _tab_batch(dev, system, dKs, NKFFT, quantities, precision, degen_thresh, pha
                                     _stream())
         _lib.check(st, "wbg_berry_tabulate")
         tabs[key] = tab
-    engine.check_flag(bd)
     cols = {'energy': slice(0, 1), 'band_gradients': slice(1, 4)}
+    # Values and the solver's flag come back with one wait, in page-locked memory (large batches in pageable
+    # memory: what was page-locked stays with the process).  A few k-points: the columns in use in one copy, cut
+    # on the host; from 4 096 rows on a quantity's columns are packed on the device first (a kernel and a copy
+    # a quantity more, some 10 us, against numpy's strided copies: 4.48 -> 3.97 ms for 10 296 k-points x 13 bands)
+    pin = nkt * nw * 7 * 8 <= 64 << 20
+
+    def fetch(t):
+        h = torch.empty(t.shape, dtype=t.dtype, pin_memory=pin)
+        h.copy_(t.contiguous(), non_blocking=True)
+        return h
+
+    parts = {}  # (term selection, first and last column) -> host buffer
+    for q in quantities:
+        c, key = cols.get(q, slice(4, 7)), terms(q)
+        if nkt * nw < 4096:
+            use = [cols.get(p, slice(4, 7)) for p in quantities if terms(p) == key]
+            c = slice(min(u.start for u in use), max(u.stop for u in use))
+        if (key, c.start, c.stop) not in parts:
+            parts[(key, c.start, c.stop)] = fetch(tabs[key][:, :, c])
+    flag = fetch(bd._flag)
+    torch.cuda.current_stream(bd.E.device).synchronize()
+    engine.check_flag_word(flag)
     out = {}
     for q in quantities:
-        t = tabs[terms(q)][:, :, cols.get(q, slice(4, 7))]
+        c = cols.get(q, slice(4, 7))
+        lo, h = next((a, h) for (key, a, e), h in parts.items() if key == terms(q) and a <= c.start and c.stop <= e)
+        t = h.numpy()[:, :, c.start - lo:c.stop - lo]
         out[q] = t[:, :, 0] if q == 'energy' else t
     return out
 
@@ -81,7 +104,7 @@ def evaluate_k(system, k=(0., 0., 0.), quantities=(), iband=None, return_single_
     if iband is None:
         iband = np.arange(system.num_wann)
     iband = list(np.atleast_1d(iband))
-    result = {q: res[q][0].cpu().numpy()[iband] for q in quantities}
+    result = {q: res[q][0][iband] for q in quantities}
     if len(result) == 1 and not return_single_as_dict:
         return next(iter(result.values()))
     return result
@@ -107,7 +130,7 @@ def tabulate(system, grid, quantities=('energy', 'berry_curvature'), ibands=None
         res = _tab_batch(dev, system, shifts[i0:i0 + nb], grid.FFT, quantities, precision, degen_thresh,
                          phases=phases, block_start=i0)
         for q in quantities:
-            parts[q].append(res[q].cpu().numpy())
+            parts[q].append(res[q] if nb >= len(shifts) else res[q].copy())  # (page-locked buffers go round)
     sel = slice(None) if ibands is None else list(np.atleast_1d(ibands))
     out = {q: np.concatenate(parts[q])[:, sel] for q in quantities}
     N = np.array(grid.FFT)
