@@ -672,8 +672,8 @@ __global__ void berry_omega_kernel(const double* __restrict__ E, const typename 
 
 // ---------------------------------------------------------------------------------------
 // Omega traces for exactly Hermitian V and A in FP32 (the mixed path: lower-triangle inputs,
-// Hermitian rotation outputs), nw <= 32 C.  Lane l owns the bands (columns) l + 32 j, j < C,
-// and the warp walks the rows n, so every load is a coalesced row segment.  Each band sums its
+// Hermitian rotation outputs), nw <= L C, L lanes a k-point.  Lane l owns the bands (columns) l + L j, j < C,
+// and the group walks the rows n, so every load is a coalesced row segment.  Each band sums its
 // own trace.  For a pair (l, n) in different degenerate groups the term of band l is
 // T(l, n) = Re[-i D^a_ln D^b_nl - D^a_ln A^b_nl + D^b_ln A^a_nl] = -T(n, l) (D anti-Hermitian,
 // A Hermitian); the two lanes that meet the pair both evaluate the one canonical term T(p, q),
@@ -685,13 +685,13 @@ __global__ void berry_omega_kernel(const double* __restrict__ E, const typename 
 // and kept as a double.  The sea group's trace is the sum of its bands' traces over their own
 // degenerate groups: equal to the reference's sea trace in exact arithmetic, since the
 // cross-group A A terms inside the sea cancel pairwise as well.  Grouping and binning as in
-// berry_omega_kernel.  One warp per k-point, G warps per block.
+// berry_omega_kernel.  G k-points per block.
 // ---------------------------------------------------------------------------------------
-template <int C>
+template <int C, int L>
 __global__ void berry_omega_cols(const double* __restrict__ E, const float2* __restrict__ Xbar, int nFbar, int iV,
                                  int iA, int iO, int nw, int nk, int G, WbgScan sp, int internal_terms,
                                  int external_terms, wbg_u64* __restrict__ hist, int shist) {
-  constexpr int NWM = 32 * C;
+  constexpr int NWM = L * C;
   extern __shared__ double smb[];
   const int nh = 3 * sp.nEF;  // histogram entries [nEF][3], fixed point (shared or global)
   wbg_u64* sh = shist ? reinterpret_cast<wbg_u64*>(smb) : hist;
@@ -701,7 +701,7 @@ __global__ void berry_omega_cols(const double* __restrict__ E, const float2* __r
   int* start = reinterpret_cast<int*>(Ehl + 2 * G * NWM);   // [G][NWM]
   if (shist) fx_zero(sh, nh);
   __syncthreads();
-  const int grp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int grp = threadIdx.x / L, lane = threadIdx.x % L;
   double* myE = Es + grp * NWM;
   double* myT = tv + 3 * grp * NWM;
   float* myEh = Ehl + 2 * grp * NWM;
@@ -714,7 +714,7 @@ __global__ void berry_omega_cols(const double* __restrict__ E, const float2* __r
     const long long kk = valid ? k : nk - 1;
 #pragma unroll
     for (int j = 0; j < C; ++j) {
-      const int i = lane + 32 * j;
+      const int i = lane + L * j;
       if (i < nw) {
         const double e = E[kk * nw + i];
         const float eh = (float)e;
@@ -726,14 +726,14 @@ __global__ void berry_omega_cols(const double* __restrict__ E, const float2* __r
     __syncwarp();
 #pragma unroll
     for (int j = 0; j < C; ++j) {
-      const int i = lane + 32 * j;
+      const int i = lane + L * j;
       if (i < nw) myS[i] = (i == 0) || (myE[i] - myE[i - 1] > sp.degen_thresh);
     }
     __syncwarp();
     int below = 0, f0 = nw;
 #pragma unroll
     for (int j = 0; j < C; ++j) {
-      const int i = lane + 32 * j;
+      const int i = lane + L * j;
       if (i < nw) {
         below += myE[i] < sp.EFmin;
         if (myS[i]) {
@@ -743,15 +743,15 @@ __global__ void berry_omega_cols(const double* __restrict__ E, const float2* __r
         }
       }
     }
-    below = group_sum_i(below, 32);
-    f0 = group_min_i(f0, 32);
+    below = group_sum_i(below, L);
+    f0 = group_min_i(f0, L);
     const int bandmax = min(below, f0);
     // own bands: degenerate group [gs, ge) and whether the scan reads the band
     int gs[C], ge[C];
     bool need[C];
 #pragma unroll
     for (int j = 0; j < C; ++j) {
-      const int l = lane + 32 * j;
+      const int l = lane + L * j;
       gs[j] = ge[j] = 0;
       need[j] = false;
       if (l < nw) {
@@ -768,7 +768,7 @@ __global__ void berry_omega_cols(const double* __restrict__ E, const float2* __r
     for (int n = 0; n < nw; ++n) {  // warp-uniform
 #pragma unroll
       for (int j = 0; j < C; ++j) {
-        const int l = lane + 32 * j;
+        const int l = lane + L * j;
         if (l >= nw || !need[j]) continue;
         float2 Vn[3], An[3];
 #pragma unroll
@@ -811,7 +811,7 @@ __global__ void berry_omega_cols(const double* __restrict__ E, const float2* __r
     }
 #pragma unroll
     for (int j = 0; j < C; ++j) {
-      const int l = lane + 32 * j;
+      const int l = lane + L * j;
       if (l < nw)
         for (int g = 0; g < 3; ++g) myT[l * 3 + g] = need[j] ? 2.0 * acc[j][g].value() : 0.0;
     }
@@ -819,7 +819,7 @@ __global__ void berry_omega_cols(const double* __restrict__ E, const float2* __r
     if (valid) {
 #pragma unroll
       for (int j = 0; j < C; ++j) {
-        const int n = lane + 32 * j;
+        const int n = lane + L * j;
         if (n >= nw) continue;
         int g0 = -1, g1 = -1;
         bool sea = false;
@@ -2174,6 +2174,44 @@ size_t hist_smem(int nh, size_t rest, int& shist) {
   return (shist ? h : 0) + rest;
 }
 
+// Launch shape of a scan kernel (L lanes a k-point, G k-points a block, every block with a histogram of nh
+// entries): from G0 k-points a block the double and the fourfold, as long as every SM keeps a block, for more
+// warps an SM where the histograms are what limits them, and one wave of resident blocks, so that a block
+// zeroes and flushes one histogram for as many k-points as it can.  Mixed path, 1 001 levels, num_wann 32,
+// 55 296 k-points: 1.21 ms (4 warps and up to 16 blocks an SM) -> 0.70 ms (2 blocks of 16 warps).
+struct ScanShape {
+  int G, shist, grid;
+  size_t sm;
+};
+template <typename K, typename R>
+int scan_shape(K kern, int nk, int L, int G0, int nh, R rest, ScanShape& s) {
+  const size_t most = 220 * 1024;
+  s.G = G0;
+  s.sm = hist_smem(nh, rest(G0), s.shist);
+  if (s.sm > most) return WBG_ERR_SIZE;
+  int dev = 0, sms = 152, blocks = 1, threads = 0;
+  if (const cudaError_t e_ = cudaGetDevice(&dev)) return wbg_cuda_status(e_);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (const cudaError_t e_ = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most))
+    return wbg_cuda_status(e_);
+  for (int G = G0; G <= 4 * G0 && G * L <= 512; G *= 2) {
+    int shist = 0, b = 0;
+    const size_t sm = hist_smem(nh, rest(G), shist);
+    if (G > G0 && ((long long)G * sms > nk || shist < s.shist || sm > most)) break;
+    if (const cudaError_t e_ = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kern, G * L, sm))
+      return wbg_cuda_status(e_);
+    if (b * G * L <= threads) continue;
+    threads = b * G * L;
+    blocks = b;
+    s.G = G;
+    s.sm = sm;
+    s.shist = shist;
+  }
+  const long long n = ((long long)nk + s.G - 1) / s.G;
+  s.grid = (int)(n < (long long)sms * blocks ? n : (long long)sms * blocks);
+  return WBG_OK;
+}
+
 int lanes_for(int n) {
   int L = 1;
   while (L < n && L < 32) L <<= 1;
@@ -2282,44 +2320,37 @@ int wbg_berry_omega_run(const double* E, const void* Xbar, int nFbar, int iV, in
   if (sel) { spv.nEF = 0; hist = nullptr; tab = nullptr; }  // per-band values: no histogram
   const WbgScan* sp = &spv;
   if (fp64 == 2 && nw <= 128 && !tab && !sel) {  // FP32, exactly Hermitian V and A: column-per-lane kernel
-    const int C = (nw + 31) / 32;
-    const int G = 4;  // k-points (warps) per block
-    int shist = 0;
-    const size_t sm = hist_smem(3 * sp->nEF, (size_t)G * 32 * C * (8 + 24 + 8 + 4), shist);
-    if (sm > 220 * 1024) return WBG_ERR_SIZE;
-    int sms = 152;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
-    long long nblk = (nk + G - 1) / G;
-    const long long cap = (long long)sms * 16;
-    if (nblk > cap) nblk = cap;
-    void (*kern)(const double*, const float2*, int, int, int, int, int, int, int, WbgScan, int, int, wbg_u64*, int) =
-        C == 1 ? berry_omega_cols<1> : C == 2 ? berry_omega_cols<2> : C == 3 ? berry_omega_cols<3> : berry_omega_cols<4>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    kern<<<(int)nblk, 32 * G, sm, stream>>>(E, (const float2*)Xbar, nFbar, iV, iA, iO, nw, nk, G, *sp, internal_terms,
-                                           external_terms, (wbg_u64*)hist, shist);
+    const int C = (nw + 31) / 32, L = nw <= 8 ? 8 : nw <= 16 ? 16 : 32;
+    const auto kern = L == 8    ? berry_omega_cols<1, 8>
+                      : L == 16 ? berry_omega_cols<1, 16>
+                      : C == 1  ? berry_omega_cols<1, 32>
+                      : C == 2  ? berry_omega_cols<2, 32>
+                      : C == 3  ? berry_omega_cols<3, 32>
+                                : berry_omega_cols<4, 32>;
+    ScanShape sh;
+    const int st = scan_shape(kern, nk, L, 128 / L, 3 * sp->nEF,
+                              [&](int g) { return (size_t)g * L * C * (8 + 24 + 8 + 4); }, sh);
+    if (st != WBG_OK) return st;
+    kern<<<sh.grid, sh.G * L, sh.sm, stream>>>(E, (const float2*)Xbar, nFbar, iV, iA, iO, nw, nk, sh.G, *sp,
+                                               internal_terms, external_terms, (wbg_u64*)hist, sh.shist);
     return wbg_cuda_status(cudaGetLastError());
   }
   if (fp64 == 2) fp64 = 0;  // the general FP32 kernel does not need the symmetry
   const int L = lanes_for(nw);
-  const int G = 128 / L;
-  int shist = 0;
-  const size_t sm = hist_smem(3 * sp->nEF, (size_t)G * nw * (8 + 24 + 8 + 4), shist);
-  if (sm > 220 * 1024) return WBG_ERR_SIZE;
-  int sms = 152;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
-  long long nblk = (nk + G - 1) / G;
-  const long long cap = (long long)sms * 8;
-  if (nblk > cap) nblk = cap;
+  ScanShape sh;
+  auto rest = [&](int g) { return (size_t)g * nw * (8 + 24 + 8 + 4); };
   if (fp64) {
-    cudaFuncSetAttribute(berry_omega_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    berry_omega_kernel<double><<<(int)nblk, G * L, sm, stream>>>(E, (const double2*)Xbar, nFbar, iV, iA, iO, nw, nk, L,
-                                                                 G, *sp, internal_terms, external_terms, (wbg_u64*)hist, shist, tab,
-                                                                 bs);
+    const auto kern = berry_omega_kernel<double>;
+    const int st = scan_shape(kern, nk, L, 128 / L, 3 * sp->nEF, rest, sh);
+    if (st != WBG_OK) return st;
+    kern<<<sh.grid, sh.G * L, sh.sm, stream>>>(E, (const double2*)Xbar, nFbar, iV, iA, iO, nw, nk, L, sh.G, *sp,
+                                               internal_terms, external_terms, (wbg_u64*)hist, sh.shist, tab, bs);
   } else {
-    cudaFuncSetAttribute(berry_omega_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    berry_omega_kernel<float><<<(int)nblk, G * L, sm, stream>>>(E, (const float2*)Xbar, nFbar, iV, iA, iO, nw, nk, L,
-                                                                G, *sp, internal_terms, external_terms, (wbg_u64*)hist, shist, tab,
-                                                                 bs);
+    const auto kern = berry_omega_kernel<float>;
+    const int st = scan_shape(kern, nk, L, 128 / L, 3 * sp->nEF, rest, sh);
+    if (st != WBG_OK) return st;
+    kern<<<sh.grid, sh.G * L, sh.sm, stream>>>(E, (const float2*)Xbar, nFbar, iV, iA, iO, nw, nk, L, sh.G, *sp,
+                                               internal_terms, external_terms, (wbg_u64*)hist, sh.shist, tab, bs);
   }
   return wbg_cuda_status(cudaGetLastError());
 }
@@ -2353,20 +2384,15 @@ int wbg_berry_scan_run(const double* E, const void* Xbar, int nFbar, int iV, int
   }
   const int nc = scan_ncomp(formula);
   const int L = lanes_for(nw);
-  const int G = 128 / L;
-  int sms = 152;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
-  long long nblk = (nk + G - 1) / G;
-  if (nblk > (long long)sms * 8) nblk = (long long)sms * 8;
-#define WBG_SCAN(TT, NCM)                                                                                          \
-  do {                                                                                                             \
-    int shist = 0;                                                                                                 \
-    const size_t sm = hist_smem(nc * sp->nEF, (size_t)G * nw * (8 + 8 * NCM + 4), shist);                         \
-    if (sm > 220 * 1024) return WBG_ERR_SIZE;                                                                      \
-    cudaFuncSetAttribute(berry_scan_kernel<TT, NCM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);     \
-    berry_scan_kernel<TT, NCM><<<(int)nblk, G * L, sm, stream>>>(E, (const typename C2<TT>::t*)Xbar, nFbar, iV, iW, \
-                                                                 nw, nk, L, G, *sp, formula, sea, (wbg_u64*)hist,  \
-                                                                 shist, bs, fs);                                   \
+#define WBG_SCAN(TT, NCM)                                                                                           \
+  do {                                                                                                              \
+    const auto kern = berry_scan_kernel<TT, NCM>;                                                                   \
+    ScanShape sh;                                                                                                   \
+    const int st = scan_shape(kern, nk, L, 128 / L, nc * sp->nEF,                                                   \
+                              [&](int g) { return (size_t)g * nw * (8 + 8 * NCM + 4); }, sh);                       \
+    if (st != WBG_OK) return st;                                                                                    \
+    kern<<<sh.grid, sh.G * L, sh.sm, stream>>>(E, (const typename C2<TT>::t*)Xbar, nFbar, iV, iW, nw, nk, L, sh.G,  \
+                                               *sp, formula, sea, (wbg_u64*)hist, sh.shist, bs, fs);                \
   } while (0)
   if (nc == 27) {
     if (fp64) WBG_SCAN(double, 27);
@@ -2419,23 +2445,20 @@ int wbg_berry_product_run(const double* E, const void* Xbar, int nFbar, const wb
   const size_t per_group = (size_t)nw * (8 + 8 * (size_t)nc + 8 + 4);
   int G = 128 / L;
   while (G > 1 && (size_t)G * per_group > 96 * 1024) G /= 2;
-  int shist = 0;
-  const size_t sm = hist_smem(nc * spv.nEF, (size_t)G * per_group, shist);
-  if (sm > 220 * 1024) return WBG_ERR_SIZE;
-  int sms = 152;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
-  long long nblk = (nk + G - 1) / G;
-  if (nblk > (long long)sms * 8) nblk = (long long)sms * 8;
+  ScanShape sh;
+  auto rest = [&](int g) { return (size_t)g * per_group; };
   if (fp64) {
-    auto kern = berry_product_kernel<double, double2>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    kern<<<(int)nblk, G * L, sm, stream>>>(E, (const double2*)Xbar, nFbar, ps, nc, nw, nk, L, G, spv, sea,
-                                           (wbg_u64*)hist, shist, bs);
+    const auto kern = berry_product_kernel<double, double2>;
+    const int st = scan_shape(kern, nk, L, G, nc * spv.nEF, rest, sh);
+    if (st != WBG_OK) return st;
+    kern<<<sh.grid, sh.G * L, sh.sm, stream>>>(E, (const double2*)Xbar, nFbar, ps, nc, nw, nk, L, sh.G, spv, sea,
+                                               (wbg_u64*)hist, sh.shist, bs);
   } else {
-    auto kern = berry_product_kernel<double, float2>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    kern<<<(int)nblk, G * L, sm, stream>>>(E, (const float2*)Xbar, nFbar, ps, nc, nw, nk, L, G, spv, sea,
-                                           (wbg_u64*)hist, shist, bs);
+    const auto kern = berry_product_kernel<double, float2>;
+    const int st = scan_shape(kern, nk, L, G, nc * spv.nEF, rest, sh);
+    if (st != WBG_OK) return st;
+    kern<<<sh.grid, sh.G * L, sh.sm, stream>>>(E, (const float2*)Xbar, nFbar, ps, nc, nw, nk, L, sh.G, spv, sea,
+                                               (wbg_u64*)hist, sh.shist, bs);
   }
   return wbg_cuda_status(cudaGetLastError());
 }
@@ -2455,26 +2478,20 @@ int wbg_berry_morb_run(const double* E, const void* Xbar, int nFbar, int iV, int
     return WBG_ERR_ARG;
   const int L = lanes_for(nw);
   if ((nw + L - 1) / L > WBG_BAND_MAXPER) return WBG_ERR_SIZE;
-  const int G = 128 / L;
-  int shist = 0;
-  const size_t sm =
-      hist_smem(3 * sp->nEF, (size_t)G * nw * 8 + (size_t)G * (nw + 1) * 24 + (size_t)G * nw * 4, shist);
-  if (sm > 220 * 1024) return WBG_ERR_SIZE;
-  int sms = 152;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
-  long long nblk = (nk + G - 1) / G;
-  const long long cap = (long long)sms * 8;
-  if (nblk > cap) nblk = cap;
+  ScanShape sh;
+  auto rest = [&](int g) { return (size_t)g * nw * 8 + (size_t)g * (nw + 1) * 24 + (size_t)g * nw * 4; };
   if (fp64) {
-    cudaFuncSetAttribute(berry_morb_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    berry_morb_kernel<double><<<(int)nblk, G * L, sm, stream>>>(E, (const double2*)Xbar, nFbar, iV, iA, iO, iB, iC,
-                                                                nw, nk, L, G, *sp, internal_terms, external_terms,
-                                                                (wbg_u64*)hist, shist, bs);
+    const auto kern = berry_morb_kernel<double>;
+    const int st = scan_shape(kern, nk, L, 128 / L, 3 * sp->nEF, rest, sh);
+    if (st != WBG_OK) return st;
+    kern<<<sh.grid, sh.G * L, sh.sm, stream>>>(E, (const double2*)Xbar, nFbar, iV, iA, iO, iB, iC, nw, nk, L, sh.G, *sp,
+                                               internal_terms, external_terms, (wbg_u64*)hist, sh.shist, bs);
   } else {
-    cudaFuncSetAttribute(berry_morb_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    berry_morb_kernel<float><<<(int)nblk, G * L, sm, stream>>>(E, (const float2*)Xbar, nFbar, iV, iA, iO, iB, iC, nw,
-                                                               nk, L, G, *sp, internal_terms, external_terms,
-                                                               (wbg_u64*)hist, shist, bs);
+    const auto kern = berry_morb_kernel<float>;
+    const int st = scan_shape(kern, nk, L, 128 / L, 3 * sp->nEF, rest, sh);
+    if (st != WBG_OK) return st;
+    kern<<<sh.grid, sh.G * L, sh.sm, stream>>>(E, (const float2*)Xbar, nFbar, iV, iA, iO, iB, iC, nw, nk, L, sh.G, *sp,
+                                               internal_terms, external_terms, (wbg_u64*)hist, sh.shist, bs);
   }
   return wbg_cuda_status(cudaGetLastError());
 }
