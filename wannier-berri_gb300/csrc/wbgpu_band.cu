@@ -251,6 +251,150 @@ __global__ void rotate_tiled(const typename C2<T>::t* __restrict__ U, long long 
   }
 }
 
+// rotate_tiled for FP32 and nw a multiple of four, with 16-byte loads and stores (a thread's tile row is one
+// 32-byte sector) and the tiles above the diagonal of a lower-triangle field read as the transposed tile.
+// INWARP (nw = 8, 16: a k-point's threads lie in one warp): warp barriers, and T and the Hermitian
+// part's staging take the place of X, so that more k-points fit an SM.  Rows of X are nwp + 2 apart and
+// k-points one more, for the banks.  The same sums in the same order.  Bound by the latency of few warps
+// (125 registers; at 80 the spills cost more): 9 fields, 110 592 k-points of nw = 8 0.511 -> 0.287 ms, 8 192 of 12
+// 0.133 -> 0.102, of 16 0.163 -> 0.136, 4 096 of 20 0.182 -> 0.179, of 24 0.285 -> 0.263; of 28 0.435 -> 0.438 and 512
+// of 36 0.124 -> 0.134, so that it serves nw <= 24.
+// complex words of one k-point: U, X (and T)
+WBG_HD size_t tiled4_words(int nw, bool inwarp) {
+  return ((size_t)nw * nw + (size_t)nw * (nw + 2) + (inwarp ? 0 : (size_t)nw * nw)) | 1;
+}
+WBG_HD bool tiled4_inwarp(int nw) { return nw == 8 || nw == 16; }
+template <bool INWARP>
+__global__ void rotate_tiled4(const float2* __restrict__ U, long long strideU, const float2* __restrict__ X, int nFin,
+                              const int* __restrict__ fsel, const int* __restrict__ herm, int nFrot,
+                              float2* __restrict__ Xbar, int nw, int nk, int KB) {
+  extern __shared__ unsigned char smr[];
+  const int nt = nw / 4, tpk = nt * nt;  // tiles per dimension, threads per k-point
+  const int kl = threadIdx.x / tpk, tid = threadIdx.x % tpk;
+  const int ty = tid / nt, tx = tid % nt;
+  const int nw2 = nw * nw, m0 = 4 * ty, n0 = 4 * tx, ldx = nw + 2, ldt = INWARP ? ldx : nw;
+  float2* Us = reinterpret_cast<float2*>(smr) + (size_t)kl * tiled4_words(nw, INWARP);  // [nw][nw]
+  float2* Xs = Us + nw2;                    // [nw][ldx] X, then the Hermitian part's staging
+  float2* Ts = INWARP ? Xs : Xs + nw * ldx;  // [nw][ldt]
+  long long k = (long long)blockIdx.x * KB + kl;
+  const bool valid = k < nk;
+  if (!valid) k = nk - 1;
+  auto sync = [&]() {
+    if (INWARP) __syncwarp();
+    else __syncthreads();
+  };
+  float4 xv[4][2];
+  auto load_rows = [&](const float2* src) {
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) xv[a][h] = *reinterpret_cast<const float4*>(src + a * nw + 2 * h);
+  };
+  auto el = [&](int a, int b) {  // element (a, b) of the loaded tile
+    const float4 v = xv[a][b >> 1];
+    return b & 1 ? make_float2(v.z, v.w) : make_float2(v.x, v.y);
+  };
+  load_rows(U + k * strideU + m0 * nw + n0);
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int b = 0; b < 4; ++b) Us[(m0 + a) * nw + n0 + b] = el(a, b);
+  // a field's tile: loaded one field ahead, while the previous one is rotated
+  auto load_tile = [&](int f) {
+    const int fs = fsel[f];
+    const bool fok = fs >= 0 && fs < nFin;  // selection lives in device memory: validate here
+    const bool tr = (herm[f] & 4) && ty < tx;
+    load_rows(X + (k * nFin + (fok ? fs : 0)) * (long long)nw2 + (tr ? n0 * nw + m0 : m0 * nw + n0));
+  };
+  load_tile(0);
+  for (int f = 0; f < nFrot; ++f) {
+    const bool fbad = fsel[f] < 0 || fsel[f] >= nFin, lower = (herm[f] & 4) != 0;
+    const float nan = rnan<float>();
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const bool mir = lower && (ty < tx || (ty == tx && a < b));  // above the diagonal: the mirror's conjugate
+        float2 v = mir ? el(b, a) : el(a, b);
+        if (mir) v.y = -v.y;
+        if (lower && ty == tx && a == b) v.y = 0.f;
+        if (fbad) v = make_float2(nan, nan);
+        Xs[(m0 + a) * ldx + n0 + b] = v;
+      }
+    sync();
+    if (f + 1 < nFrot) load_tile(f + 1);
+    float2 acc[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) acc[a][b] = make_float2(0.f, 0.f);
+    for (int j = 0; j < nw; ++j) {  // T = X U
+      float2 xa[4], ub[4];
+#pragma unroll
+      for (int a = 0; a < 4; ++a) xa[a] = Xs[(m0 + a) * ldx + j];
+#pragma unroll
+      for (int b = 0; b < 4; ++b) ub[b] = Us[j * nw + n0 + b];
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) cfma(acc[a][b], xa[a], ub[b]);
+    }
+    if (INWARP) sync();  // X is read: T takes its place
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) Ts[(m0 + a) * ldt + n0 + b] = acc[a][b];
+    sync();
+    const int hmode = herm[f] & 3;
+    float2* dst = Xbar + (k * nFrot + f) * (long long)nw2;
+    if (hmode == 2) {  // diagonal only: Y_mm = sum_j conj(U_jm) T_jm, Hermitian part = Re
+      for (int m = tid; m < nw; m += tpk) {
+        float2 y = make_float2(0.f, 0.f);
+        for (int j = 0; j < nw; ++j) cfmac(y, Us[j * nw + m], Ts[j * ldt + m]);
+        if (valid) dst[m * nw + m] = real_only(y);
+      }
+      if (INWARP) sync();
+      continue;  // (not INWARP: the next field's barrier comes before T is written again)
+    }
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) acc[a][b] = make_float2(0.f, 0.f);
+    for (int j = 0; j < nw; ++j) {  // Y = U^dagger T
+      float2 ua[4], tb[4];
+#pragma unroll
+      for (int a = 0; a < 4; ++a) ua[a] = Us[j * nw + m0 + a];
+#pragma unroll
+      for (int b = 0; b < 4; ++b) tb[b] = Ts[j * ldt + n0 + b];
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) cfmac(acc[a][b], ua[a], tb[b]);
+    }
+    if (INWARP) sync();  // T is read
+    if (hmode != 0) {    // Hermitian part: the transposed tile comes from shared memory (X is read)
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) Xs[(m0 + a) * ldx + n0 + b] = acc[a][b];
+      sync();
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) acc[a][b] = herm_pair(acc[a][b], Xs[(n0 + b) * ldx + m0 + a]);
+      sync();
+    }
+    if (valid) {
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          *reinterpret_cast<float4*>(dst + (m0 + a) * nw + n0 + 2 * h) =
+              make_float4(acc[a][2 * h].x, acc[a][2 * h].y, acc[a][2 * h + 1].x, acc[a][2 * h + 1].y);
+    }
+  }
+}
+
 WBG_D int group_sum_i(int v, int L) {
   for (int off = L / 2; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
   return v;
@@ -2244,13 +2388,24 @@ int launch_rotate(const void* U, long long strideU, const void* X, int nFin, con
   }
   if (nw >= 5) {
     const int tpk = ((nw + 3) / 4) * ((nw + 3) / 4);
-    const size_t per_k = tiled_words(nw) * sizeof(V);
+    const bool wide = std::is_same<T, float>::value && nw % 4 == 0 && nw <= 24 && strideU % 2 == 0 &&
+                      ((reinterpret_cast<uintptr_t>(U) | reinterpret_cast<uintptr_t>(X) |
+                        reinterpret_cast<uintptr_t>(Xbar)) & 15) == 0;  // 16-byte pieces of every matrix
+    const bool inw = tiled4_inwarp(nw);
+    const size_t per_k = wide ? tiled4_words(nw, inw) * 8 : tiled_words(nw) * sizeof(V);
     // k-points per block: up to 256 threads and 64 KB, but no fewer blocks than two per SM (152)
     int KB = 1;
     while (KB * 2 * tpk <= 256 && (KB * 2) * per_k <= 64 * 1024 && nk / (KB * 2) >= 304) KB *= 2;
     if (KB * per_k <= 200 * 1024) {
       const int t = wbg_tuned(WBG_TUNE_ROTATE_KPOINTS, sizeof(T) == 8 ? 1 : 0, nw);
       if (t > 0 && tiled_kpoints_fit(t, tpk, per_k)) KB = t;
+      if (wide) {
+        const auto kern = inw ? rotate_tiled4<true> : rotate_tiled4<false>;
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+        kern<<<(nk + KB - 1) / KB, KB * tpk, KB * per_k, stream>>>((const float2*)U, strideU, (const float2*)X, nFin, fsel,
+                                                                 herm, nFrot, (float2*)Xbar, nw, nk, KB);
+        return wbg_cuda_status(cudaGetLastError());
+      }
       cudaFuncSetAttribute(rotate_tiled<T, VO>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
       rotate_tiled<T, VO><<<(nk + KB - 1) / KB, KB * tpk, KB * per_k, stream>>>(
           (const V*)U, strideU, (const V*)X, nFin, fsel, herm, nFrot, (VO*)Xbar, nw, nk, KB);
