@@ -1952,11 +1952,12 @@ __global__ void berry_deromega_kernel(const double* __restrict__ E, const VS* __
 // and no access down a column (XV(a, m, p) over lanes m) in the loop.
 // A block takes one k-point: a thread owns band m of the bands that contribute (compacted) and
 // every S-th l outside its group, S = threads / bands, so the lanes are filled whatever num_wann and
-// however many bands the window leaves; the S partial traces add up in order.  Bound by FP32 issue:
-// 44 instructions per double-float multiply-add (11 per real product: exact two-sum, errors collected).
-// AHC + dipole, num_wann 82, 512 k-points: 67.4 -> 11.3 ms; num_wann 21, 4 096 k-points: 12.8 -> 2.3 ms (both with the
-// other kernel's check of the k-points, 0.2-0.3 ms).  One pass over both sums (18 accumulators, 168 registers, 3 blocks
-// an SM) took 12.3 and 2.9 ms, 5 blocks an SM (spills) 15.8 and 2.35 ms.
+// however many bands the window leaves; the S partial traces add up in order.  Bound by the FP32 pipe:
+// 44 operations per double-float multiply-add (11 per real product: exact two-sum, errors collected), issued as 22
+// packed instructions on (re, im): 10.9 -> 9.9 and 2.20 -> 1.78 ms below, the same bits.
+// AHC + dipole, num_wann 82, 512 k-points: 67.4 -> 10.4 ms; num_wann 21, 4 096 k-points: 12.8 -> 1.9 ms (both with the
+// other kernel's check of the k-points, 0.1-0.5 ms).  In scalar instructions, one pass over both sums (18 accumulators, 168 registers, 3 blocks
+// an SM) took 12.3 and 2.9 ms instead of 11.3 and 2.3, 5 blocks an SM (spills) 15.8 and 2.35 ms.
 // ---------------------------------------------------------------------------------------
 constexpr int DH_THR = 128, DH_OCC = 4;
 
@@ -1970,21 +1971,26 @@ WBG_D cdf wmul(df64 w, float2 v) {
   r.y = df_quick(p, fmaf(w.lo, v.y, fmaf(w.hi, v.y, -p)));
   return r;
 }
-WBG_D void df_lazy_fmaf(df64& acc, df64 a, float b) {
-  const float p = a.hi * b;
-  const float e = fmaf(a.lo, b, fmaf(a.hi, b, -p));
-  const float s = acc.hi + p;
-  const float v = s - acc.hi;
-  const float t = (acc.hi - (s - v)) + (p - v);
-  acc.hi = s;
-  acc.lo = acc.lo + (t + e);
+// (re, im) += a (b.x, b.y) with a double-float and nb = -b, in packed FP32 instructions: the products' exact errors
+// collected in the low halves
+WBG_D void df_lazy_fma2(cdf& acc, df64 a, float2 b, float2 nb) {
+  const float2 ah = make_float2(a.hi, a.hi), m1 = make_float2(-1.0f, -1.0f), hi = make_float2(acc.x.hi, acc.y.hi);
+  const float2 np = __fmul2_rn(ah, nb);  // -p, p = a.hi b
+  const float2 e = __ffma2_rn(make_float2(a.lo, a.lo), b, __ffma2_rn(ah, b, np));
+  const float2 s = __ffma2_rn(np, m1, hi);                         // hi + p
+  const float2 v = __ffma2_rn(hi, m1, s);                          // s - hi
+  const float2 u = __ffma2_rn(__ffma2_rn(v, m1, s), m1, hi);       // hi - (s - v)
+  const float2 t = __ffma2_rn(__fadd2_rn(np, v), m1, u);           // + (p - v)
+  const float2 lo = __fadd2_rn(make_float2(acc.x.lo, acc.y.lo), __fadd2_rn(t, e));
+  acc.x.hi = s.x;
+  acc.y.hi = s.y;
+  acc.x.lo = lo.x;
+  acc.y.lo = lo.y;
 }
 WBG_D void smac(double2& acc, const double2& r, const double2& v) { cfma(acc, r, v); }
 WBG_D void smac(cdf& acc, const cdf& r, const float2& v) {
-  df_lazy_fmaf(acc.x, r.x, v.x);
-  df_lazy_fmaf(acc.x, r.y, -v.y);
-  df_lazy_fmaf(acc.y, r.x, v.y);
-  df_lazy_fmaf(acc.y, r.y, v.x);
+  df_lazy_fma2(acc, r.x, v, make_float2(-v.x, -v.y));
+  df_lazy_fma2(acc, r.y, make_float2(-v.y, v.x), make_float2(v.y, -v.x));
 }
 
 template <typename T> size_t deromega_herm_smem(int nw) {
