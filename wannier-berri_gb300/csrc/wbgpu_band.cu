@@ -1956,8 +1956,8 @@ __global__ void berry_deromega_kernel(const double* __restrict__ E, const VS* __
 // 44 operations per double-float multiply-add (11 per real product: exact two-sum, errors collected), issued as 22
 // packed instructions on (re, im): 10.9 -> 9.9 and 2.20 -> 1.78 ms below, the same bits.
 // AHC + dipole, num_wann 82, 512 k-points: 67.4 -> 10.4 ms; num_wann 21, 4 096 k-points: 12.8 -> 1.9 ms (both with the
-// other kernel's check of the k-points, 0.1-0.5 ms).  In scalar instructions, one pass over both sums (18 accumulators, 168 registers, 3 blocks
-// an SM) took 12.3 and 2.9 ms instead of 11.3 and 2.3, 5 blocks an SM (spills) 15.8 and 2.35 ms.
+// other kernel's check of the k-points, 0.1-0.5 ms).  In scalar instructions, one pass over both sums (18 accumulators,
+// 168 registers, 3 blocks an SM) took 12.3 and 2.9 ms instead of 11.3 and 2.3, 5 blocks an SM (spills) 15.8 and 2.35 ms.
 // ---------------------------------------------------------------------------------------
 constexpr int DH_THR = 128, DH_OCC = 4;
 
