@@ -500,11 +500,13 @@ __global__ void __launch_bounds__(KG_THR, 1)
 // FP64 path, NC = 9 or 27: the same sums in FP64 as a register-tiled product.  FR: f_w is real
 // (injection, shift current), MR: the elements are real (SHC, shift current) -- the products that are
 // zero by construction are not formed (1, 2 or 4 multiply-adds an output and record).  A block takes
-// K6_TW frequencies x 16 JN columns; sums run over one k-point's records in registers, then over the
-// block's k-points in shared memory, and go to `out` once.  Bound by the FP64 pipe; at 61 frequencies
-// x 3 levels x 27 components, num_wann 12 and 1 680 k-points: 10.8 ms with accumulators read and
-// written in shared memory for every record and flushed per k-point (and four multiply-adds each),
-// now 2.5 ms (the pairs: 1.6 -> 1.4 ms).
+// K6_TW frequencies x 16 JN columns; the sums over one k-point's records stay in registers and go to the
+// fixed-point `out` k-point by k-point, so that a result does not depend on which k-points share a block
+// or a launch (added up in FP64 over a block's k-points first, its last bits followed the batch size and the
+// number of SMs).  Bound by the FP64 pipe; at 61 frequencies x 3 levels x 27 components, num_wann 12 and
+// 1 680 k-points: 10.8 ms with accumulators read and written in shared memory for every record (and four
+// multiply-adds each), now 2.5 ms (the pairs: 1.6 -> 1.4 ms).  On their way out the sums pass through shared memory
+// and a loop: the additions unrolled over registers spilled and cost 1.5% of the call (5.78 against 5.70 ms).
 // ---------------------------------------------------------------------------------------
 constexpr int K6_TW = 64, K6_RC = 16, K6_THR = 256;
 template <bool FR, bool MR> struct K6 {
@@ -523,15 +525,15 @@ __global__ void __launch_bounds__(K6_THR, 2)
   typedef K6<FR, MR> K;
   constexpr int JN = K::JN, TC = K::TC, FW = K::FW, GW = K::GW, AW = K::AW;
   extern __shared__ __align__(16) unsigned char smg[];
-  double* accd = reinterpret_cast<double*>(smg);  // [4 JN AW][K6_THR]
-  double* Fs = accd + 4 * JN * AW * K6_THR;       // [K6_RC][K6_TW][FW]
+  double* sums = reinterpret_cast<double*>(smg);  // [4 JN AW][K6_THR] on their way from registers to the output
+  double* Fs = sums + 4 * JN * AW * K6_THR;       // [K6_RC][K6_TW][FW]
   double* Gs = Fs + K6_RC * K6_TW * FW;           // [K6_RC][TC][GW]
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int w0 = blockIdx.x * K6_TW, col0 = blockIdx.z * TC;
   const int ncol = kp.nEF * NC;
   const int jn = min(JN, (ncol - col0 + 15) / 16);  // column groups in use
   const int fgroup = formula >= WBG_DYN_SHC_SIMPLE && formula <= WBG_DYN_SHC_RYOO ? kShcFactor : formula;
-  for (int q = 0; q < 4 * JN * AW; ++q) accd[q * K6_THR + tid] = 0.0;
+  wbg_u64* bad = out + 4 * (long long)kp.nEF * kp.nOmega * NC;
   const long long k0 = (long long)blockIdx.y * kchunk;
   const long long k1 = min((long long)nk, k0 + kchunk);
   for (long long k = k0; k < k1; ++k) {
@@ -602,21 +604,17 @@ __global__ void __launch_bounds__(K6_THR, 2)
 #pragma unroll
       for (int j = 0; j < JN; ++j)
 #pragma unroll
-        for (int a = 0; a < AW; ++a) accd[((i * JN + j) * AW + a) * K6_THR + tid] += acc[i][j][a];
-  }
-  wbg_u64* bad = out + 4 * (long long)kp.nEF * kp.nOmega * NC;
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < JN; ++j) {
-      const int w = w0 + ty + 16 * i, col = col0 + tx + 16 * j;
+        for (int a = 0; a < AW; ++a) sums[((j * 4 + i) * AW + a) * K6_THR + tid] = acc[i][j][a];
+#pragma unroll 1
+    for (int q = 0; q < 4 * jn; ++q) {  // (a thread's own sums: no barrier)
+      const int w = w0 + ty + 16 * (q & 3), col = col0 + tx + 16 * (q >> 2);
       if (w >= kp.nOmega || col >= ncol) continue;
       const int e = col / NC, c = col - e * NC;
-      const double* a = accd + (i * JN + j) * AW * K6_THR + tid;
       wbg_u64* o = out + 4 * (((long long)e * kp.nOmega + w) * NC + c);
-      fx_add_double(o, a[0], bad);
-      if (AW == 2) fx_add_double(o + 2, a[(AW - 1) * K6_THR], bad);
+      fx_add_double(o, sums[q * AW * K6_THR + tid], bad);
+      if (AW == 2) fx_add_double(o + 2, sums[(q * AW + 1) * K6_THR + tid], bad);
     }
+  }
 }
 
 template <int NC, bool FR, bool MR>
