@@ -438,7 +438,7 @@ def column_list(dev, quantities, with_H, lower, rtol=1e-12):
 
 
 def fp64_columns(dev, quantities, nkt):
-    """Column list of an FP64 batch of `nkt` k-points (H and the quantities' fields) and the fields given by
+    """Column list of an FP64 run of `nkt` k-points (H and the quantities' fields) and the fields given by
     their lower triangle; (None, all False): every element."""
     if nkt >= FP64_LOWER_MIN_K and dev.hermitian_bases(0.0):
         return column_list(dev, quantities, True, True, 0.0)
@@ -571,10 +571,11 @@ MIXED_EIGH_REFINE_NW = (24, 32)
 # Berry-curvature dipole on two 12^3 blocks: 1.9e-6 and 4.8e-7).
 MIXED_FIELDS_PREC = 3  # PREC_FP32S
 MIXED_DF64_QUANTITIES = {'V'}
-# From this many k-points a batch's FP64 transform writes only the lower triangles of the fields whose
+# From this many k-points a run's FP64 transform writes only the lower triangles of the fields whose
 # R-space matrices are Hermitian bit for bit (half the transform: 18.9 -> 9.6 ms per 13 824 k-points at
 # num_wann 32, 5.0 ms on conjugate pairs of R); below, building the column list on a
-# fresh system (0.1 ms) costs more than it saves.
+# fresh system (0.1 ms) costs more than it saves.  The two ways differ in the last bits, so the k-points of the
+# whole run decide (`run_kpoints`), not those of a batch: results do not depend on how its blocks are batched.
 FP64_LOWER_MIN_K = 64
 # Arithmetic of the mixed path's Berry-curvature dipole (wbg_berry_deromega fp64 argument): 2 =
 # double-float on the complex64 band-basis fields.  Its sums over intermediate bands of V D terms
@@ -724,13 +725,14 @@ def rotate(U, fields, nFin, sel, herm, nw, nk, fp64, out=None):
     return out, (s, h)
 
 
-def band_data(dev, dKs, NKFFT, quantities, precision='fp64', phases=None, block_start=0, ws=None):
+def band_data(dev, dKs, NKFFT, quantities, precision='fp64', phases=None, block_start=0, ws=None, run_kpoints=None):
     """Stages 1-3 for a batch of blocks.  precision 'fp64': everything in FP64;
     'mixed': H(k) transform and eigh in double-float, the other fields and the rotation in FP32.
     All per-batch arrays live in persistent buffers of `dev` (reused by the next call: consume
     the returned BandData before calling again).  `phases` maps a precision code to the tables
     of DeviceSystem.grid_phases; `block_start` is the index of dKs[0] in that grid.  `ws`: the
-    Workspace holding the per-batch arrays (default: the system's own), one per concurrent run."""
+    Workspace holding the per-batch arrays (default: the system's own), one per concurrent run.
+    `run_kpoints`: k-points of the run's grid (FP64_LOWER_MIN_K; default: those of this batch)."""
     require_cuda()
     quantities = set(quantities)
     if 'O' in quantities:
@@ -762,7 +764,7 @@ def band_data(dev, dKs, NKFFT, quantities, precision='fp64', phases=None, block_
     _lib.check(_lib.load().wbg_eigh_workspace_size(nw, nkt, ctypes.byref(ews)), "wbg_eigh_workspace_size")
     ework = arena.buffer('eigh_ws', (int(ews.value),), torch.uint8)
     if precision == 'fp64':
-        cols, lower_in = fp64_columns(dev, quantities, nkt)
+        cols, lower_in = fp64_columns(dev, quantities, nkt if run_kpoints is None else run_kpoints)
         fields, index, nF, k1 = fields_for(quantities, True, PREC_FP64, 'fields', cols=cols)
         keep.append(k1)
         U = arena.buffer('U', (nkt, nw, nw), torch.complex128)
@@ -903,7 +905,7 @@ def _fill_phase_inputs(dev, tabs, dKs, NKFFT, phases, block_start):
 
 
 def band_data_graphed(dev, dKs, NKFFT, quantities, precision='fp64', phases=None, block_start=0, ws=None,
-                      more=True):
+                      more=True, run_kpoints=None):
     """band_data (stages 1-3) replayed from a CUDA graph of its launch sequence.
 
     One graph per (FFT grid, blocks per batch, quantities, precision) and workspace.  The first
@@ -917,13 +919,16 @@ def band_data_graphed(dev, dKs, NKFFT, quantities, precision='fp64', phases=None
     workspace; a capture (which synchronises the device) is made only then.  Stage timers
     (set_timer) need plain launches: with a timer set this is band_data itself.  The returned
     BandData is valid until the next batch on the same workspace, as for band_data."""
+    run = {} if run_kpoints is None else dict(run_kpoints=run_kpoints)
     if _TIMER is not None:
-        return band_data(dev, dKs, NKFFT, quantities, precision, phases=phases, block_start=block_start, ws=ws)
+        return band_data(dev, dKs, NKFFT, quantities, precision, phases=phases, block_start=block_start, ws=ws, **run)
     arena = ws if ws is not None else dev.workspace()
     NKFFT = [int(n) for n in NKFFT]
     quantities = frozenset(quantities)
     nb = len(dKs)
     key = (tuple(NKFFT), nb, quantities, precision)
+    if run_kpoints is not None and precision == 'fp64':  # runs on both sides of the line share a workspace
+        key += (run_kpoints >= FP64_LOWER_MIN_K,)
     ent = arena.graphs.get(key)
     if ent is not None and (ent.dev is not dev or ent.generation != arena.generation):
         del arena.graphs[key]
@@ -936,7 +941,7 @@ def band_data_graphed(dev, dKs, NKFFT, quantities, precision='fp64', phases=None
     seen = arena.__dict__.setdefault('_graph_seen', set())
     if (key, id(dev)) not in seen or not more:
         seen.add((key, id(dev)))
-        return band_data(dev, dKs, NKFFT, quantities, precision, phases=phases, block_start=block_start, ws=ws)
+        return band_data(dev, dKs, NKFFT, quantities, precision, phases=phases, block_start=block_start, ws=ws, **run)
     # capture: fixed inputs, one plain run on them (this batch's result; every buffer at its final
     # size), then the same call captured
     g = dev.geom
@@ -952,21 +957,21 @@ def band_data_graphed(dev, dKs, NKFFT, quantities, precision='fp64', phases=None
                                         torch.complex64))
         tabs[p] = lst
     _fill_phase_inputs(dev, tabs, dKs, NKFFT, phases, block_start)
-    bd = band_data(dev, dKs, NKFFT, quantities, precision, phases=tabs, block_start=0, ws=ws)
+    bd = band_data(dev, dKs, NKFFT, quantities, precision, phases=tabs, block_start=0, ws=ws, **run)
     generation = arena.generation
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph, capture_error_mode='relaxed'):
-        gbd = band_data(dev, dKs, NKFFT, quantities, precision, phases=tabs, block_start=0, ws=ws)
+        gbd = band_data(dev, dKs, NKFFT, quantities, precision, phases=tabs, block_start=0, ws=ws, **run)
     if arena.generation != generation:  # band_data grew a buffer while capturing: do not keep it
         raise RuntimeError("band_data_graphed: workspace changed during capture")
     arena.graphs[key] = _GraphEntry(graph, gbd, tabs, generation, dev)
     return bd
 
 
-def energies(dev, dKs, NKFFT, precision='fp64', out=None, phases=None, block_start=0, ws=None):
+def energies(dev, dKs, NKFFT, precision='fp64', out=None, phases=None, block_start=0, ws=None, run_kpoints=None):
     """Eigenvalues of H(k) only (np.linalg.eigvalsh) for a batch of blocks: (nblocks*nk, nw)
     float64 written to `out` when given.  FP64 ('fp64') or double-float ('mixed') transform and
-    tridiagonal QL, no eigenvectors.  Returns (E, flag)."""
+    tridiagonal QL, no eigenvectors.  `run_kpoints` as for band_data.  Returns (E, flag)."""
     require_cuda()
     nw = dev.nw
     NKFFT = [int(n) for n in NKFFT]
@@ -975,7 +980,7 @@ def energies(dev, dKs, NKFFT, precision='fp64', out=None, phases=None, block_sta
     flag = arena.buffer('flag_E', (1,), torch.int32)
     flag.zero_()
     if precision == 'fp64':
-        cols, lower_in = fp64_columns(dev, set(), nkt)
+        cols, lower_in = fp64_columns(dev, set(), nkt if run_kpoints is None else run_kpoints)
         lower, prec, mode = False, PREC_FP64, 1 | (EIGH_LOWER if lower_in[0] else 0)
     elif precision == 'mixed':
         lower, cols = 'Ham' in dev.hermitian_bases(), None
@@ -1039,7 +1044,7 @@ class TetraCorners:
         for i0 in range(0, len(cb), batch):
             n = min(batch, len(cb) - i0)
             _, flag = energies(dev, shifts[i0:i0 + n], fft, precision, out=self.Ec[i0 * nk:(i0 + n) * nk],
-                               phases=phases, block_start=i0, ws=ws)
+                               phases=phases, block_start=i0, ws=ws, run_kpoints=self.nblocks_total * nk)
             self.flags.append(flag.clone())
         self.device = dev.device
 
@@ -1080,7 +1085,7 @@ class BlockCorners(TetraCorners):
     s = 4 sx + 2 sy + sz (0: minus side) at Ecorner row 8 b + s; the kernels address them through
     wbg_tetra_grid.per_block.  Blocks are identified by their position in `shifts`."""
 
-    def __init__(self, dev, shifts, cells, NKFFT, precision='fp64', ws=None):
+    def __init__(self, dev, shifts, cells, NKFFT, precision='fp64', ws=None, run_kpoints=None):
         fft = np.array(NKFFT, dtype=int) * np.ones(3, dtype=int)
         self.grid = _lib.TetraGrid((ctypes.c_int * 3)(1, 1, 1), (ctypes.c_int * 3)(*fft.tolist()), 1)
         shifts, cells = np.asarray(shifts, dtype=float), np.asarray(cells, dtype=float)
@@ -1095,7 +1100,7 @@ class BlockCorners(TetraCorners):
         for i0 in range(0, len(corner_shifts), batch):
             n = min(batch, len(corner_shifts) - i0)
             _, flag = energies(dev, corner_shifts[i0:i0 + n], fft, precision, out=self.Ec[i0 * nk:(i0 + n) * nk],
-                               ws=ws)
+                               ws=ws, run_kpoints=run_kpoints)
             self.flags.append(flag.clone())
         self.device = dev.device
 

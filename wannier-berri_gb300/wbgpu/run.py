@@ -32,11 +32,12 @@ def more_batches_of_size(nblocks, nb, i0):
     return nblocks - (i0 + n_this) >= n_this
 
 
-def block_results(dev, system, shifts, NKFFT, calculators, precision, cells=None):
+def block_results(dev, system, shifts, NKFFT, calculators, precision, cells=None, run_kpoints=None):
     """One result per block -- what the reference's calculators return for one Data_K (normalised
     by the block's k-points, K-point factor 1): [{key: EnergyResult}] for the blocks at `shifts`.
     Each block gets fresh copies of the calculators; batches of blocks share stages 1-3.
-    `cells`: each block's dense-grid cell (dK_block / NKFFT), for tetrahedron calculators."""
+    `cells`: each block's dense-grid cell (dK_block / NKFFT), for tetrahedron calculators.
+    `run_kpoints`: k-points of the run's grid (engine.band_data)."""
     quantities = set()
     for c in calculators.values():
         quantities |= c.quantities(system)
@@ -49,8 +50,9 @@ def block_results(dev, system, shifts, NKFFT, calculators, precision, cells=None
     for i0 in range(0, len(shifts), nb):
         corners = None
         if tetra:  # computed before band_data: both use the system's default workspace
-            corners = engine.BlockCorners(dev, shifts[i0:i0 + nb], cells[i0:i0 + nb], NKFFT, precision)
-        bd = engine.band_data(dev, shifts[i0:i0 + nb], NKFFT, quantities, precision)
+            corners = engine.BlockCorners(dev, shifts[i0:i0 + nb], cells[i0:i0 + nb], NKFFT, precision,
+                                          run_kpoints=run_kpoints)
+        bd = engine.band_data(dev, shifts[i0:i0 + nb], NKFFT, quantities, precision, run_kpoints=run_kpoints)
         if corners is not None:
             corners.attach(bd, np.arange(bd.nblocks))
         for b in range(bd.nblocks):
@@ -77,6 +79,7 @@ class Refinement:
 
     def __init__(self, system, grid, calculators, adpt_num_iter, adpt_mesh=2, adpt_fac=1):
         self.div, self.fft = np.array(grid.div, dtype=int), np.array(grid.FFT, dtype=int)
+        self.run_kpoints = grid.nblocks * grid.nk_per_block
         if adpt_num_iter < 0:
             adpt_num_iter = -adpt_num_iter * np.prod(self.div) / np.prod(adpt_mesh) / adpt_fac / 3
         self.num_iter = int(round(adpt_num_iter))
@@ -138,7 +141,8 @@ def run_adaptive(system, grid, calculators, precision, dev, adpt_num_iter, adpt_
     """run() with adaptive refinement (Refinement): returns (ResultDict, K, dK, factor)."""
     ref = Refinement(system, grid, calculators, adpt_num_iter, adpt_mesh, adpt_fac)
     while True:
-        ref.add(block_results(dev, system, ref.new_shifts(), ref.fft, ref.templates, precision, ref.new_cells()))
+        ref.add(block_results(dev, system, ref.new_shifts(), ref.fft, ref.templates, precision, ref.new_cells(),
+                              ref.run_kpoints))
         if not ref.refine():
             break
     return ref.total(), np.array(ref.K), np.array(ref.dK), np.array(ref.fac)
@@ -184,7 +188,7 @@ def _omega_scores(bd, degen_thresh):
 
 
 def _evaluate_blocks(dev, system, shifts, NKFFT, step, calculators, quantities, precision, scores,
-                     degen_thresh=1e-4, cached_phases=True):
+                     degen_thresh=1e-4, cached_phases=True, run_kpoints=None):
     """Stages 1-3 and every calculator over blocks of NKFFT points (spacing `step`, None: 1/NKFFT)
     at `shifts`; with `scores` the per-k Berry-curvature scores of the blocks in order (device)."""
     nk = int(np.prod(NKFFT))
@@ -198,7 +202,8 @@ def _evaluate_blocks(dev, system, shifts, NKFFT, step, calculators, quantities, 
             keep.append(host)
     out, flags = [], []
     for i0 in range(0, len(shifts), nb):
-        bd = engine.band_data(dev, shifts[i0:i0 + nb], NKFFT, quantities, precision, phases=phases, block_start=i0)
+        bd = engine.band_data(dev, shifts[i0:i0 + nb], NKFFT, quantities, precision, phases=phases, block_start=i0,
+                              run_kpoints=run_kpoints)
         for c in calculators.values():
             c.accumulate(bd, system)
         if scores:
@@ -301,7 +306,7 @@ def run_refine_omega(system, grid, calculators, precision='mixed', rounds=1, top
         scores = None
         for job in ref.jobs():
             sc = _evaluate_blocks(dev, system, job.shifts, job.fft, job.step, job.calcs, ref.quantities, precision,
-                                  job.scores, degen_thresh, cached_phases=ref.round == 0)
+                                  job.scores, degen_thresh, cached_phases=ref.round == 0, run_kpoints=ref.n_grid)
             if job.scores:
                 scores = sc
         if not ref.end_round(scores):
@@ -351,10 +356,11 @@ def run(system, grid, calculators, precision='fp64', blocks_per_batch=None, devi
     for i0 in range(0, len(shifts), nb):
         if cuda_graph:  # a graph is captured only when a later batch of this size will replay it
             bd = engine.band_data_graphed(dev, shifts[i0:i0 + nb], grid.FFT, quantities, precision, phases=phases,
-                                          block_start=i0, more=more_batches_of_size(len(shifts), nb, i0))
+                                          block_start=i0, more=more_batches_of_size(len(shifts), nb, i0),
+                                          run_kpoints=grid.nblocks * nk)
         else:
             bd = engine.band_data(dev, shifts[i0:i0 + nb], grid.FFT, quantities, precision, phases=phases,
-                                  block_start=i0)
+                                  block_start=i0, run_kpoints=grid.nblocks * nk)
         if tetra is not None:
             tetra.attach(bd, block_ids[i0:i0 + nb])
         for c in calculators.values():

@@ -318,7 +318,7 @@ class Server:
         job = req.oref.jobs()[j]
         ph = {p: t for p, t in req.ophases[j].items() if not isinstance(p, tuple)}
         bd = engine.band_data(dev, job.shifts[idx], job.fft, req.quantities, self.precision, phases=ph,
-                              block_start=int(idx[0]), ws=req.ws)
+                              block_start=int(idx[0]), ws=req.ws, run_kpoints=req.oref.n_grid)
         for c in job.calcs.values():
             c.accumulate(bd, system)
         if job.scores:
@@ -329,9 +329,10 @@ class Server:
         corners = None
         if any(getattr(c, 'tetra', False) for c in req.refine.templates.values()):
             corners = engine.BlockCorners(dev, req.shifts[idx], req.cells[idx], req.grid.FFT, self.precision,
-                                          ws=req.ws)
+                                          ws=req.ws, run_kpoints=req.refine.run_kpoints)
             req.flags.extend(corners.flags)
-        bd = engine.band_data(dev, req.shifts[idx], req.grid.FFT, req.quantities, self.precision, ws=req.ws)
+        bd = engine.band_data(dev, req.shifts[idx], req.grid.FFT, req.quantities, self.precision, ws=req.ws,
+                              run_kpoints=req.refine.run_kpoints)
         if corners is not None:
             corners.attach(bd, np.arange(bd.nblocks))
         for b in range(bd.nblocks):  # per-block results: fresh calculators for every block
@@ -381,6 +382,7 @@ class Server:
             return
         with torch.cuda.stream(req.stream):
             contiguous = np.all(np.diff(idx) == 1)
+            kpts = req.grid.nblocks * req.grid.nk_per_block
             stages = engine.band_data
             if self.cuda_graph:  # capture only when a later batch of this request has the same size
                 more = later_batch_of_size(req.batches, req.next_batch, len(idx))
@@ -389,9 +391,10 @@ class Server:
                 bd = self._issue_adaptive(req, idx, system, dev)
             elif contiguous:
                 bd = stages(dev, shifts[idx], req.grid.FFT, req.quantities, self.precision,
-                            phases=req.phases, block_start=int(idx[0]), ws=req.ws)
+                            phases=req.phases, block_start=int(idx[0]), ws=req.ws, run_kpoints=kpts)
             else:
-                bd = stages(dev, shifts[idx], req.grid.FFT, req.quantities, self.precision, ws=req.ws)
+                bd = stages(dev, shifts[idx], req.grid.FFT, req.quantities, self.precision, ws=req.ws,
+                            run_kpoints=kpts)
             if req.tetra is not None:
                 req.tetra.attach(bd, idx)
             for c in req.calculators.values():

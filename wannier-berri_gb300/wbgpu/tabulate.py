@@ -39,10 +39,11 @@ def _band_quantities(system, quantities):
     return {'V', 'A', 'Od'} if ext else {'V'}
 
 
-def _tab_batch(dev, system, dKs, NKFFT, quantities, precision, degen_thresh, phases=None, block_start=0):
+def _tab_batch(dev, system, dKs, NKFFT, quantities, precision, degen_thresh, phases=None, block_start=0,
+               run_kpoints=None):
     """Per-k, per-band values of `quantities` for a batch of blocks: dict q -> array."""
     bd = engine.band_data(dev, dKs, NKFFT, _band_quantities(system, quantities), precision, phases=phases,
-                          block_start=block_start)
+                          block_start=block_start, run_kpoints=run_kpoints)
     nkt, nw = bd.nk_total, bd.nw
     lib = _lib.load()
     iA, iO = bd.index.get('A', 0), bd.index.get('Od', 0)
@@ -128,7 +129,7 @@ def tabulate(system, grid, quantities=('energy', 'berry_curvature'), ibands=None
     parts = {q: [] for q in quantities}
     for i0 in range(0, len(shifts), nb):
         res = _tab_batch(dev, system, shifts[i0:i0 + nb], grid.FFT, quantities, precision, degen_thresh,
-                         phases=phases, block_start=i0)
+                         phases=phases, block_start=i0, run_kpoints=grid.nblocks * nk)
         for q in quantities:
             parts[q].append(res[q] if nb >= len(shifts) else res[q].copy())  # (page-locked buffers go round)
     sel = slice(None) if ibands is None else list(np.atleast_1d(ibands))
