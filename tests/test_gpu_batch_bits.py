@@ -72,3 +72,14 @@ def test_tabulated_and_refined_batches(monkeypatch, iters):
     b = go()
     for q in a:
         assert np.isfinite(a[q]).all() and np.array_equal(a[q], b[q]), q
+
+
+@pytest.mark.parametrize("nw", [5, 23])
+def test_odd_numbers_of_k_points_and_bands(nw):
+    """FP64 pair records of 9 k-points with an odd number of pairs each (the complex elements start on 16 bytes all the
+    same), against 18 k-points at once."""
+    s = wsys.System_R.from_dict(models.random_tb(nw, 1, LAT, seed=nw, keys=('Ham', 'AA', 'SS')))
+    opt = dict(Efermi=np.linspace(-0.5, 0.5, 5), omega=np.linspace(0.0, 4.0, 7), smr_fixed_width=0.05)
+    cal = lambda: {'optical': C.OpticalConductivity(**opt), 'shift': C.ShiftCurrent(sc_eta=0.04, **opt),
+                   'injection': C.InjectionCurrent(**opt), 'shc': C.SHC(SHC_type='simple', **opt)}
+    _same(s, wbgpu.Grid(s, NKdiv=(1, 1, 2), NKFFT=(3, 3, 1)), cal, (2, 1))

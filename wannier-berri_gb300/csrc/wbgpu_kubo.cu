@@ -697,8 +697,10 @@ int wbg_dynamic_run(const double* E, const void* Xbar, int nFbar, const wbg_dyna
   if (workspace_bytes < wbg_dynamic_workspace_bytes(F, nw, nk, kp->nEF)) return WBG_ERR_WORKSPACE;
   const int P = nw * nw;
   char* w = (char*)workspace;
-  double* rec_dE = (double*)w; w += (size_t)nk * P * 8;
+  // M first: its FP64 elements are read and written in 16-byte pieces, and after nk P doubles (odd for an odd
+  // number of k-points and of bands) it would start in the middle of one
   void* rec_M = w; w += (size_t)nk * P * 16 * nc;
+  double* rec_dE = (double*)w; w += (size_t)nk * P * 8;
   void* rec_fE = w; w += (size_t)nk * P * 8 * kp->nEF;
   int* count = (int*)w;
   const size_t smp = 8 * pairs_words(nw) + (F == WBG_DYN_SHIFT ? (size_t)nw * nw * (fp64 ? 8 : 4) : 0);
