@@ -197,8 +197,12 @@ int wbg_eigh_batched_noalloc(const void* H, long long strideH, int nw, int nk, d
  * fp64 == 0 and nw == 32 run on the tensor cores (tcgen05, products split into three TF32
  * terms, FP32 accumulation) when X is 16-byte aligned.  fp64 == 1 with 4 <= nw <= 128 and fp64 == 2
  * with 32 < nw <= 128 (16-byte aligned U and X) also run on the tensor cores: operands in 8-bit slices
- * whose fp16 products sum exactly, one rounding per GEMM; a field (or U) with a non-finite element
- * gives NaN throughout.  Other cases on the CUDA cores. */
+ * whose fp16 products sum exactly up to nw = 64 (above, sums of the lower slices may round at 2^-44 of
+ * theirs), one rounding per GEMM.  Operands are fixed point relative to the largest element of each row of X
+ * and of each column of U and X U, so that blocks which U does not mix keep their own accuracy whatever
+ * their sizes; within such a vector the error is relative to its largest element (2^-58 of the product of two
+ * of them, fp64 == 2: 2^-50), not to each element.  Subnormal elements count as zero; a field (or U) with a
+ * non-finite element gives NaN throughout.  Other cases on the CUDA cores. */
 int wbg_rotate(const void* U, long long strideU, const void* X, int nFin, const int* fsel, const int* herm,
                int nFrot, void* Xbar, int nw, int nk, int fp64, void* stream);
 

@@ -2,26 +2,33 @@
 // cores: the operands are cut into 8-bit slices whose products the tensor cores sum exactly.
 // Included by wbgpu_rotate_tc.cu inside its namespace (shared tcgen05 / mbarrier helpers).
 //
-// Every operand is brought to 64-bit fixed point relative to the largest exponent of its matrix,
-// v with |v| < 2^62, and written as signed digits v = sum_i d_i 2^(56 - 8 i), d_i in [-128, 127]:
+// The scheme is Ozaki's (K. Ozaki, T. Ogita, S. Oishi, S. M. Rump, Numer. Algorithms 59, 2012): slices
+// short enough that their products sum without rounding.
+//
+// Every operand is brought to 64-bit fixed point relative to the largest exponent of its vector along the
+// contraction -- a row of X, a column of U, a column of T = X U (whose rows enter with the exponents of the
+// rows of X) --, v with |v| < 2^62, and written as signed digits v = sum_i d_i 2^(56 - 8 i), d_i in [-128, 127]:
 // the bytes of v + 0x8080..80, less 128 each.  A digit is an exact fp16 number, a product of two
 // an integer below 2^14, and the products of one significance g = i + j, summed over K <= 256 and
-// the pairs of a group, stay below 2^24 (up to K = 128; beyond, only the groups g >= 4 could pass it,
-// whose last unit is 2^-44 of the result): FP32 accumulation in tensor memory is exact.  The NG
+// the pairs of a group, stay below 2^24 (up to K = 128; beyond, that is above nw = 64, only the groups g >= 4
+// could pass it, whose last unit is 2^-44 of the result): FP32 accumulation in tensor memory is exact.  The NG
 // groups g < NG are kept (8 for FP64: 36 pairs; 7 for double-float: 28) and recombined in 64-bit
 // integers: sum_g acc_g 2^(8 (NG - 1 - g)).  The dropped pairs lie 2^-58 (FP64) and 2^-50
-// (double-float) below the largest products, so each GEMM rounds once, like an FP64 sum of exact
-// products.  Against 113-bit products, 2-norm, random X and unitary U: 5.0e-17 at nw = 32 and
-// 7.4e-17 at nw = 128, where the CUDA-core FP64 chains gave 3.8e-16 and 7.6e-16.  The scale is one per
-// matrix: with elements spread over e^+-16 the error is 1e-16 (chains: 4e-16) up to nw = 32 and
-// 1.3e-15 (chains: 6e-16) at nw = 128.
+// (double-float) below the product of the two vectors' largest elements, so each GEMM rounds once, like an FP64 sum
+// of exact products.  What that floor leaves open, next to FP64 products of every element: a sum in which
+// the large elements of a row of X meet only elements of U below 2^-9 of their column's largest.  Subnormals
+// count as zero.
+// Error against 113-bit products, 2-norm, random X and unitary U: 4.9e-17 at nw = 32 and 5.5e-17 at nw = 128, with
+// elements of X spread over e^+-16 5.4e-17 and 8.2e-17; the CUDA-core FP64 chains gave 3.8e-16, 7.6e-16, 4e-16 and
+// 6e-16.  One scale per matrix gave 1.3e-15 in the last case and lost small blocks next to large ones.
 //
 // Bound by the CUDA cores: cutting the operands (about 40 instructions an element), recombining
 // the groups and the conversions run on integer units, since the FP64 pipe (64 times slower than FP32)
 // is what this avoids.  nw = 32, 9 fields, 13 824 k-points: 44.8 ms (CUDA-core FP64, 97% of the pipe)
-// -> 5.7 ms; of the 44 k cycles of a 96-row tile 13 k wait for the products (36 pairs x 4 K steps of
-// M = 128, N = 64: 4.6 k at full rate per GEMM).  nw = 96, 9 fields, 512 k-points: 27.7 ms
-// (double-float) -> 4.5 ms, 53.4 ms (FP64) -> 4.6 ms.
+// -> 5.9 ms (as with one scale per matrix; T goes to its columns through shared memory, so that a thread finds most
+// of a column's exponent by itself and writes its digits in 16-byte pieces: from the rows' side, with warp
+// reductions, 6.6 ms).  nw = 8, 110 592 k-points: 3.1 ms (2.9 with one scale).  nw = 96, 9 fields, 512 k-points:
+// 27.7 ms (double-float) -> 3.8 ms, 53.4 ms (FP64) -> 4.0 ms.
 //
 // Complex products are embedded in real ones as in the TF32 kernel above; operand rows are 128-byte
 // (64-byte) swizzled K-major rows of 64 (32) fp16.  Consecutive B slices are consecutive rows of
@@ -263,8 +270,14 @@ template <int NG, int KMAX> WBG_D void oz_cols4(uint32_t taddr, int ncol, int sh
   }
 }
 
-// left shift that brings values whose magnitudes have the largest high word hw just below 2^62
-WBG_D int oz_norm(int hw) { return hw == 0 ? 30 : max(0, __clz(hw) - 2); }
+// Exponent of a value q 2^ex for the scale of its column: |q| < 2^bits with bits >= 32 (a smaller q is an
+// integer all the same, and loses nothing at this scale), 0 of q = 0
+WBG_D int oz_top(long long q, int ex) {
+  const int h = (int)(q >> 32);
+  return q != 0 ? ex + 64 - __clz(h ^ (h >> 31)) : 0;
+}
+// q 2^s (s < 63), the fraction cut off (floor)
+WBG_D long long oz_shift(long long q, int s) { return s >= 0 ? q << min(s, 62) : q >> min(-s, 63); }
 WBG_D int warp_max(int v) { return __reduce_max_sync(0xffffffffu, v); }
 
 // ---------------------------------------------------------------------------------------
@@ -272,6 +285,7 @@ WBG_D int warp_max(int v) { return __reduce_max_sync(0xffffffffu, v); }
 // in a 128-row tile), both GEMMs share the embedded U.  KP = 16 (nw <= 8), 32 (nw <= 16) or 64 fp16
 // of K; 8 KP threads a CTA and 64 / KP CTAs an SM (512 tensor memory columns in all).
 // ---------------------------------------------------------------------------------------
+constexpr int OZ_LDQ = 129;  // 64-bit words from a column of T to the next: its readers fall on distinct banks
 template <int KP> constexpr int oz_small_smem() { return 8 * 128 * KP * 2 + 8 * KP * KP * 2 + 1024; }
 
 template <int KP>
@@ -290,20 +304,26 @@ __global__ void __launch_bounds__(8 * KP, 64 / KP)
   unsigned char* Bs = As + NG * ASTR;
   __shared__ __align__(8) uint64_t mbar;
   __shared__ uint32_t tmem_base_s;
-  __shared__ int abort_s, ue_s;
+  __shared__ int abort_s, ubad_s;
   __shared__ int code_s[OZ_FMAX];  // per field: -1 invalid selection, else source | herm << 28
-  __shared__ int fe_s[128], qm_s[128];  // per field of the tile: largest exponent of X, high word of max |T|
+  // largest exponents: of each column of U, of each row (field, m) of X, of each column (field, n) of T (exponent of
+  // the row of X + bits, 0: the column is zero); fields with a non-finite element
+  __shared__ int ue_s[32], xe_s[128], te_s[128], fbad_s[32];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t mb = smem_u32(&mbar);
   if (tid == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mb) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     abort_s = 0;
-    ue_s = 1;
+    ubad_s = 0;
   }
   if (tid < 128) {
-    fe_s[tid] = 1;
-    qm_s[tid] = 0;
+    xe_s[tid] = 1;
+    te_s[tid] = 0;
+  }
+  if (tid < 32) {
+    ue_s[tid] = 1;
+    fbad_s[tid] = 0;
   }
   for (int f = tid; f < nFrot; f += THR) {
     const int fs = fsel[f];
@@ -329,6 +349,7 @@ __global__ void __launch_bounds__(8 * KP, 64 / KP)
   const int ldst = nwp + 1;  // staging: [row][m'] re plane, then im plane
   long long* stre = reinterpret_cast<long long*>(As);
   long long* stim = stre + 128 * ldst;
+  long long* tq = stre;  // between the GEMMs: T, [column][row]
   const unsigned long long wait_ns = g_tc_wait_ns;
   uint32_t phase = 0;
   // task of the X loads: 8 columns n0.. of row r; 8 lanes take 8 rows (16-byte stores: no conflicts).
@@ -362,11 +383,11 @@ __global__ void __launch_bounds__(8 * KP, 64 / KP)
         u[c] = ok ? Uk[(j0 + c) * nw + n] : make_double2(0.0, 0.0);
         e = max(e, oz_cexp(u[c]));
       }
-      e = warp_max(e);
-      if (lane == 0) atomicMax(&ue_s, e);
+      if (j0 < nw) atomicMax(&ue_s[n], e);
+      if (e >= Cfg::EMAX) ubad_s = 1;
       __syncthreads();
       if (j0 < nwp) {
-        const int eu = ue_s;
+        const int eu = ue_s[n];
         long long v[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) v[c] = oz_re(u[c], eu);
@@ -378,7 +399,6 @@ __global__ void __launch_bounds__(8 * KP, 64 / KP)
         oz_put4x2<NG>(Bs, bstr, oz_off<KP>(nwp + n, cr) + h, oz_off<KP>(n, ci) + h, 0x80008000u, v);
       }
     }
-    const int eu = ue_s;
     for (int t = 0; t < ntiles; ++t) {
       const int f0 = t * fpt, nfl = min(fpt, nFrot - f0), rows = nfl * nw;
       // ---- A1: rows (fl, m), K = [Re X[m][:] | Im X[m][:]]
@@ -390,11 +410,12 @@ __global__ void __launch_bounds__(8 * KP, 64 / KP)
           if (xlow && 8 * xc8 + c == xm) xr[c].y = 0.0;  // a mirrored field's diagonal is real
           e = max(e, oz_cexp(xr[c]));
         }
-        atomicMax(&fe_s[xfl], e);
+        atomicMax(&xe_s[xrow], e);
+        if (e >= Cfg::EMAX) fbad_s[xfl] = 1;
       }
       __syncthreads();
       if (xrow < 128) {
-        const int ex = xrow < rows ? fe_s[xfl] : 1;
+        const int ex = xe_s[xrow];
         long long v[8];
 #pragma unroll
         for (int c = 0; c < 8; ++c) v[c] = oz_re(xr[c], ex);
@@ -416,59 +437,46 @@ __global__ void __launch_bounds__(8 * KP, 64 / KP)
       if (!wait_all(mb, phase, &abort_s, wait_ns)) break;
       phase ^= 1;
       tc_fence_after();
-      // ---- T in fixed point: thread (field, m) holds columns c0.. of [Re T[m][:] | Im T[m][:]]
+      // ---- T in fixed point: thread (field, m) holds columns c0.. of [Re T[m][:] | Im T[m][:]]; to its columns
+      // through shared memory, [column][row]
       const bool live = 32 * quarter < rows;  // warp-uniform: some row of this warp is in use
-      const int fl = row < rows ? row / nw : 0, m = row - fl * nw;
-      long long q[16];
       if (live) {
-        int hm = 0;
 #pragma unroll
         for (int c = 0; c < 16; c += 4) {
           if (c < ncg) {
-            oz_cols4<NG, KP>(tbase + lane_base + c0 + c, ncol, SH, q + c);
+            long long q[4];
+            oz_cols4<NG, KP>(tbase + lane_base + c0 + c, ncol, SH, q);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) hm = max(hm, (int)((q[c + i] ^ (q[c + i] >> 63)) >> 32));
+            for (int i = 0; i < 4; ++i) tq[(c0 + c + i) * OZ_LDQ + row] = q[i];
           }
         }
-        if (row < rows) atomicMax(&qm_s[fl], hm);
       }
       __syncthreads();
-      const int nsh = oz_norm(qm_s[fl]);
-      if (live) {  // ---- A2: row (fl, n), K = m: [Re T[m][n] | -Im T[m][n]]
-        const bool even = (nw & 1) == 0;  // rows 2 i, 2 i + 1 belong to one field: exchanged for 4-byte stores
+      // ---- A2: row (fl, n), K = m: [Re T[m][n] | -Im T[m][n]], thread as for X: 8 m of one row, both parts
+      long long tr[8], ti[8];
+      if (xrow < rows) {
+        int te = 0;
 #pragma unroll
-        for (int c = 0; c < 16; c += 2) {
-          const bool im = c0 + c >= nwp;
-          const int n = c0 + c - (im ? nwp : 0), kk = (im ? nwp : 0) + m;
-          if (c >= ncg || n >= nw) continue;  // warp-uniform
-          long long a = q[c] << nsh, b = q[c + 1] << nsh;
-          if (im) {
-            a = -a;
-            b = -b;
-          }
-          const int r0 = fl * nw + n;
-          if (even) {  // even lanes take column n of rows m, m + 1, odd lanes column n + 1 of rows m - 1, m
-            const bool odd = lane & 1;
-            const long long o = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
-            const unsigned long long wa = oz_bias(odd ? o : a), wb = oz_bias(odd ? b : o);
-            unsigned char* d0 = As + oz_off<KP>(r0 + odd, kk >> 3) + (kk & 6) * 2;
-            if (row < rows) {
-#pragma unroll
-              for (int i = 0; i < NG; ++i)
-                *reinterpret_cast<uint32_t*>(d0 + i * ASTR) = oz_dig2(oz_word(wa, i), oz_word(wb, i), 3 - (i & 3));
-            }
-          } else if (row < rows) {
-            const unsigned long long wa = oz_bias(a), wb = oz_bias(b);
-            unsigned char* d0 = As + oz_off<KP>(r0, kk >> 3) + (kk & 7) * 2;
-            unsigned char* d1 = As + oz_off<KP>(r0 + 1, kk >> 3) + (kk & 7) * 2;
-#pragma unroll
-            for (int i = 0; i < NG; ++i) {
-              const uint32_t d = oz_dig2(oz_word(wa, i), oz_word(wb, i), 3 - (i & 3));
-              *reinterpret_cast<unsigned short*>(d0 + i * ASTR) = (unsigned short)d;
-              if (n + 1 < nw) *reinterpret_cast<unsigned short*>(d1 + i * ASTR) = (unsigned short)(d >> 16);
-            }
-          }
+        for (int c = 0; c < 8; ++c) {
+          const int m = 8 * xc8 + c, j = xfl * nw + m;
+          tr[c] = m < nw ? tq[xm * OZ_LDQ + j] : 0;
+          ti[c] = m < nw ? tq[(nwp + xm) * OZ_LDQ + j] : 0;
+          const int ex = m < nw ? xe_s[j] : 0;
+          te = max(te, max(oz_top(tr[c], ex), oz_top(ti[c], ex)));
         }
+        atomicMax(&te_s[xrow], te);
+      }
+      __syncthreads();
+      if (xrow < 128) {  // at the scale of the column of T: its rows' exponents come in, so that K has one exponent
+        const int te = te_s[xrow];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const int sh = xrow < rows && 8 * xc8 + c < nw ? 62 + xe_s[xfl * nw + 8 * xc8 + c] - te : 0;
+          tr[c] = xrow < rows ? oz_shift(tr[c], sh) : 0;
+          ti[c] = xrow < rows ? -oz_shift(ti[c], sh) : 0;
+        }
+        oz_put8<NG>(As, ASTR, oz_off<KP>(xrow, xc8), tr);
+        oz_put8<NG>(As, ASTR, oz_off<KP>(xrow, cpr + xc8), ti);
       }
       tc_fence_before();
       fence_async_smem();
@@ -510,25 +518,32 @@ __global__ void __launch_bounds__(8 * KP, 64 / KP)
         const int r = (int)__umulhi((uint32_t)e, magic), n = e - r * nw;  // row (field, m') and column n
         const int f = (int)__umulhi((uint32_t)r, magic), mr = r - f * nw;
         const int code = code_s[f0 + f], hmode = (code >> 28) & 3;
-        const bool bad = code < 0 || fe_s[f] >= Cfg::EMAX || eu >= Cfg::EMAX;
+        const bool bad = code < 0 || fbad_s[f] || ubad_s;
         if (code >= 0 && hmode == 2 && n != mr) continue;
-        const int E = 2 * EP - oz_norm(qm_s[f]) + fe_s[f] + 2 * eu - 3 * Cfg::BIAS;
+        int te = te_s[f * nw + n];
         const int o = (f * nw + n) * ldst + mr;  // Y[m'][n] = conj(Y^H[n][m'])
-        long long re = stre[o], im = -stim[o];
-        if (hmode != 0) {  // + Y^H[m'][n], halved in the exponent
-          const int p = r * ldst + n;
-          re += stre[p];
-          im += stim[p];
+        long long re = stre[o], im = stim[o];
+        if (hmode != 0) {  // + Y^H[m'][n] at the larger of the two scales, halved in the exponent
+          const int p = r * ldst + n, d = te_s[r] - te, so = min(max(d, 0), 63), sp = min(max(-d, 0), 63);
+          re = (re >> so) + (stre[p] >> sp);
+          im = (im >> so) - (stim[p] >> sp);
+          te = max(te, te_s[r]);
         }
+        im = -im;
+        const int E = 2 * EP - 62 + te + ue_s[n] + ue_s[mr] - 3 * Cfg::BIAS;
         Xbar[(k * ldf + f0 + f) * (long long)nw2 + mr * nw + n] =
             bad ? oz_nan(double2()) : oz_pack(double2(), re, im, hmode != 0 ? E - 1 : E);
       }
       __syncthreads();  // TMEM, the operands and the staging are free
       if (tid < 128) {
-        fe_s[tid] = 1;
-        qm_s[tid] = 0;
+        xe_s[tid] = 1;
+        te_s[tid] = 0;
       }
-      if (tid == 0 && t + 1 == ntiles) ue_s = 1;
+      if (tid < 32) {
+        fbad_s[tid] = 0;
+        if (t + 1 == ntiles) ue_s[tid] = 1;
+      }
+      if (tid == 0 && t + 1 == ntiles) ubad_s = 0;
       __syncthreads();
     }
   }
@@ -554,12 +569,53 @@ __global__ void __launch_bounds__(8 * KP, 64 / KP)
 // Hermitian part on input and write the lower triangle with its mirror, as rotate_panel does, so
 // that the stored matrix is Hermitian bit for bit.
 // ---------------------------------------------------------------------------------------
-// Bound by the cutting: issue slots 46% active, the tensor pipe 27%.  One buffer of 32 rows, every product waited
+// Bound by the cutting.  One buffer of 32 rows, every product waited
 // for: 17.3 ms at nw = 82 (double-float, 36 fields, 512 k-points) and 8.1 ms at nw = 48 (9 fields, 2 048);
 // two buffers with all threads meeting at each stage: 17.7 and 7.0 ms; this, with a warp for the products and
-// full / done barriers a stage, so that no cutting warp waits for another one: 14.7 and 6.2 ms.
+// full / done barriers a stage, so that no cutting warp waits for another one: 14.0 and 5.7 ms (13.8 and 5.4 ms with one
+// scale per matrix).
 constexpr int OZ_PN = 32, OZ_WK = 512, OZ_THR = OZ_WK + 32;  // 16 warps at the operands, one for the products
 template <int DF> constexpr int oz_large_smem() { return 2 * OzCfg<DF>::NG * (128 + 64) * 64 + 1024; }
+
+// Largest exponents of the columns of U (mode 3) or of the rows of X as the kernel reads it: mode 0 as it is, 1 its
+// Hermitian part (element (m, n) is part of row n, too), 2 the lower triangle and its mirror.  Coalesced, all 16 warps;
+// a function of its own, so that its registers do not push the caller's out: nw = 82 as below 14.8 -> 14.1 ms.
+template <int DF>
+__device__ __noinline__ void oz_scales(const typename OzCfg<DF>::VI* __restrict__ M, int nw, int warp, int lane, int mode,
+                                       int* e_s, int* bad_s) {
+  typedef typename OzCfg<DF>::VI VI;
+  int ec[4] = {1, 1, 1, 1}, er[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int m = warp + i * (OZ_WK / 32);
+    er[i] = 1;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {  // of a lower triangle only m >= n counts, of its diagonal the real part
+      const int n = 32 * c + lane;
+      if (m < nw && n < nw && (mode != 2 || m >= n)) {
+        const VI v = M[m * nw + n];
+        const int e = oz_cexp(mode == 2 && m == n ? oz_real(v) : v);
+        er[i] = max(er[i], e);
+        ec[c] = max(ec[c], e);
+      }
+    }
+  }
+  int top = 1;
+  if (mode != 3)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int m = warp + i * (OZ_WK / 32);
+      if (m >= nw) break;
+      const int e = warp_max(er[i]);
+      if (lane == 0) atomicMax(&e_s[m], e);
+    }
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    if (mode != 0 && 32 * c < nw) atomicMax(&e_s[32 * c + lane], ec[c]);
+    top = max(top, ec[c]);
+  }
+  if (top >= OzCfg<DF>::EMAX) *bad_s = 1;
+}
 
 template <int DF>
 __global__ void __launch_bounds__(OZ_THR, 1)
@@ -583,7 +639,10 @@ __global__ void __launch_bounds__(OZ_THR, 1)
   long long* stim = stre + 128 * LDS;
   __shared__ __align__(8) uint64_t mbar[4];  // full[2]: an arrival a warp; done[2]: the products' commit
   __shared__ uint32_t tmem_base_s;
-  __shared__ int abort_s, ue_s, fe_s, qm_s;
+  // largest exponents of each column of U, each row of X and each column of the panel of T (0: zero); non-finite
+  // elements of U and of the field
+  __shared__ int ue_s[128], xe_s[128], te_s[OZ_PN];
+  __shared__ int abort_s, ubad_s, fbad_s;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t full = smem_u32(mbar), done = full + 16;
   if (tid == 0) {
@@ -663,34 +722,18 @@ __global__ void __launch_bounds__(OZ_THR, 1)
     // ---- largest exponents of U_k and of the field (kept while the CTA stays on them)
     const bool newk = k != kprev, newf = newk || f != fprev;
     if (named_any(1, OZ_WK, !ok || *ab)) break;
+    if (tid < 128) {
+      if (newk) ue_s[tid] = 1;
+      if (newf) xe_s[tid] = 1;
+    }
+    if (tid < OZ_PN) te_s[tid] = 0;
     if (tid == 0) {
-      if (newk) ue_s = 1;
-      if (newf) fe_s = 1;
-      qm_s = 0;
+      if (newk) ubad_s = 0;
+      if (newf) fbad_s = 0;
     }
     wsync();
-    if (newk) {
-      int e = 1;
-#pragma unroll 4
-      for (int i = tid; i < nw2; i += OZ_WK) e = max(e, oz_cexp(Uk[i]));
-      e = warp_max(e);
-      if (lane == 0) atomicMax(&ue_s, e);
-    }
-    if (newf) {
-      int e = 1;
-#pragma unroll 2
-      for (int m = warp; m < nw; m += OZ_WK / 32)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {  // of a lower-triangle field only m >= n counts, of its diagonal the real part
-          const int n = 32 * c + lane;
-          if (n < nw && (inmode != 2 || m >= n)) {
-            const VI v = Xf[m * nw + n];
-            e = max(e, oz_cexp(inmode == 2 && m == n ? oz_real(v) : v));
-          }
-        }
-      e = warp_max(e);
-      if (lane == 0) atomicMax(&fe_s, e);
-    }
+    if (newk) oz_scales<DF>(Uk, nw, warp, lane, 3, ue_s, &ubad_s);
+    if (newf) oz_scales<DF>(Xf, nw, warp, lane, inmode, xe_s, &fbad_s);
     kprev = k;
     fprev = f;
     const PI* Xp = reinterpret_cast<const PI*>(Xf) + apart;
@@ -709,6 +752,7 @@ __global__ void __launch_bounds__(OZ_THR, 1)
         br[q] = n0 + lane < nw && j < nw ? Up[2 * (j * nw + n0 + lane) + bpart] : oz_zero(PI());
       }
     };
+    int eua = 0;  // exponent of the column of U that this thread's row of U^H is
     auto load_uh = [&](int i) {  // stage i of GEMM2: row m' of U^H: U[j][m']
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
@@ -716,17 +760,18 @@ __global__ void __launch_bounds__(OZ_THR, 1)
         xr[q] = am < nw && j < nw ? Up[2 * (j * nw + am) + apart] : oz_zero(PI());
       }
     };
-    auto put_uh = [&](int eu) {
+    auto put_uh = [&]() {
       if (am < nw && ok) {
         long long v[8];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) v[q] = oz_part(xr[q], eu);
+        for (int q = 0; q < 8; ++q) v[q] = oz_part(xr[q], eua);
         oz_put8<NG>(As + (g & 1) * STAGE, ASTR, oz_off<KP>(am, akc), v);
       }
     };
     load_x(0);
     wsync();
-    const int eu = ue_s, ex = fe_s;
+    const int ex = xe_s[am], eub = ue_s[n0 + lane];
+    eua = ue_s[am];
     // ---- GEMM1
     for (int i = 0; i < nst; ++i) {
       if (i >= 2) wait_stage(g - 2);  // (the previous unit's stages are done)
@@ -759,8 +804,8 @@ __global__ void __launch_bounds__(OZ_THR, 1)
         const int rc = bj >> 3;
         const uint32_t h = (bj & 7) * 2;
         oz_put2x2<NG>(B, BSTR, oz_off<KP>(bpart ? 32 + lane : lane, rc) + h,
-                      oz_off<KP>(bpart ? lane : 32 + lane, 2 + rc) + h, bpart ? 0x80008000u : 0u, oz_part(br[0], eu),
-                      oz_part(br[1], eu));
+                      oz_off<KP>(bpart ? lane : 32 + lane, 2 + rc) + h, bpart ? 0x80008000u : 0u, oz_part(br[0], eub),
+                      oz_part(br[1], eub));
       }
       stage_full();
       if (i + 1 < nst) load_x(i + 1);
@@ -768,29 +813,33 @@ __global__ void __launch_bounds__(OZ_THR, 1)
     }
     // the first stage of U^H while the last products run
     wait_stage(g - 2);
-    put_uh(eu);
+    put_uh();
     load_uh(1);
     wait_stage(g - 1);
     tc_fence_after();
     // ---- T: thread (row j) holds 16 columns n of Re (half 0) or Im (half 1) T[j][n0 + 16 sub ..]
     long long q[16];
     const bool live = 32 * quarter < nw;
+    const int exr = xe_s[row];
     if (live && ok) {
-      int hmx = 0;
+      int top = 0;
 #pragma unroll
       for (int c = 0; c < 16; c += 4) {
         oz_cols4<NG, 256>(tbase + lane_base + c, 64, SH, q + c);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           if (row >= nw) q[c + i] = 0;
-          hmx = max(hmx, (int)((q[c + i] ^ (q[c + i] >> 63)) >> 32));
+          const int e = warp_max(oz_top(q[c + i], exr));
+          if (lane == c + i) top = e;
         }
       }
-      hmx = warp_max(hmx);
-      if (lane == 0) atomicMax(&qm_s, hmx);
+      if (lane < 16) atomicMax(&te_s[16 * sub + lane], top);
     }
     wsync();
-    const int nsh = oz_norm(qm_s);
+    // to the scale of the column of T: its row's exponent comes in, so that K has one exponent
+    if (live)
+#pragma unroll
+      for (int c = 0; c < 16; ++c) q[c] = oz_shift(q[c], 62 + exr - te_s[16 * sub + c]);
     // lanes l and l + 16 exchange half of their columns, so that the 16 rows of a stage lie on all lanes: lane l
     // then holds columns 16 sub + 8 (l >> 4) .. + 7 of rows l & 15 (q[0 .. 7]) and 16 + (l & 15) (q[8 .. 15])
 #pragma unroll
@@ -807,7 +856,7 @@ __global__ void __launch_bounds__(OZ_THR, 1)
     for (int i = 0; i < nst; ++i) {
       if (i > 0) {
         if (i >= 2) wait_stage(g - 2);
-        put_uh(eu);
+        put_uh();
         if (i + 1 < nst) load_uh(i + 1);
       }
       if (quarter == i >> 1 && ok) {  // this quarter's rows j
@@ -816,7 +865,7 @@ __global__ void __launch_bounds__(OZ_THR, 1)
         unsigned char* b1 = B + (kb & 6) * 2;
 #pragma unroll
         for (int c = 0; c < 8; c += 2) {
-          const long long a = (i & 1 ? q[8 + c] : q[c]) << nsh, b = (i & 1 ? q[9 + c] : q[c + 1]) << nsh;
+          const long long a = i & 1 ? q[8 + c] : q[c], b = i & 1 ? q[9 + c] : q[c + 1];
           const long long o = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
           const unsigned long long wa = oz_bias(odd ? o : a), wb = oz_bias(odd ? b : o);
           const int n = 16 * sub + 8 * (lane >> 4) + c + odd;
@@ -848,22 +897,24 @@ __global__ void __launch_bounds__(OZ_THR, 1)
     }
     tc_fence_before();
     wsync();
-    const bool bad = !fok || ex >= Cfg::EMAX || eu >= Cfg::EMAX;
-    const int E = 2 * EP - nsh + ex + 2 * eu - 3 * Cfg::BIAS;
+    const bool bad = !fok || fbad_s || ubad_s;
+    auto yexp = [&](int nl) { return 2 * EP - 62 + te_s[nl] + ue_s[n0 + nl] - 3 * Cfg::BIAS; };  // less that of row m'
     VO* dst = Xbar + (k * nFrot + f) * (long long)nw2;
-    const int mode = hm & 3, n = n0 + lane;
+    const int mode = hm & 3, n = n0 + lane, E = yexp(lane);
     for (int m = warp; m < nw && ok; m += OZ_WK / 32) {
       if (n >= nw || (mode != 0 && n > m) || (mode == 2 && n != m)) continue;
-      VO y = oz_pack(VO(), stre[m * LDS + lane], stim[m * LDS + lane], E);
+      VO y = oz_pack(VO(), stre[m * LDS + lane], stim[m * LDS + lane], E + ue_s[m]);
       if (mode != 0 && m == n) y.y = 0;
       dst[m * nw + n] = bad ? oz_nan(y) : y;
     }
     if (mode == 1 && ok) {  // the mirror: row n of the panel, columns m > n
-      for (int nl = warp; nl < OZ_PN && n0 + nl < nw; nl += OZ_WK / 32)
+      for (int nl = warp; nl < OZ_PN && n0 + nl < nw; nl += OZ_WK / 32) {
+        const int En = yexp(nl);
         for (int m = n0 + nl + 1 + lane; m < nw; m += 32) {
-          const VO y = oz_pack(VO(), stre[m * LDS + nl], -stim[m * LDS + nl], E);
+          const VO y = oz_pack(VO(), stre[m * LDS + nl], -stim[m * LDS + nl], En + ue_s[m]);
           dst[(n0 + nl) * nw + m] = bad ? oz_nan(y) : y;
         }
+      }
     }
   }
   }

@@ -932,9 +932,10 @@ int wbg_rotate_tc_run(const void* U, long long strideU, const void* X, int nFin,
   return wbg_cuda_status(cudaGetLastError());
 }
 
-// FP64 from nw = 4 (4 096 k-points, 9 fields: 0.086 ms against 0.096 ms for rotate_kernel; 44.8 -> 5.7 ms
-// at nw = 32 and 13 824 k-points), double-float above nw = 32 (nw = 48: 6.2 against 9.9 ms, nw = 96:
-// 4.5 against 27.7 ms; below, the engine rotates in FP32) where the operands allow 16-byte loads.
+// FP64 from nw = 4 (4 096 k-points, 9 fields: 0.108 ms against 0.117 ms for rotate_kernel, nw = 5 0.112 against
+// 0.133, nw = 8 0.131 against 0.303; 44.8 -> 5.9 ms at nw = 32 and 13 824 k-points), double-float above nw = 32
+// (nw = 48: 5.7 against 9.9 ms, nw = 96: 3.8 against 27.7 ms; below, the engine rotates in FP32) where the operands
+// allow 16-byte loads.
 bool wbg_rotate_oz_supported(const void* U, const void* X, int nw, int fp64) {
   if (nw > 128) return false;
   if (fp64 == 2) return nw > NW && ((reinterpret_cast<uintptr_t>(U) | reinterpret_cast<uintptr_t>(X)) & 15) == 0;
