@@ -472,6 +472,8 @@ int wbg_scan_finalize(const void* hist, int nEF, int ncomp, double scale, double
  *                                4 for modes 2 / 3 with WBG_EIGH_PRECISE_VECTORS,
  *                                5 for modes 2 / 3 with WBG_EIGH_REFINE
  *   WBG_TUNE_EIGH_QL_BLOCK       matrices (threads) per block of the QL sweep   variant: eigh mode & 3
+ *                                (batches of up to four matrices an SM take a warp a matrix in
+ *                                FP64 and double-float, whatever block is set)
  *   WBG_TUNE_EIGH_VECTORS_GROUP  matrices per block of the inverse iteration and
  *                                back-transform                                variant: eigh mode & 3
  *                                (above nw = 32 both groups are listed and kept for saved tables:

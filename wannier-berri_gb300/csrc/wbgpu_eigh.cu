@@ -1273,10 +1273,12 @@ int launch_eigh(const void* H, long long strideH, int n, int nk, void* E, void* 
   }
   const int BQ = sh.choose(WBG_TUNE_EIGH_QL_BLOCK, variant, n, sh.ql_default(nk));
   const size_t smQ = (size_t)BQ * sh.smQ1;
-  // up to four matrices an SM: a warp each (unless the tuner chose a block of matrices).  Not the FP32 solve,
+  // up to four matrices an SM: a warp each, whatever block of matrices the tuner chose (it measures large
+  // batches, one choice for every size: 512 of 96 x 96 in double-float take 3.8 ms here, 7.9 ms in blocks of
+  // 32, the smallest listed).  Not the FP32 solve,
   // whose last bits depend on which products the compiler fuses in this very loop, and the refined
   // eigenvectors on them (3e-8 of an AHC at num_wann 32).
-  if (!std::is_same<R, float>::value && wbg_tuned(WBG_TUNE_EIGH_QL_BLOCK, variant, n) == 0 && nk <= 4 * 152) {
+  if (!std::is_same<R, float>::value && nk <= 4 * 152) {
     eigh_ql_warp<R><<<(nk + QW_WARPS - 1) / QW_WARPS, 32 * QW_WARPS, QW_WARPS * sh.smQ1, stream>>>(d, e, n, nk,
                                                                                                   (double*)E, errflag);
   } else {
