@@ -30,6 +30,9 @@ PARAM_NAMES = {EIGH_TRIDIAG_GROUP: 'eigh_tridiag_group', EIGH_QL_BLOCK: 'eigh_ql
                ROTATE_ENGINE: 'rotate_engine', KUBO_ENGINE: 'kubo_engine'}
 EIGH_PARAMS = (EIGH_TRIDIAG_GROUP, EIGH_QL_BLOCK, EIGH_VECTORS_GROUP)
 ROTATE_PARAMS = (ROTATE_KPOINTS, ROTATE_ENGINE)
+# Generation of the kernels that the parameters shape, part of a cached table's key: raise it when a step changes
+# what a shape costs, so that tables measured on the former kernels are measured again
+KERNELS = 2
 # eigh mode and rotation variant (fp64 flag) of each precision of run()
 PRECISE_VECTORS = 64  # wbg_eigh_batched mode bit WBG_EIGH_PRECISE_VECTORS
 PRECISION_VARIANTS = {'fp64': (1, 1), 'mixed': (3 | PRECISE_VECTORS, 0)}
@@ -156,7 +159,8 @@ def tune_eigh(nw, mode, nk=None, reps=3, seed=0, device='cuda'):
     import torch
     variant = eigh_variant(mode)
     run = _eigh_runner(nw, mode, default_batch(nw, nk), seed, device)
-    params = {p: candidates(p, nw, variant) for p in EIGH_PARAMS}
+    # above nw = 32 the reduction and the vectors take a matrix a block whatever group is set
+    params = {p: candidates(p, nw, variant) for p in (EIGH_PARAMS if nw <= 32 else (EIGH_QL_BLOCK,))}
     params = {p: c for p, c in params.items() if len(c) > 1}
     if EIGH_QL_BLOCK in params:  # the built-in sweep spreads few matrices over the SMs, which no listed block does
         params[EIGH_QL_BLOCK] = [0] + params[EIGH_QL_BLOCK]  # (1 024 of 96 x 96: 15.7 against 17.7 ms)
@@ -171,7 +175,8 @@ def tune_rotate(nw, fp64, nk=None, nfields=9, reps=3, seed=0, device='cuda'):
     count of the mixed path by default); the table holds the choice afterwards."""
     import torch
     from . import engine
-    params = {p: candidates(p, nw, int(bool(fp64))) for p in ROTATE_PARAMS}
+    # the tensor-core rotation that serves FP64 reads no shape
+    params = {} if fp64 else {p: candidates(p, nw, 0) for p in ROTATE_PARAMS}
     params = {p: c for p, c in params.items() if len(c) > 1}
     if not params:
         return {}, {}
@@ -209,7 +214,7 @@ def cache_path():
 
 def _entry_key(device_name, nw, precision):
     abi = _lib.load().wbg_abi_version()
-    return f"{device_name}|abi{abi}|nw{int(nw)}|{precision}"
+    return f"{device_name}|abi{abi}|kernels{KERNELS}|nw{int(nw)}|{precision}"
 
 
 def load_cache(path=None):
