@@ -2399,9 +2399,10 @@ int launch_rotate(const void* U, long long strideU, const void* X, int nFin, con
                         reinterpret_cast<uintptr_t>(Xbar)) & 15) == 0;  // 16-byte pieces of every matrix
     const bool inw = tiled4_inwarp(nw);
     const size_t per_k = wide ? tiled4_words(nw, inw) * 8 : tiled_words(nw) * sizeof(V);
-    // k-points per block: up to 256 threads and 64 KB, but no fewer blocks than two per SM (152)
+    // k-points per block: up to 256 threads and 64 KB, but no fewer blocks than two per SM
+    const int blocks = 2 * wbg_sm_count();
     int KB = 1;
-    while (KB * 2 * tpk <= 256 && (KB * 2) * per_k <= 64 * 1024 && nk / (KB * 2) >= 304) KB *= 2;
+    while (KB * 2 * tpk <= 256 && (KB * 2) * per_k <= 64 * 1024 && nk / (KB * 2) >= blocks) KB *= 2;
     if (KB * per_k <= 200 * 1024) {
       const int t = wbg_tuned(WBG_TUNE_ROTATE_KPOINTS, sizeof(T) == 8 ? 1 : 0, nw);
       if (t > 0 && tiled_kpoints_fit(t, tpk, per_k)) KB = t;

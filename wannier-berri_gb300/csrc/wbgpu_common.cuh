@@ -61,3 +61,11 @@ template <typename V> WBG_HD V czero() { V r; r.x = 0; r.y = 0; return r; }
 // Records e as the library's last CUDA error (wbg_last_cuda_error_string) and returns WBG_ERR_CUDA.
 int wbg_note_cuda_error(cudaError_t e);
 static inline int wbg_cuda_status(cudaError_t e) { return e == cudaSuccess ? WBG_OK : wbg_note_cuda_error(e); }
+// SMs of the current device (a GB300's where the query fails: the launch that follows reports the error)
+static inline int wbg_sm_count() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
+    return 152;
+  return sms;
+}

@@ -1199,14 +1199,14 @@ struct EighShape {
   }
   int tridiag_default() const { return pick_group(smT, LT, gmaxT); }
   // Matrices (threads) per block of the QL sweep, a power of two up to 128: as few as spread the batch over
-  // the SMs (152) with `warps` warps each, since a warp takes as long as the longest and most divergent of
+  // the SMs with `warps` warps each, since a warp takes as long as the longest and most divergent of
   // its matrices.  An FP64 warp instruction takes the SM's FP64 pipe for 17 cycles whatever its active
   // lanes, so 3 FP64 warps fill it; 4 warps hide the FP32 and double-float chains.
   // 512 double-float matrices of 96 x 96: 6.7 ms (32 a warp) -> 4.7 ms (one a warp).
-  int ql_default(int nk) const {
+  int ql_default(int nk, int sms) const {
     const int warps = std::is_same<R, double>::value ? 3 : 4;
     int BQ = 1;
-    while (BQ < 128 && (long long)BQ * 152 * warps < nk) BQ *= 2;
+    while (BQ < 128 && (long long)BQ * sms * warps < nk) BQ *= 2;
     while (BQ > 32 && (size_t)BQ * smQ1 > 64 * 1024) BQ /= 2;
     return BQ;
   }
@@ -1271,14 +1271,15 @@ int launch_eigh(const void* H, long long strideH, int n, int nk, void* E, void* 
     }
     if (stage == 1) return wbg_cuda_status(cudaGetLastError());
   }
-  const int BQ = sh.choose(WBG_TUNE_EIGH_QL_BLOCK, variant, n, sh.ql_default(nk));
+  const int sms = wbg_sm_count();
+  const int BQ = sh.choose(WBG_TUNE_EIGH_QL_BLOCK, variant, n, sh.ql_default(nk, sms));
   const size_t smQ = (size_t)BQ * sh.smQ1;
   // up to four matrices an SM: a warp each, whatever block of matrices the tuner chose (it measures large
   // batches, one choice for every size: 512 of 96 x 96 in double-float take 3.8 ms here, 7.9 ms in blocks of
   // 32, the smallest listed).  Not the FP32 solve,
   // whose last bits depend on which products the compiler fuses in this very loop, and the refined
   // eigenvectors on them (3e-8 of an AHC at num_wann 32).
-  if (!std::is_same<R, float>::value && nk <= 4 * 152) {
+  if (!std::is_same<R, float>::value && nk <= 4 * sms) {
     eigh_ql_warp<R><<<(nk + QW_WARPS - 1) / QW_WARPS, 32 * QW_WARPS, QW_WARPS * sh.smQ1, stream>>>(d, e, n, nk,
                                                                                                   (double*)E, errflag);
   } else {
