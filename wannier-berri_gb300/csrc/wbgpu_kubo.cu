@@ -750,11 +750,14 @@ int wbg_dynamic_run(const double* E, const void* Xbar, int nFbar, const wbg_dyna
 #undef WBG_GEMM64
   } else if (nc == 1) {
     WBG_ACCUM(1, float);
-  } else if (wbg_tuned(WBG_TUNE_KUBO_ENGINE, 0, 1) != 2) {  // tensor cores (the built-in choice)
-    const int st = wbg_kubo_tc_run(rec_dE, rec_fE, rec_M, count, P, nk, omega, kp->nOmega, kp->nEF, nc, kp->eta,
-                                   kp->gaussian, F, out, stream);
-    if (st != WBG_OK) return st;
-  } else {  // the register-tiled GEMM: one block per SM, frequency x column tiles x k chunks
+  } else {
+    int st = WBG_ERR_SIZE;
+    if (wbg_tuned(WBG_TUNE_KUBO_ENGINE, 0, 1) != 2)  // tensor cores (the built-in choice)
+      st = wbg_kubo_tc_run(rec_dE, rec_fE, rec_M, count, P, nk, omega, kp->nOmega, kp->nEF, nc, kp->eta,
+                           kp->gaussian, F, out, stream);
+    if (st != WBG_ERR_SIZE) return st;
+    // the register-tiled GEMM (chosen, or a build in which the tensor-core kernel's registers do not fit): one
+    // block per SM, frequency x column tiles x k chunks
     const int gw = (kp->nOmega + KG_TW - 1) / KG_TW, gc = (kp->nEF * nc + KG_TC - 1) / KG_TC;
     int gk = sms / (gw * gc);  // one wave of one block per SM
     if (gk < 1) gk = 1;

@@ -1009,6 +1009,7 @@ int wbg_kubo_tc_run(const double* rec_dE, const void* rec_fE, const void* rec_M,
   if (const cudaError_t e_ = cudaFuncSetAttribute(kubo_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, KT_SMEM))
     return wbg_cuda_status(e_);
   // the roles' register shares come out of the launch's: a build with fewer registers a thread would wait forever
+  // (the caller then takes the CUDA-core GEMM)
   cudaFuncAttributes fa;
   if (const cudaError_t e_ = cudaFuncGetAttributes(&fa, kubo_tc)) return wbg_cuda_status(e_);
   if (fa.numRegs < KT_REG_LAUNCH) return WBG_ERR_SIZE;
