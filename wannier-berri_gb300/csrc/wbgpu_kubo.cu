@@ -189,7 +189,7 @@ template <typename T, int F>
 __global__ void kubo_pairs(const double* __restrict__ E, const typename C2<T>::t* __restrict__ Xbar, int nFbar,
                            wbg_dynamic_spec fs, int nw, WbgKubo kp, const double* __restrict__ efermi,
                            double* __restrict__ rec_dE, T* __restrict__ rec_fE, typename C2<T>::t* __restrict__ rec_M,
-                           int* __restrict__ count, int P) {
+                           int* __restrict__ count, int P, int table) {
   typedef typename C2<T>::t V;
   constexpr int NC = dyn_ncomp(F);
   extern __shared__ double smk[];
@@ -226,12 +226,12 @@ __global__ void kubo_pairs(const double* __restrict__ E, const typename C2<T>::t
   band.nw2 = nw2;
   band.f = fs;
   band.pf = nullptr;
-  if (F == WBG_DYN_SHIFT) {  // nw^2 principal-value factors once, instead of two divisions per pair and band
+  // nw^2 principal-value factors once, instead of two divisions per pair and band.  One block an SM is all that
+  // fits at num_wann 128 in FP64, and it still pays: 125 k-points 109.6 -> 93.1 ms (mixed 26.7 -> 10.8), num_wann 48,
+  // 216 k-points 11.0 -> 9.4 (1.9 -> 0.53), 12, 1 000 k-points 0.99 -> 0.85 ms (0.23 -> 0.08).
+  if (F == WBG_DYN_SHIFT && table) {
     T* pf = reinterpret_cast<T*>(smk + pairs_words(nw));
-    for (int i = threadIdx.x; i < nw * nw; i += blockDim.x) {
-      const double d = Es[i / nw] - Es[i % nw];
-      pf[i] = (T)(-d / (d * d + fs.sc_eta * fs.sc_eta));
-    }
+    for (int i = threadIdx.x; i < nw * nw; i += blockDim.x) pf[i] = band.pv(i / nw, i % nw);
     band.pf = pf;
     __syncthreads();
   }
@@ -635,13 +635,13 @@ void launch_gemm64(int sms, cudaStream_t stream, const double* rec_dE, const voi
 template <typename T>
 void launch_pairs(int formula, int nk, size_t smp, cudaStream_t stream, const double* E, const void* Xbar, int nFbar,
                   const wbg_dynamic_spec& fs, int nw, const WbgKubo& kp, const double* efermi, double* rec_dE,
-                  void* rec_fE, void* rec_M, int* count, int P) {
+                  void* rec_fE, void* rec_M, int* count, int P, int table) {
   typedef typename C2<T>::t V;
   const V* X = (const V*)Xbar;
   if (formula == WBG_DYN_SHIFT)
     cudaFuncSetAttribute(kubo_pairs<T, WBG_DYN_SHIFT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
 #define WBG_PAIRS(F) kubo_pairs<T, F><<<nk, 128, smp, stream>>>(E, X, nFbar, fs, nw, kp, efermi, rec_dE, (T*)rec_fE, \
-                                                                (V*)rec_M, count, P)
+                                                                (V*)rec_M, count, P, table)
   switch (formula) {
     case WBG_DYN_OPTCOND: WBG_PAIRS(WBG_DYN_OPTCOND); break;
     case WBG_DYN_JDOS: WBG_PAIRS(WBG_DYN_JDOS); break;
@@ -703,12 +703,15 @@ int wbg_dynamic_run(const double* E, const void* Xbar, int nFbar, const wbg_dyna
   double* rec_dE = (double*)w; w += (size_t)nk * P * 8;
   void* rec_fE = w; w += (size_t)nk * P * 8 * kp->nEF;
   int* count = (int*)w;
-  const size_t smp = 8 * pairs_words(nw) + (F == WBG_DYN_SHIFT ? (size_t)nw * nw * (fp64 ? 8 : 4) : 0);
-  if (smp > 220 * 1024) return WBG_ERR_SIZE;
+  const size_t smtab = F == WBG_DYN_SHIFT ? (size_t)nw * nw * (fp64 ? 8 : 4) : 0;
+  const int table = 8 * pairs_words(nw) + smtab <= 220 * 1024;  // else each pair divides for itself
+  const size_t smp = 8 * pairs_words(nw) + (table ? smtab : 0);
   if (fp64)
-    launch_pairs<double>(F, nk, smp, stream, E, Xbar, nFbar, *fs, nw, *kp, efermi, rec_dE, rec_fE, rec_M, count, P);
+    launch_pairs<double>(F, nk, smp, stream, E, Xbar, nFbar, *fs, nw, *kp, efermi, rec_dE, rec_fE, rec_M, count, P,
+                         table);
   else
-    launch_pairs<float>(F, nk, smp, stream, E, Xbar, nFbar, *fs, nw, *kp, efermi, rec_dE, rec_fE, rec_M, count, P);
+    launch_pairs<float>(F, nk, smp, stream, E, Xbar, nFbar, *fs, nw, *kp, efermi, rec_dE, rec_fE, rec_M, count, P,
+                        table);
   // threads per block and levels per block: fewest passes over the records
   // (frequency blocks x level chunks), accumulators within 96 KB of shared memory
   const size_t smax = 96 * 1024;

@@ -13,7 +13,7 @@ struct KBand {
   int nw;
   long long nw2;
   wbg_dynamic_spec f;
-  const T* pf;  // [nw][nw] -(E_p - E_q) / ((E_p - E_q)^2 + sc_eta^2), the shift current's only
+  const T* pf;  // [nw][nw] pv(p, q), the shift current's where it fits in shared memory, else null
   WBG_D V x(int fld, int p, int q) const { return X[fld * nw2 + (long long)p * nw + q]; }
   WBG_D T dinv(int p, int q) const {  // dEig_inv (data_K.py:290-298)
     const double d = E[p] - E[q];
@@ -25,8 +25,12 @@ struct KBand {
     if (f.external_terms) r = cadd(r, x(f.A + a, p, q));
     return r;
   }
+  WBG_D T pv(int p, int q) const {
+    const double d = E[p] - E[q];
+    return (T)(-d / (d * d + f.sc_eta * f.sc_eta));
+  }
   // principal-value D of the shift current: -V_pq (E_p - E_q) / ((E_p - E_q)^2 + eta^2)
-  WBG_D V Dp(int a, int p, int q) const { return cscale(x(f.V + a, p, q), pf[p * nw + q]); }
+  WBG_D V Dp(int a, int p, int q) const { return cscale(x(f.V + a, p, q), pf ? pf[p * nw + q] : pv(p, q)); }
 };
 
 // J'[p][q][a][s] of the spin current before (J' + J'^dagger) / 2 (formula/covariant.py:721-756),
