@@ -2051,8 +2051,10 @@ __global__ void __launch_bounds__(DH_THR, DH_OCC)
             gs = 0;
             ge = bandmax;
             in = true;
+          } else if (bs.sel) {  // the whole group when any of its bands is selected: dinvS's columns of a group are
+            for (int q = gs; q < ge; ++q) in |= bs.sel[k * nw + q] == 1;  // consecutive (the others' values are dropped)
           } else {
-            in = bs.sel ? bs.sel[k * nw + m] == 1 : (Es[ge - 1] >= sp.EFmin && Es[gs] <= sp.EFmax);
+            in = Es[ge - 1] >= sp.EFmin && Es[gs] <= sp.EFmax;
           }
           gsS[m] = gs;
           geS[m] = ge;
@@ -2233,7 +2235,8 @@ __global__ void __launch_bounds__(DH_THR, DH_OCC)
       const int im = i / 9, c = i - im * 9;
       double v = 0.0;
       for (int s = 0; s < S; ++s) v += part[(s * M + im) * 9 + c];
-      tv[act[im] * 9 + c] = v;
+      const int m = act[im];
+      if (m < bandmax || !bs.sel || bs.sel[k * nw + m] == 1) tv[m * 9 + c] = v;
     }
     __syncthreads();
     if (bs.P) {
