@@ -56,12 +56,16 @@ def test_batches_around_the_lower_triangle_line(div, fft, batches):
             assert np.array_equal(t.wait()[q].data, ref[q].data), q
 
 
-@pytest.mark.parametrize("iters", [0, 2])
-def test_tabulated_and_refined_batches(monkeypatch, iters):
+@pytest.mark.parametrize("iters,fft", [(0, (2, 2, 3)),  # values of a batch cut on the host
+                                       (0, (9, 9, 6)),  # 4 860 rows a batch: packed on the device
+                                       (2, (2, 2, 3))])
+def test_tabulated_and_refined_batches(monkeypatch, iters, fft):
+    """Energies, gradients and curvatures of two blocks at a time through the page-locked buffers, against all at once;
+    adaptive refinement."""
     import importlib
     R = importlib.import_module('wbgpu.run')
     s = wsys.System_R.from_dict(models.random_tb(5, 1, LAT, seed=4))
-    grid = wbgpu.Grid(s, NKdiv=3, NKFFT=(2, 2, 3))
+    grid = wbgpu.Grid(s, NKdiv=3, NKFFT=fft)
     EF = np.linspace(-1.0, 1.0, 11)
     if iters:
         go = lambda: {k: v.data for k, v in wbgpu.run(s, grid, {'ahc': C.AHC(Efermi=EF)}, adpt_num_iter=iters).items()}
