@@ -17,7 +17,7 @@
 
 typedef unsigned long long wbg_u64;
 
-// (lo, hi) of floor(v 2^60) for finite v, from the bits of v: the FP64 pipe issues 64 times slower than the
+// (lo, hi) of floor(v 2^60) for finite v (of |v| >= 2^67 the nearest end of the range), from the bits of v: the FP64 pipe issues 64 times slower than the
 // integer one, and its v 2^-4 - floor(v 2^-4) would round the fraction of a negative v
 WBG_D void fx_split(double v, wbg_u64& lo, wbg_u64& hi) {
   const wbg_u64 u = (wbg_u64)__double_as_longlong(v);
@@ -25,9 +25,12 @@ WBG_D void fx_split(double v, wbg_u64& lo, wbg_u64& hi) {
   const wbg_u64 m = (u & 0xfffffffffffffull) | (e ? 0x10000000000000ull : 0ull);
   const int s = (e ? e : 1) - 1015;  // |v| 2^60 = m 2^s
   bool frac = false;                 // a fraction was cut off |v| 2^60
-  if (s >= 128) {
-    lo = hi = 0;
-  } else if (s >= 64) {
+  if (s >= 75) {  // |v| >= 2^67
+    lo = 0;
+    hi = (long long)u < 0 ? 0x8000000000000000ull : 0x7fffffffffffffffull;
+    return;
+  }
+  if (s >= 64) {
     lo = 0;
     hi = m << (s - 64);
   } else if (s > 0) {
