@@ -2276,44 +2276,56 @@ __global__ void __launch_bounds__(DH_THR, DH_OCC)
 // cumulative sum over Fermi levels and normalisation: out[ie][c] = scale * sum_{j<=ie} hist[j][c],
 // hist in the fixed-point layout of wbgpu_fixed.cuh; NaN throughout when a contribution was not finite.
 // One block per component: every thread adds a run of levels, the block scans the runs, every thread
-// writes its run -- all in the histogram's 128-bit integers, so a level is rounded once whatever the
-// split (a chain of FP64 additions rounds at every level).  Bound by launch latency: 5 us where one
+// writes its run -- all in the histogram's 128-bit integers and a word above them (sums over the levels may
+// leave the range of one entry), so a level is rounded once whatever the split (a chain of FP64 additions
+// rounds at every level).  Bound by launch latency: 5 us where one
 // thread per component walked 1 001 levels of dependent loads in 360 us.
 constexpr int SCAN_THR = 256;
-WBG_D void add128(wbg_u64& lo, wbg_u64& hi, wbg_u64 l, wbg_u64 h) {
-  const wbg_u64 s = lo + l;
-  hi += h + (s < l ? 1ull : 0ull);
-  lo = s;
+struct Sum192 {  // two's complement: lo, hi, top
+  wbg_u64 lo, hi, top;
+};
+WBG_D void add192(Sum192& a, const Sum192& b) {
+  const wbg_u64 l = a.lo + b.lo, c = l < a.lo ? 1ull : 0ull, h = a.hi + b.hi, h2 = h + c;
+  a.top += b.top + (h < a.hi ? 1ull : 0ull) + (h2 < h ? 1ull : 0ull);
+  a.lo = l;
+  a.hi = h2;
 }
+WBG_D Sum192 neg192(const Sum192& a) {
+  Sum192 n = {~a.lo, ~a.hi, ~a.top};
+  const Sum192 one = {1ull, 0ull, 0ull};
+  add192(n, one);
+  return n;
+}
+// entry of a histogram, sign-extended
+WBG_D Sum192 entry192(const wbg_u64* e) { return {e[0], e[1], (long long)e[1] < 0 ? ~0ull : 0ull}; }
 __global__ void __launch_bounds__(SCAN_THR) scan_finalize_kernel(const wbg_u64* __restrict__ hist, int nEF, int ncomp,
                                                                  double scale, double* __restrict__ out) {
-  __shared__ wbg_u64 tot[SCAN_THR / 32][2];
+  __shared__ Sum192 tot[SCAN_THR / 32];
   const int c = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool bad = hist[2 * (size_t)nEF * ncomp] != 0ull;
   const int run = (nEF + SCAN_THR - 1) / SCAN_THR;
   const long long i0 = (long long)tid * run, i1 = i0 + run < nEF ? i0 + run : nEF;
-  wbg_u64 lo = 0, hi = 0;
-  for (long long ie = i0; ie < i1; ++ie) add128(lo, hi, hist[2 * (ie * ncomp + c)], hist[2 * (ie * ncomp + c) + 1]);
-  const wbg_u64 lo0 = lo, hi0 = hi;
+  Sum192 sum = {0ull, 0ull, 0ull};
+  for (long long ie = i0; ie < i1; ++ie) add192(sum, entry192(hist + 2 * (ie * ncomp + c)));
+  const Sum192 own = sum;
 #pragma unroll
   for (int off = 1; off < 32; off <<= 1) {  // inclusive scan of the warp's runs
-    const wbg_u64 l = __shfl_up_sync(0xffffffffu, lo, off), h = __shfl_up_sync(0xffffffffu, hi, off);
-    if (lane >= off) add128(lo, hi, l, h);
+    const Sum192 o = {__shfl_up_sync(0xffffffffu, sum.lo, off), __shfl_up_sync(0xffffffffu, sum.hi, off),
+                      __shfl_up_sync(0xffffffffu, sum.top, off)};
+    if (lane >= off) add192(sum, o);
   }
-  if (lane == 31) {
-    tot[warp][0] = lo;
-    tot[warp][1] = hi;
-  }
+  if (lane == 31) tot[warp] = sum;
   __syncthreads();
-  for (int w = 0; w < warp; ++w) add128(lo, hi, tot[w][0], tot[w][1]);
-  add128(lo, hi, ~lo0 + 1ull, ~hi0 + (lo0 == 0 ? 1ull : 0ull));  // exclusive: less the own run
+  for (int w = 0; w < warp; ++w) add192(sum, tot[w]);
+  add192(sum, neg192(own));  // exclusive: less the own run
   for (long long ie = i0; ie < i1; ++ie) {
     const size_t e = (size_t)(ie * ncomp + c);
-    add128(lo, hi, hist[2 * e], hist[2 * e + 1]);
+    add192(sum, entry192(hist + 2 * e));
     // through the magnitude: of a small negative sum, hi 2^4 and the fraction would cancel
-    const bool neg = (long long)hi < 0;
-    const wbg_u64 ml = neg ? ~lo + 1ull : lo, mh = neg ? ~hi + (lo == 0 ? 1ull : 0ull) : hi;
-    const double v = fx_value(ml, mh);
+    const bool neg = (long long)sum.top < 0;
+    const Sum192 m = neg ? neg192(sum) : sum;
+    // below 2^67 as an entry; above, the fraction is far below the last bit
+    const double v = m.top == 0 && (long long)m.hi >= 0 ? fx_value(m.lo, m.hi) : (double)m.top * 0x1p68 + (double)m.hi * 0x1p4;
     out[e] = bad ? nan("") : (neg ? -v : v) * scale;
   }
 }
