@@ -22,7 +22,7 @@
 // its accumulator drained.  Two stages and two accumulators alternate: a fill is formed while the
 // previous one multiplies and the one before that is drained.  Every mbarrier wait is bounded by the
 // kernel's wait limit, as in the rotation.
-// Bound by the producers' instruction streams (issue slots 44% active, tensor pipe 30%).  At 400
+// Bound by the producers' instruction streams (one 4^3 block: issue slots 50% active, tensor pipe 30%).  At 400
 // frequencies x 11 levels x 9 components, num_wann 96 and 512 k-points: 27.8 ms with eight-record
 // chunks, three producer barriers each and the sums in shared memory; 11.9 ms with fills formed in one
 // go and the sums in registers by eight producer warps, 10.7 ms by these twelve.
